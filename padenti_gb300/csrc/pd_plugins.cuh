@@ -10,6 +10,12 @@
 //   eval_train(prep, cand)   the same on the trainer's copy of the images, which
 //                            kTrainMapsZero plugins store with 0 replaced by the
 //                            background depth (equal responses, one test fewer);
+// and the histogram kernel's form of the same response, from per-sample words
+// that a warp stages in shared memory (word 3 is the kernel's):
+//   fast_candidate(f)        the constants of a candidate whose P::fast holds;
+//   fast_stage(im, x, y, pre, w)  fills the words of a sample; false where the
+//                            form does not hold (the sample takes eval_train);
+//   eval_fast(a, b, cand)    the response from words a = w[0..3], b = w[4..7];
 // and kOrderDim, the feature dims (kOrderDim, kOrderDim + 1) of its first probe
 // offset, by which the trainer orders a node's candidates.
 // eval(prep, f) runs all of it for a single evaluation.
@@ -120,6 +126,56 @@ struct OffsetConst {
   }
 };
 
+// The same rounding in one fused multiply-add.  With i = fl(1/d), u' = u + 1/4
+// sgn(u) and M = 3*2^22, fl(u' i + (M + x)) - M is x + round_half_away(u / d) for
+// |u| <= 2^21, d in [1, 65535] and 0 <= x < 2^16: floats in [2^23, 2^24) are the
+// integers, so the fused operation rounds the exact u' i + M + x once, to the
+// nearest integer.  |u|/d + 1/2 lies a multiple of 1/(2d) above an integer; the
+// quarter moves it to at least 1/(4d) from both ends of its unit interval, so no
+// tie is left, and the error of i, |u'| / d * 2^-24 < 1/(7d), does not reach
+// either end.  Two instructions per coordinate (the multiply-add and the
+// subtraction of M's bits) where the wide multiply, the shift by the divider's
+// exponent and the sign's multiply-add take three, and one constant per offset
+// in place of two.
+constexpr float kRoundMagic = 12582912.0f;
+constexpr uint32_t kRoundBits = 0x4B400000u;  // the bits of kRoundMagic
+PD_D float fast_offset(int32_t u) { return (float)u + (u < 0 ? -0.25f : 0.25f); }
+// x + round_half_away(u / d) as an unsigned number (negative: above every side);
+// base = kRoundMagic + x.
+PD_D uint32_t fast_coord(float u, float inv_d, float base) {
+#if defined(__CUDA_ARCH__)
+  return __float_as_uint(__fmaf_rn(u, inv_d, base)) - kRoundBits;
+#else
+  return 0u;
+#endif
+}
+PD_D float inv_depth(uint32_t d) {
+#if defined(__CUDA_ARCH__)
+  return __frcp_rn((float)d);
+#else
+  return 1.0f / (float)d;
+#endif
+}
+PD_D uint32_t float_bits(float f) {
+#if defined(__CUDA_ARCH__)
+  return __float_as_uint(f);
+#else
+  return 0u;
+#endif
+}
+PD_D float bits_float(uint32_t u) {
+#if defined(__CUDA_ARCH__)
+  return __uint_as_float(u);
+#else
+  return 0.0f;
+#endif
+}
+// An image pointer in two staged words.
+template <typename ImgT>
+PD_D const ImgT *staged_ptr(uint32_t lo, uint32_t hi) {
+  return reinterpret_cast<const ImgT *>((uint64_t)lo | ((uint64_t)hi << 32));
+}
+
 // I(x+u/d(x)) - I(x+v/d(x)); u,v in pixel*mm, d(x) the centre depth in mm.
 // Probes outside the image or on zero depth read 10000; a zero centre depth
 // scales as 10000.  Offsets are (int)roundf((float)u / (float)d), computed
@@ -199,6 +255,39 @@ struct DepthDiff2 {
   template <bool FAST = false>
   static PD_D int32_t eval_train(const Prep &p, const Cand &c) { return eval<FAST, true>(p, c); }
   static PD_D int32_t eval(const Prep &p, const int32_t *f) { return eval(p, candidate(f)); }
+  // ---- staged form (on the trainer's copy): words 1/d, M + x, M + y, -, image, w, h ----
+  static constexpr bool kFastAlways = true;   // fast_stage never fails
+  static constexpr bool kSmallResp = true;    // |response| < 2^17
+  struct FastCand {
+    float o[4];
+  };
+  static PD_D FastCand fast_candidate(const int32_t *f) {
+    FastCand c;
+#pragma unroll
+    for (int k = 0; k < 4; k++) c.o[k] = fast_offset(f[k]);
+    return c;
+  }
+  static PD_D bool fast_stage(const ImageRef<uint16_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint32_t *w) {
+    const uint64_t p = (uint64_t)im.data;
+    w[0] = float_bits(inv_depth(pre[0]));
+    w[1] = float_bits(kRoundMagic + (float)x);
+    w[2] = float_bits(kRoundMagic + (float)y);
+    w[4] = (uint32_t)p;
+    w[5] = (uint32_t)(p >> 32);
+    w[6] = (uint32_t)im.w;
+    w[7] = (uint32_t)im.h;
+    return true;
+  }
+  static PD_D int32_t fast_probe(const uint4 &a, const uint4 &b, float u, float v) {
+    const float inv = bits_float(a.x);
+    const uint32_t x = fast_coord(u, inv, bits_float(a.y)), y = fast_coord(v, inv, bits_float(a.z));
+    uint32_t r = (uint32_t)kBgDepth;
+    if (x < b.z && y < b.w) r = ldg(staged_ptr<uint16_t>(b.x, b.y) + (y * b.z + x));
+    return (int32_t)r;
+  }
+  static PD_D int32_t eval_fast(const uint4 &a, const uint4 &b, const FastCand &c) {
+    return fast_probe(a, b, c.o[0], c.o[1]) - fast_probe(a, b, c.o[2], c.o[3]);
+  }
 };
 
 // The reference example plugin test/feature.cl:29-64 with feat_t = short:
@@ -280,6 +369,40 @@ struct DepthDiff1 {
   template <bool FAST = false>
   static PD_D int16_t eval_train(const Prep &p, const Cand &c) { return eval<FAST>(p, c); }
   static PD_D int16_t eval(const Prep &p, const int16_t *f) { return eval(p, candidate(f)); }
+  // ---- staged form: words 1/d, M + x, M + y, -, image, w | h << 16, d.  A zero
+  // centre depth reads every probe as outside (w = 0); a negative one (a depth
+  // above 32767 read as short) takes eval_train. ----
+  static constexpr bool kFastAlways = false;
+  static constexpr bool kSmallResp = true;
+  struct FastCand {
+    float o[2];
+  };
+  static PD_D FastCand fast_candidate(const int16_t *f) {
+    FastCand c;
+    c.o[0] = fast_offset(500 * (int32_t)f[0]);
+    c.o[1] = fast_offset(500 * (int32_t)f[1]);
+    return c;
+  }
+  static PD_D bool fast_stage(const ImageRef<uint16_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint32_t *w) {
+    const uint64_t p = (uint64_t)im.data;
+    const int32_t d = (int16_t)(int32_t)pre[0];
+    w[0] = float_bits(inv_depth(d > 0 ? (uint32_t)d : 1u));
+    w[1] = float_bits(kRoundMagic + (float)x);
+    w[2] = float_bits(kRoundMagic + (float)y);
+    w[4] = (uint32_t)p;
+    w[5] = (uint32_t)(p >> 32);
+    w[6] = (d ? (uint32_t)im.w : 0u) | ((uint32_t)im.h << 16);
+    w[7] = (uint32_t)d;
+    return d >= 0;
+  }
+  static PD_D int16_t eval_fast(const uint4 &a, const uint4 &b, const FastCand &c) {
+    const float inv = bits_float(a.x);
+    const uint32_t x = fast_coord(c.o[0], inv, bits_float(a.y)), y = fast_coord(c.o[1], inv, bits_float(a.z));
+    const uint32_t w = b.z & 0xffffu;
+    int16_t v = 0;
+    if (x < w && y < (b.z >> 16)) v = (int16_t)ldg(staged_ptr<uint16_t>(b.x, b.y) + (y * w + x));
+    return (int16_t)((int32_t)b.w - (v ? (int32_t)v : kBgDepth));
+  }
 };
 
 // I_c1(x+u) - I_c2(x+v) on an RGB uint8 image; channels clamped to [0,2]
@@ -338,6 +461,47 @@ struct ChannelDiff {
   template <bool FAST = false>
   static PD_D int32_t eval_train(const Prep &p, const Cand &c) { return eval<FAST>(p, c); }
   static PD_D int32_t eval(const Prep &p, const int32_t *f) { return eval(p, candidate(f)); }
+  // ---- staged form: words 3w, x, y, -, the pixel's address, w, h.  A probe is
+  // uy * 3w + (3 ux + c) bytes from the pixel, in 32 bits (images of fewer than
+  // 2^31 bytes; an offset that leaves the image loads nothing, whatever it
+  // wraps to). ----
+  static constexpr bool kFastAlways = false;
+  static constexpr bool kSmallResp = true;
+  struct FastCand {
+    int32_t ux, uy, vx, vy;
+    uint32_t o1, o2;
+  };
+  static PD_D FastCand fast_candidate(const int32_t *f) {
+    const Cand c = candidate(f);
+    FastCand r;
+    r.ux = c.ux;
+    r.uy = c.uy;
+    r.vx = c.vx;
+    r.vy = c.vy;
+    r.o1 = 3u * (uint32_t)c.ux + (uint32_t)c.c1;
+    r.o2 = 3u * (uint32_t)c.vx + (uint32_t)c.c2;
+    return r;
+  }
+  static PD_D bool fast_stage(const ImageRef<uint8_t> &im, int32_t x, int32_t y, const uint32_t *, uint32_t *w) {
+    const uint64_t p = (uint64_t)im.data + ((uint64_t)((uint32_t)y * (uint32_t)im.w + (uint32_t)x)) * 3u;
+    w[0] = 3u * (uint32_t)im.w;
+    w[1] = (uint32_t)x;
+    w[2] = (uint32_t)y;
+    w[4] = (uint32_t)p;
+    w[5] = (uint32_t)(p >> 32);
+    w[6] = (uint32_t)im.w;
+    w[7] = (uint32_t)im.h;
+    return 3ull * (uint64_t)im.w * (uint64_t)im.h < (1ull << 31);
+  }
+  static PD_D int32_t fast_read(const uint4 &a, const uint4 &b, int32_t ux, int32_t uy, uint32_t o) {
+    uint32_t r = 0u;
+    if (a.y + (uint32_t)ux < b.z && a.z + (uint32_t)uy < b.w)
+      r = ldg(staged_ptr<uint8_t>(b.x, b.y) + (int32_t)((uint32_t)uy * a.x + o));
+    return (int32_t)r;
+  }
+  static PD_D int32_t eval_fast(const uint4 &a, const uint4 &b, const FastCand &c) {
+    return fast_read(a, b, c.ux, c.uy, c.o1) - fast_read(a, b, c.vx, c.vy, c.o2);
+  }
 };
 
 // Calls fn.template operator()<Plugin>() for the plugin id; returns

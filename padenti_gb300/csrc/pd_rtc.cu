@@ -115,7 +115,7 @@ struct RtcPlugin {
   std::string source, arch;
   std::vector<cudaLibrary_t> libs;
   RtcKernels base;
-  std::map<int, cudaKernel_t> hist;  // TP * 16 + SPI
+  std::map<std::string, cudaKernel_t> hist;  // by name expression
 };
 
 int rtc_kernels(pd_ctx *ctx, const RtcKernels **out) {
@@ -124,16 +124,15 @@ int rtc_kernels(pd_ctx *ctx, const RtcKernels **out) {
   return PD_OK;
 }
 
-int rtc_hist_kernel(pd_ctx *ctx, uint32_t TP, int SPI, cudaKernel_t *out) {
+// A histogram kernel of the plugin, compiled on first use.
+static int rtc_hist(pd_ctx *ctx, const std::string &expr, cudaKernel_t *out) {
   PD_CHECK(ctx->rtc, PD_ERR_STATE, "the user feature plugin is not compiled (pd_plugin_compile)");
-  const int key = (int)TP * 16 + SPI;
-  auto it = ctx->rtc->hist.find(key);
+  auto it = ctx->rtc->hist.find(expr);
   if (it != ctx->rtc->hist.end()) {
     *out = it->second;
     return PD_OK;
   }
-  const std::vector<std::string> exprs = {"pd::k_hist<pd::UserPlugin, " + std::to_string(TP) + ", " +
-                                          std::to_string(SPI) + ">"};
+  const std::vector<std::string> exprs = {expr};
   std::string cubin;
   std::vector<std::string> low;
   PD_TRY(compile_unit(ctx->cfg, ctx->rtc->source, ctx->rtc->arch, exprs, &cubin, &low, nullptr));
@@ -141,7 +140,7 @@ int rtc_hist_kernel(pd_ctx *ctx, uint32_t TP, int SPI, cudaKernel_t *out) {
   std::vector<cudaKernel_t> ks;
   PD_TRY(load_kernels(cubin, low, &lib, &ks));
   ctx->rtc->libs.push_back(lib);
-  ctx->rtc->hist[key] = ks[0];
+  ctx->rtc->hist[expr] = ks[0];
   *out = ks[0];
   return PD_OK;
 }
@@ -162,32 +161,56 @@ int rtc_launch(pd_ctx *ctx, cudaKernel_t k, dim3 grid, dim3 block, size_t smem, 
 
 // The histogram launch of a user feature: the same work list, shared memory
 // and launch shapes as the compiled-in kernel (pd_hist_grid_impl.cuh), with
-// k_hist<UserPlugin, TP, SPI> compiled for the context's GPU.
+// k_hist<UserPlugin, TP, SPI> and k_hist_small<UserPlugin, NC> compiled for the
+// context's GPU.
 int launch_hist_grid_rtc(pd_ctx *ctx, const HistGrid &g) {
-  const int spi = (int)ctx->hist_spi;
-  const int resident = spi <= 2 ? 3 : 2;
-  cudaKernel_t uk = nullptr;
-  PD_TRY(rtc_hist_kernel(ctx, g.TP, spi, &uk));
+  const int spi = g.TP == 0 && ctx->hist_spi < 4 ? 4 : (int)ctx->hist_spi;
+  const int resident = g.TP == 0 ? kRankCtas : spi <= 2 ? 3 : 2;
+  DevSet ds = g.ds;
+  const SampleRec *rec = g.rec;
+  const void *cf = g.cand_feat, *ct = g.cand_thr;
+  uint32_t *hist = g.hist;
+  uint32_t F = g.F, T = g.T, K = g.K;
+  FusedSplit fs = g.fs;
+  int32_t lo = g.thr_lo;
+  uint32_t span = g.thr_span;
+  const uint64_t most = 0x7fffffffull / g.tiles;  // items of one grid
+  // the kernels first, so that their compilation stays outside the timed launches
+  cudaKernel_t uk = nullptr, sk[4] = {};
+  for (int i = 0; i < 4; i++)
+    if (g.small[i].n_items)
+      PD_TRY(rtc_hist(ctx, "pd::k_hist_small<pd::UserPlugin, " + std::to_string(g.small[i].nc) + ">", &sk[i]));
+  if (g.n_items)
+    PD_TRY(rtc_hist(ctx, "pd::k_hist<pd::UserPlugin, " + std::to_string(g.TP) + ", " + std::to_string(spi) + ">", &uk));
+  if (g.ev_before) PD_CUDA(cudaEventRecord(g.ev_before, ctx->stream));
+  const WorkItem *items = g.items + g.n_items;
+  for (int i = 0; i < 4; i++) {
+    const auto &s = g.small[i];
+    if (!s.n_items) continue;
+    PD_TRY(rtc_set_smem(ctx, sk[i], s.smem, small_carveout(s.nc, s.smem)));
+    for (uint64_t b = 0; b < s.n_items; b += most) {
+      const uint64_t cnt = std::min<uint64_t>(s.n_items - b, most);
+      const WorkItem *it = items + b;
+      void *args[] = {&ds, &rec, &it, &cf, &ct, &F, &T, &K, &fs, &lo, &span};
+      PD_TRY(rtc_launch(ctx, sk[i], dim3((unsigned)(cnt * g.tiles)), dim3(small_threads(s.nc)), s.smem, args));
+    }
+    items += s.n_items;
+  }
+  if (!g.n_items) return PD_OK;
   // shared memory carve-out for the resident CTAs (dynamic + a static allowance + reserved)
   const size_t per_cta = g.smem + 4096 + 1024;
   const int pct = (int)std::min<size_t>(100, (resident * per_cta * 100 + 233471) / 233472);
   PD_TRY(rtc_set_smem(ctx, uk, g.smem, pct));
   if (g.queue) PD_CUDA(cudaMemsetAsync(g.queue, 0, 4, ctx->stream));
-  if (g.ev_before) PD_CUDA(cudaEventRecord(g.ev_before, ctx->stream));
-  for (uint64_t b = 0; b < g.n_items; b += 0x7fffffffull) {
-    const uint64_t cnt = std::min<uint64_t>(g.n_items - b, 0x7fffffffull);
-    DevSet ds = g.ds;
-    const SampleRec *rec = g.rec;
-    const WorkItem *items = g.items + b;
+  for (uint64_t b = 0; b < g.n_items; b += most) {
+    const uint64_t cnt = std::min<uint64_t>(g.n_items - b, most);
+    const WorkItem *it = g.items + b;
     uint32_t n = (uint32_t)cnt;
     unsigned *queue = g.queue;
-    const void *cf = g.cand_feat, *ct = g.cand_thr;
-    uint32_t *hist = g.hist;
-    uint32_t F = g.F, T = g.T, K = g.K;
-    FusedSplit fs = g.fs;
-    void *args[] = {&ds, &rec, &items, &n, &queue, &cf, &ct, &hist, &F, &T, &K, &fs};
-    const unsigned grid = g.queue ? (unsigned)std::min<uint64_t>(cnt, (uint64_t)ctx->n_sms * resident) : (unsigned)cnt;
-    PD_TRY(rtc_launch(ctx, uk, dim3(grid), dim3(kHistThreads), g.smem, args));
+    void *args[] = {&ds, &rec, &it, &n, &queue, &cf, &ct, &hist, &F, &T, &K, &fs, &lo, &span};
+    const unsigned grid = g.queue ? (unsigned)std::min<uint64_t>(cnt * g.tiles, (uint64_t)ctx->n_sms * resident)
+                                  : (unsigned)(cnt * g.tiles);
+    PD_TRY(rtc_launch(ctx, uk, dim3(grid), dim3(hist_threads(g.TP)), g.smem, args));
     if (g.queue) break;
   }
   return PD_OK;

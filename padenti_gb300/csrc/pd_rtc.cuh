@@ -19,8 +19,6 @@ struct RtcKernels {
 
 // The compiled base kernels; PD_ERR_STATE when pd_plugin_compile has not run.
 int rtc_kernels(pd_ctx *ctx, const RtcKernels **out);
-// k_hist<UserPlugin, TP, SPI>, compiled on first use.
-int rtc_hist_kernel(pd_ctx *ctx, uint32_t TP, int SPI, cudaKernel_t *out);
 // Dynamic shared memory limit (and carve-out when pct >= 0) of a kernel.
 int rtc_set_smem(pd_ctx *ctx, cudaKernel_t k, size_t smem, int carveout_pct = -1);
 int rtc_launch(pd_ctx *ctx, cudaKernel_t k, dim3 grid, dim3 block, size_t smem, void **args);

@@ -35,6 +35,46 @@ static size_t hist_smem(const pd_ctx *ctx, uint32_t T, bool fused = true) {
   return hist + (fused ? std::max(thr, scratch) : thr);
 }
 
+// Shared memory of a CTA of the rank-table form with `rows` class rows and
+// `threads` threads: packed tile histogram, `first` bits, table, staged words.
+static size_t rank_smem(uint32_t rows, uint32_t T, uint32_t span, int threads) {
+  return (size_t)rows * (T + 1) * 32 * 4 + (size_t)kTileF * ((T + 31) / 32) * 4 + (size_t)rank_words(span) * 64 * 8 +
+         (size_t)threads / 32 * 64 * 16;
+}
+constexpr size_t kRankSmemMax = 227 * 1024 - 4096;  // dynamic; the kernels' static arrays take less than 4 KB
+
+// Whether the histogram kernels take the rank-table form: the thresholds are the
+// draws of [thr_low, thr_up] without wrapping, the table has at most
+// kRankWordsMax words a column, and a CTA's histogram of all classes fits the
+// shared memory beside it (the search form takes what is left, such as 64 classes
+// with many thresholds).
+static bool rank_form(const pd_ctx *ctx, const pd_train_params *p, const PropSrc *prop) {
+  if (prop) {  // proposals are clamped to the network's bounds: they must be these
+    const int D = ctx->cfg.feat_dim;
+    if (prop->lo[D] != (float)p->thr_low || prop->span[D] != (float)((int64_t)p->thr_up - p->thr_low) ||
+        p->thr_low < -(1 << 23) || p->thr_up > (1 << 23))
+      return false;
+  }
+  const int64_t lo = p->thr_low, hi = p->thr_up, span = hi - lo;
+  const int64_t fmax = ctx->cfg.feat_type == PD_FEAT_I16 ? 32767 : (1 << 29);
+  if (span < 0 || lo < -fmax || hi > fmax || span + 1 >= (int64_t)kRankWordsMax * 32) return false;
+  return rank_smem((uint32_t)ctx->cfg.n_classes, p->n_thresholds, (uint32_t)span, kRankThreads) <= kRankSmemMax;
+}
+
+// The class rows of the small-node kernel for a node with nc classes present (an
+// index into kSmallRows), or -1 when none fits.  A user feature's kernels are
+// compiled on first use: only two of them.
+constexpr int kSmallRows[4] = {4, 8, 16, 32};
+static int small_bucket(const pd_ctx *ctx, const pd_train_params *p, uint32_t nc) {
+  const uint32_t span = (uint32_t)(p->thr_up - p->thr_low);
+  for (int b = is_user_plugin(ctx) ? 1 : 0; b < 4; b++) {
+    if (is_user_plugin(ctx) && b == 2) continue;
+    if ((int)nc <= kSmallRows[b])
+      return rank_smem(kSmallRows[b], p->n_thresholds, span, small_threads(kSmallRows[b])) <= kRankSmemMax ? b : -1;
+  }
+  return -1;
+}
+
 static DevSet devset(const pd_ctx *ctx) {
   DevSet d;
   d.magic = ctx->magic_tab.as<uint32_t>();
@@ -229,32 +269,59 @@ static int launch_candidates(pd_ctx *ctx, const pd_train_params *p, uint32_t tre
 }
 
 // Builds the work list of slots [0, n) whose samples are act[off[i], off[i+1])
-// and launches the histogram kernel.
+// and launches the histogram kernels.  With `split_slots` non-null, nodes whose
+// samples fit one work item get their split fused into the histogram kernel (multi
+// = 2, rows never written) and the other slots are returned for the split kernels;
+// h_class_tot: their class totals [n][K] on the host.
 template <class P>
-// With `split_slots` non-null, nodes whose samples fit one work item get their
-// split fused into the histogram kernel (multi = 2, rows never written) and the
-// other slots are returned for the split kernels.
 static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *off, uint32_t n,
                        const SampleRec *d_rec, uint64_t *n_items_out, cudaEvent_t ev_before = nullptr,
                        cudaEvent_t ev_after = nullptr, std::vector<uint32_t> *split_slots = nullptr,
-                       const uint32_t *d_class_tot = nullptr, const uint32_t *d_ord = nullptr) {
+                       const uint32_t *d_class_tot = nullptr, const uint32_t *h_class_tot = nullptr,
+                       const uint32_t *d_ord = nullptr, const PropSrc *prop = nullptr) {
   using FeatT = typename P::feat_t;
   const uint32_t F = p->n_features, T = p->n_thresholds, K = ctx->cfg.n_classes;
   const uint32_t tiles = (F + kTileF - 1) / kTileF;
   PD_CHECK(ctx->chunk >= 1 && ctx->chunk <= kMaxChunk, PD_ERR_INVALID, "chunk %u outside [1,%u]", ctx->chunk, kMaxChunk);
-  // the work list is written straight into pinned staging (sized by a first
-  // pass); for a persistent launch it is ordered largest item first (by the
-  // power of two of its sample count, stable), so the last items to start are
-  // the short ones
+  const bool rank = rank_form(ctx, p, prop);
+  const uint32_t span = rank ? (uint32_t)(p->thr_up - p->thr_low) : 0u;
+  // Samples per work item: the chunk, or less when the level has too few tiles to
+  // fill the GPU (four items a resident CTA, at least kMinChunk samples each: the
+  // set-up of a tile costs about as much as 200 samples).  64 maps of 160x120 with
+  // 200 candidates: the root's 8 CTAs of 16384 samples took 0.33 ms, its 500 of 256
+  // take 0.05 ms.
+  constexpr uint64_t kMinChunk = 256;
+  const uint64_t total = off[n] - off[0];
+  const uint64_t want = (total * tiles + 4ull * ctx->n_sms - 1) / (4ull * ctx->n_sms);
+  const uint64_t chunk = rank ? std::min<uint64_t>(ctx->chunk, std::max(kMinChunk, (want + 31) / 32 * 32)) : ctx->chunk;
+  // Per node: fused (a small-node launch of its class count in the rank-table form,
+  // an item with multi = 2 in the search form) or chunked.  The list is written
+  // straight into pinned staging: the items of k_hist -- for a persistent launch
+  // largest first (by the power of two of their sample count, stable), so that the
+  // last to start are the short ones -- then the small nodes by class bucket.
   const bool persist = ctx->persist;
   auto bucket = [](uint64_t cnt) { return cnt ? 63 - __builtin_clzll(cnt) : 0; };  // floor(log2), <= 15
-  uint64_t n_items = 0, pos[17] = {};
+  std::vector<int8_t> kind(n);  // -2 empty, -1 chunked, -3 fused in k_hist, b >= 0 small bucket
+  uint64_t n_small[4] = {}, n_big = 0, pos[17] = {};
   for (uint32_t i = 0; i < n; i++) {
-    const uint64_t cnt = off[i + 1] - off[i];
-    const uint64_t chunks = (cnt + ctx->chunk - 1) / ctx->chunk;
-    n_items += chunks * tiles;
-    for (uint64_t c = 0; persist && c < chunks; c++)
-      pos[bucket(std::min<uint64_t>(cnt - c * ctx->chunk, ctx->chunk))] += tiles;
+    const uint64_t cnt = off[i + 1] - off[i], chunks = (cnt + chunk - 1) / chunk;
+    int k = cnt ? -1 : -2;
+    if (split_slots && chunks == 1 && cnt <= ctx->fuse_max) {
+      if (!rank) {
+        k = -3;
+      } else {
+        uint32_t nc = 0;
+        for (uint32_t l = 0; l < K; l++) nc += h_class_tot[(size_t)i * K + l] != 0u;
+        k = small_bucket(ctx, p, nc);
+      }
+    }
+    kind[i] = (int8_t)k;
+    if (k >= 0) {
+      n_small[k]++;
+      continue;
+    }
+    n_big += chunks;
+    for (uint64_t c = 0; persist && c < chunks; c++) pos[bucket(std::min<uint64_t>(cnt - c * chunk, chunk))]++;
   }
   uint64_t acc = 0;
   for (int b = 15; persist && b >= 0; b--) {  // start of each bucket, largest first
@@ -262,40 +329,47 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
     pos[b] = acc;
     acc += c;
   }
+  uint64_t at[4], n_items = n_big;
+  for (int b = 0; b < 4; b++) {
+    at[b] = n_items;
+    n_items += n_small[b];
+  }
   PD_TRY(ctx->h_items.ensure(std::max<uint64_t>(1, n_items) * sizeof(WorkItem)));
   WorkItem *items = ctx->h_items.as<WorkItem>();
   uint64_t ni = 0;
   std::vector<uint32_t> zero;
+  bool any_fused = false;
   for (uint32_t i = 0; i < n; i++) {
     const uint64_t b = off[i], e = off[i + 1];
-    const uint64_t cnt = e - b;
-    if (!cnt) {
+    if (kind[i] == -2) {
       zero.push_back(i);
       if (split_slots) split_slots->push_back(i);
       continue;
     }
-    const uint64_t chunks = (cnt + ctx->chunk - 1) / ctx->chunk;
+    WorkItem w;
+    memset(&w, 0, sizeof(w));
+    w.slot = i;
+    if (kind[i] >= 0) {
+      w.begin = (uint32_t)b;
+      w.end = (uint32_t)e;
+      w.multi = 2;
+      items[at[kind[i]]++] = w;
+      continue;
+    }
+    const uint64_t chunks = (e - b + chunk - 1) / chunk;
     if (chunks > 1) zero.push_back(i);
-    const bool fused = split_slots && chunks == 1 && cnt <= ctx->fuse_max;
-    if (split_slots && !fused) split_slots->push_back(i);
+    any_fused |= kind[i] == -3;
+    if (split_slots && kind[i] != -3) split_slots->push_back(i);
+    w.multi = chunks > 1 ? 1u : (kind[i] == -3 ? 2u : 0u);
     for (uint64_t c = 0; c < chunks; c++) {
-      const uint32_t cb = (uint32_t)(b + c * ctx->chunk);
-      const uint32_t ce = (uint32_t)std::min<uint64_t>(e, b + (c + 1) * ctx->chunk);
-      for (uint32_t t = 0; t < tiles; t++) {
-        WorkItem w;
-        memset(&w, 0, sizeof(w));
-        w.slot = i;
-        w.tile = t;
-        w.begin = cb;
-        w.end = ce;
-        w.multi = chunks > 1 ? 1u : (fused ? 2u : 0u);
-        items[persist ? pos[bucket(ce - cb)]++ : ni] = w;
-        ni++;
-      }
+      w.begin = (uint32_t)(b + c * chunk);
+      w.end = (uint32_t)std::min<uint64_t>(e, b + (c + 1) * chunk);
+      items[persist ? pos[bucket(w.end - w.begin)]++ : ni] = w;
+      ni++;
     }
   }
-  *n_items_out = ni;
-  PD_TRY(ctx->items.ensure(std::max<size_t>(1, ni) * sizeof(WorkItem)));
+  *n_items_out = n_items * tiles;
+  PD_TRY(ctx->items.ensure(std::max<size_t>(1, n_items) * sizeof(WorkItem)));
   PD_TRY(ctx->zero_slots.ensure(std::max<size_t>(1, zero.size()) * 4));
   const uint64_t per_slot = (uint64_t)K * T * F;
   if (!zero.empty()) {
@@ -305,15 +379,12 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
     PD_CUDA(cudaGetLastError());
   }
   if (!zero.empty()) ctx->launches++;
-  if (!ni) {
+  if (!n_items) {
     if (ev_before) PD_CUDA(cudaEventRecord(ev_before, ctx->stream));
     if (ev_after) PD_CUDA(cudaEventRecord(ev_after, ctx->stream));
     return PD_OK;
   }
-  PD_CUDA(h2d(ctx, ctx->items.ptr, items, ni * sizeof(WorkItem)));
-  bool any_fused = false;
-  for (uint64_t k = 0; k < ni; k++) any_fused |= items[k].multi == 2;
-  const size_t smem = hist_smem(ctx, T, any_fused);
+  PD_CUDA(h2d(ctx, ctx->items.ptr, items, n_items * sizeof(WorkItem)));
   FusedSplit fs;
   memset(&fs, 0, sizeof(fs));
   if (split_slots) {
@@ -340,22 +411,31 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
     fs.ord = d_ord;
   }
   HistGrid g;
+  memset(&g, 0, sizeof(g));
   g.ds = devset(ctx);
   g.rec = d_rec;
   g.items = ctx->items.as<WorkItem>();
-  g.n_items = ni;
+  g.n_items = n_big;
+  g.tiles = tiles;
+  for (int b = 0; b < 4; b++) {
+    g.small[b].nc = kSmallRows[b];
+    g.small[b].n_items = n_small[b];
+    g.small[b].smem = n_small[b] ? rank_smem(kSmallRows[b], T, span, small_threads(kSmallRows[b])) : 0;
+  }
   g.cand_feat = ctx->cand_feat.ptr;
   g.cand_thr = ctx->cand_thr.ptr;
   g.hist = ctx->hist.as<uint32_t>();
   g.F = F;
   g.T = T;
   g.K = K;
-  g.TP = padded_rows(T);
-  g.smem = smem;
+  g.TP = rank ? 0 : padded_rows(T);
+  g.thr_lo = p->thr_low;
+  g.thr_span = span;
+  g.smem = rank ? rank_smem(K, T, span, kRankThreads) : hist_smem(ctx, T, any_fused);
   g.fs = fs;
   g.ev_before = ev_before;
   g.queue = nullptr;
-  if (persist && ni < 0x7fffffffull) {
+  if (persist && n_big * tiles < 0x7fffffffull) {
     PD_TRY(ctx->hist_queue.ensure(16));
     g.queue = ctx->hist_queue.as<unsigned>();
   }
@@ -594,9 +674,9 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
       std::vector<uint64_t> off(cur_off.begin() + s0, cur_off.begin() + s0 + ns + 1);
       PD_CUDA(cudaEventRecord(ev[0], st));
       const uint32_t *d_ord = nullptr;
+      PropSrc src;
       if (prop) {
         // the network's mixture for every node of the slice, then the table drawn from it
-        PropSrc src;
         PD_TRY(proposer_infer(prop, d_ctot.as<uint32_t>(), ns, depth, n_prop, &src));
         PD_TRY(launch_candidates<P>(ctx, p, tree_id, d_nodes.as<int32_t>(), ns, ctx->cand_order, &d_ord, &src));
       } else {
@@ -607,7 +687,7 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
       uint64_t n_items = 0;
       std::vector<uint32_t> split_slots;
       PD_TRY(launch_hist<P>(ctx, p, off.data(), ns, ctx->act_rec[cur].as<SampleRec>(), &n_items, ev[6], ev[2],
-                            &split_slots, d_ctot.as<uint32_t>(), d_ord));
+                            &split_slots, d_ctot.as<uint32_t>(), ctot.data(), d_ord, prop ? &src : nullptr));
       stats.hist_launches++;
       stats.hist_bytes += hist_algorithmic_bytes(ctx, p, off.back() - off.front(), ns, (uint32_t)split_slots.size(),
                                                  image_bytes);

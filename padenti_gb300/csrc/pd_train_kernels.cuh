@@ -20,7 +20,26 @@
 
 namespace pd {
 
-constexpr int kHistThreads = 256;  // 8 warps, each on its own samples
+constexpr int kHistThreads = 256;  // 8 warps, each on its own samples (search form)
+// Rank-table form, large nodes: one CTA of 16 warps per SM shares one histogram, so
+// that most of the SM's 256 KB stays L1 for the probe gathers, which bound the loop:
+// root of 200 640x480 depth maps (8.2e8 evaluations), one CTA of 512 threads 1.70 ms
+// (L1 hit rate 82 %, 18 cycles per 32 evaluations), two of 256 2.58 ms (35 %, 26
+// cycles); 768 and 1024 threads were 7 and 18 % slower over a tree (more windows
+// in flight than L1 holds).  The search form's two CTAs: 2.68 ms.
+constexpr int kRankThreads = 512;
+constexpr int kRankCtas = 1;
+// Small nodes (split fused), by class rows: 16 warps per SM, in as many CTAs as the
+// histogram rows leave L1 for, so that the barriers of one item hide behind the
+// others (a depth-16 tree on 600 maps, all histogram launches: 114.8 ms; 8 rows in
+// three CTAs of 128 threads and 16 rows in two: 142.5 ms).
+PD_HD constexpr int small_threads(int NC) { return NC <= 4 ? 128 : NC <= 8 ? 256 : 512; }
+PD_HD constexpr int small_ctas(int NC) { return NC <= 4 ? 4 : NC <= 8 ? 2 : 1; }
+constexpr int kSmallSpi = 4;  // samples per warp iteration (8 measured the same, with more registers)
+constexpr uint32_t kRankWordsMax = 64;  // rank-table words per column: threshold ranges up to 2046
+// Table words per column for thresholds in [lo, lo + span] (responses reach span + 1).
+PD_HD constexpr uint32_t rank_words(uint32_t span) { return (span + 1) / 32 + 1; }
+PD_HD constexpr int hist_threads(uint32_t TP) { return TP ? kHistThreads : kRankThreads; }
 constexpr int kScanItems = 4096;   // active samples per scan block (256 threads x 16)
 // FP32 gain window rechecked in FP64.  Each FP32 entropy term -p log2 p (fast
 // reciprocal and log2) is within about 2e-7 of its exact value and each of the
@@ -51,13 +70,14 @@ struct CandBounds {
   uint32_t f_base;  // candidate f of a table is the node's candidate f_base + f (candidate-sharded training)
 };
 
-// One histogram work item: candidates [tile*64, tile*64+64) of frontier slot
-// `slot` over the active samples act[begin, end) (end - begin <= 65535).
+// One histogram work item: the active samples act[begin, end) of frontier slot
+// `slot` (end - begin <= 65535).  Every tile of 64 candidates of the slot is one CTA
+// of the item: CTA b of a launch takes tile b % tiles of item b / tiles.
 // multi = 0: the only work item of its rows, stores them; 1: other work items
 // add into the same rows (atomics); 2: the only work item of its rows, and the
 // node's split is fused into the kernel (no rows are written).
 struct WorkItem {
-  uint32_t slot, tile, begin, end, multi, pad0, pad1, pad2;
+  uint32_t slot, tile, begin, end, multi, pad0, pad1, pad2;  // tile: set by the CTA
 };
 
 struct DevSet {
@@ -606,6 +626,257 @@ PD_D void hist_samples(const DevSet &ds, const SampleRec *__restrict__ rec, cons
   }
 }
 
+// ---- rank-table form -------------------------------------------------------
+// For threshold ranges up to 2046 the place of a response among the thresholds is
+// looked up instead of searched (36 instructions per evaluation in place of 69): per candidate, word k of a table holds a bit per
+// value of [lo + 32k, lo + 32k + 32) that is a threshold, and the number of
+// distinct thresholds below lo + 32k (as the byte offset of the histogram row and
+// lane).  The place is that number plus the population count of the bits below
+// the response: one 64-bit shared load and ten instructions, where the search
+// took three register levels, three dependent loads and nineteen.  It counts
+// distinct thresholds; a candidate's duplicates (bit t of `first` clear) share
+// their predecessor's counts and are put back when the rows are read.
+struct RankTab {
+  uint2 *tab;             // [2][words][32]: {bits, row and lane offset in bytes}
+  uint32_t words;         // per column
+  uint32_t *first;        // [64][first_words]: bit t set when sorted threshold t differs from t - 1
+  uint32_t first_words;
+  int32_t lo, cap;        // responses are taken as clamp(r - lo, 0, cap), cap = hi - lo + 1
+};
+
+// The tables of one tile (all threads; ends with a barrier).  Thread (column c,
+// part) walks consecutive sorted thresholds, then the part's table words.
+template <int NT, typename FeatT>
+PD_D void build_rank_tab(const RankTab &rt, const FeatT *__restrict__ thr, uint32_t F, uint32_t T, uint32_t f0) {
+  constexpr uint32_t kParts = NT / kTileF;
+  __shared__ uint32_t s_part[kParts][kTileF];
+  const uint32_t c = threadIdx.x & (kTileF - 1), part = threadIdx.x / kTileF;
+  for (uint32_t i = threadIdx.x; i < rt.words * 32; i += NT) reinterpret_cast<uint4 *>(rt.tab)[i] = make_uint4(0, 0, 0, 0);
+  for (uint32_t i = threadIdx.x; i < kTileF * rt.first_words; i += NT) rt.first[i] = 0u;
+  __syncthreads();
+  uint2 *col = rt.tab + (c >> 5) * rt.words * 32 + (c & 31);
+  if (f0 + c < F) {
+    const uint32_t per = (T + kParts - 1) / kParts, tb = part * per, te = min(T, tb + per);
+    const FeatT *p = thr + f0 + c;
+    int32_t prev = tb > 0 && tb < te ? (int32_t)ldg(p + (size_t)(tb - 1) * F) : 0;
+    for (uint32_t t = tb; t < te; t++) {
+      const int32_t v = (int32_t)ldg(p + (size_t)t * F);
+      if (t == 0 || v != prev) {
+        const uint32_t b = (uint32_t)(v - rt.lo);
+        atomicOr(&col[(b >> 5) * 32].x, 1u << (b & 31));
+        atomicOr(&rt.first[c * rt.first_words + (t >> 5)], 1u << (t & 31));
+      }
+      prev = v;
+    }
+  }
+  __syncthreads();
+  const uint32_t per = (rt.words + kParts - 1) / kParts, wb = part * per, we = min(rt.words, wb + per);
+  uint32_t n = 0;
+  for (uint32_t k = wb; k < we; k++) n += __popc(col[k * 32].x);
+  s_part[part][c] = n;
+  __syncthreads();
+  uint32_t base = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < kParts; q++) base += q < part ? s_part[q][c] : 0u;
+  for (uint32_t k = wb; k < we; k++) {
+    const uint32_t bits = col[k * 32].x;
+    col[k * 32].y = base * 128u + (c & 31) * 4u;
+    base += __popc(bits);
+  }
+  __syncthreads();
+}
+
+PD_D uint32_t low_mask(uint32_t n) {  // bits below n mod 32
+#if defined(__CUDA_ARCH__)
+  uint32_t m;
+  asm("bmsk.wrap.b32 %0, 0, %1;" : "=r"(m) : "r"(n));
+  return m;
+#else
+  return (1u << (n & 31)) - 1u;
+#endif
+}
+// Byte offset (row and lane) of the response's histogram word in its class block.
+template <bool SMALL>
+PD_D uint32_t rank_offset(int32_t r, int32_t lo, int32_t cap, const uint2 *col) {
+  uint32_t v;
+  if constexpr (SMALL) v = (uint32_t)max(min(r - lo, cap), 0);
+  else v = (uint32_t)(min(max(r, lo), lo + cap) - lo);
+  const uint2 e = *reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(col) + (v & ~31u) * 8u);
+  return e.y + (uint32_t)__popc(e.x & low_mask(v)) * 128u;
+}
+
+// Staged words of a plugin without its own form, and of samples or tiles that
+// do not take it: position, preload words, size, image pointer, map offset.
+template <class P>
+struct PlainStage {
+  using Cand = typename P::Cand;
+  static PD_D Cand candidate(const typename P::feat_t *f) { return P::candidate(f); }
+  static PD_D bool stage(const ImageRef<typename P::img_t> &im, int32_t x, int32_t y, const uint32_t *pre,
+                         uint64_t moff, uint32_t *w) {
+    const uint64_t p = (uint64_t)im.data;
+    w[0] = (uint32_t)x | ((uint32_t)y << 16);
+    w[1] = pre[0];
+    w[2] = (uint32_t)im.w | ((uint32_t)im.h << 16);
+    w[4] = (uint32_t)p;
+    w[5] = (uint32_t)(p >> 32);
+    if constexpr (P::kUsesTree) {
+      w[6] = (uint32_t)moff;
+      w[7] = (uint32_t)(moff >> 32);
+    } else {
+      w[6] = P::kPreWords > 1 ? pre[P::kPreWords - 1] : 0u;
+      w[7] = 0u;
+    }
+    return true;
+  }
+  static PD_D typename P::feat_t eval(const DevSet &ds, const uint4 &a, const uint4 &b, const Cand &c) {
+    ImageRef<typename P::img_t> im;
+    im.data = staged_ptr<typename P::img_t>(b.x, b.y);
+    im.w = (int32_t)(a.z & 0xffffu);
+    im.h = (int32_t)(a.z >> 16);
+    im.magic = ds.magic;
+    if constexpr (P::kUsesTree) attach_tree<P>(im, ds, (uint64_t)b.z | ((uint64_t)b.w << 32));
+    const uint32_t pre[2] = {a.y, b.z};
+    return P::template eval_train<false>(P::prepare(im, (int32_t)(a.x & 0xffffu), (int32_t)(a.x >> 16), pre), c);
+  }
+};
+// The plugin's own staged form.
+template <class P>
+struct FastStage {
+  using Cand = typename P::FastCand;
+  static PD_D Cand candidate(const typename P::feat_t *f) { return P::fast_candidate(f); }
+  static PD_D bool stage(const ImageRef<typename P::img_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint64_t,
+                         uint32_t *w) {
+    return P::fast_stage(im, x, y, pre, w);
+  }
+  static PD_D typename P::feat_t eval(const DevSet &, const uint4 &a, const uint4 &b, const Cand &c) {
+    return P::eval_fast(a, b, c);
+  }
+};
+
+// Candidate `col` of the tile's slot (feature values 0 past the last column).
+template <class P, class S>
+PD_D typename S::Cand tile_candidate(const typename P::feat_t *__restrict__ feat, uint32_t F, uint32_t col) {
+  typename P::feat_t fv[P::kFeatDim];
+#pragma unroll
+  for (int d = 0; d < P::kFeatDim; d++) fv[d] = col < F ? feat[(size_t)d * F + col] : (typename P::feat_t)0;
+  return S::candidate(fv);
+}
+
+// The table arrays laid out from `at` (16-byte aligned) on.
+PD_D RankTab rank_tab(uint32_t *at, uint32_t T, int32_t lo, uint32_t span) {
+  RankTab rt;
+  rt.words = rank_words(span);
+  rt.first_words = (T + 31) / 32;
+  rt.lo = lo;
+  rt.cap = (int32_t)span + 1;
+  rt.first = at;
+  rt.tab = reinterpret_cast<uint2 *>(at + kTileF * rt.first_words);
+  return rt;
+}
+
+// The sample loop of the rank-table form.  A warp stages the words of up to 32
+// samples in its own shared memory, one lane a sample, then takes them SPI at a
+// time: two 128-bit broadcast loads bring a sample's words to all lanes (eight
+// shuffles before), every lane evaluates its two candidates, and the probe loads
+// of the SPI samples are in flight together.
+template <class P, class S, int SPI, int NT, class RowOf>
+PD_D void hist_samples_rank(const DevSet &ds, const SampleRec *__restrict__ rec, const WorkItem &w,
+                            const typename P::feat_t *__restrict__ feat, uint32_t F, uint32_t f0, char *sh_hist,
+                            const RankTab &rt, uint4 *sh_stage, uint32_t T, RowOf row_of) {
+  constexpr uint32_t kWarps = NT / 32;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const typename S::Cand ca = tile_candidate<P, S>(feat, F, f0 + lane), cb = tile_candidate<P, S>(feat, F, f0 + 32 + lane);
+  const uint2 *ta = rt.tab + lane, *tb = ta + rt.words * 32;
+  const int32_t lo = rt.lo, cap = rt.cap;
+  const uint32_t class_bytes = (T + 1) * 128;
+  uint4 *st = sh_stage + warp * 64;
+  // samples per warp batch: 32, or for a small item an equal share (rounded up to
+  // SPI) so that every warp of the CTA has samples
+  const uint32_t n_item = w.end - w.begin;
+  const uint32_t share = (n_item + kWarps - 1) / kWarps;
+  const uint32_t bs = share >= 32u ? 32u : (share + SPI - 1) / SPI * SPI;
+  for (uint32_t base = w.begin + warp * bs; base < w.end; base += bs * kWarps) {
+    const uint32_t n_here = min(bs, w.end - base);
+    bool ok = true;
+    if (lane < n_here) {
+      const uint4 r = ldg(reinterpret_cast<const uint4 *>(rec + base + lane));
+      const uint32_t imi = r.y & 0xffffffu;
+      const uint32_t wh = ds.img_wh[imi];
+      ImageRef<typename P::img_t> im;
+      im.data = reinterpret_cast<const typename P::img_t *>(ds.pixels + ds.img_off[imi]);
+      im.w = (int32_t)(wh & 0xffffu);
+      im.h = (int32_t)(wh >> 16);
+      const uint32_t pre[2] = {r.z, r.w};
+      uint64_t moff = 0;
+      if constexpr (P::kUsesTree) moff = ds.map_off ? ds.map_off[imi] : 0ull;
+      uint32_t v[8];
+      ok = S::stage(im, (int32_t)(r.x & 0xffffu), (int32_t)(r.x >> 16), pre, moff, v);
+      if (!P::kFastAlways && !ok) ok = !PlainStage<P>::stage(im, (int32_t)(r.x & 0xffffu), (int32_t)(r.x >> 16), pre, moff, v);
+      v[3] = row_of(r.y >> 24) * class_bytes;
+      st[2 * lane] = make_uint4(v[0], v[1], v[2], v[3]);
+      st[2 * lane + 1] = make_uint4(v[4], v[5], v[6], v[7]);
+    }
+    // samples whose words are plain ones (none for most plugins)
+    const uint32_t plain = P::kFastAlways ? 0u : __ballot_sync(0xffffffffu, !ok);
+    __syncwarp();
+    auto add = [&](uint32_t row, int32_t ra, int32_t rb) {
+      // Rank T (no threshold >= r) and the columns past F (no bits: rank 0) land in
+      // words that are never read.
+      atomicAdd(reinterpret_cast<uint32_t *>(sh_hist + row + rank_offset<P::kSmallResp>(ra, lo, cap, ta)), 1u);
+      atomicAdd(reinterpret_cast<uint32_t *>(sh_hist + row + rank_offset<P::kSmallResp>(rb, lo, cap, tb)), 0x10000u);
+    };
+    if (P::kFastAlways || plain == 0u) {
+      uint32_t i = 0;
+      for (; i + SPI <= n_here; i += SPI) {
+        int32_t ra[SPI], rb[SPI];
+        uint32_t row[SPI];
+#pragma unroll
+        for (int k = 0; k < SPI; k++) {
+          const uint4 a = st[2 * (i + k)], b = st[2 * (i + k) + 1];
+          row[k] = a.w;
+          ra[k] = (int32_t)S::eval(ds, a, b, ca);
+          rb[k] = (int32_t)S::eval(ds, a, b, cb);
+        }
+#pragma unroll
+        for (int k = 0; k < SPI; k++) add(row[k], ra[k], rb[k]);
+      }
+      for (; i < n_here; i++) {
+        const uint4 a = st[2 * i], b = st[2 * i + 1];
+        add(a.w, (int32_t)S::eval(ds, a, b, ca), (int32_t)S::eval(ds, a, b, cb));
+      }
+    } else {
+      const auto pa = tile_candidate<P, PlainStage<P>>(feat, F, f0 + lane);
+      const auto pb = tile_candidate<P, PlainStage<P>>(feat, F, f0 + 32 + lane);
+      for (uint32_t i = 0; i < n_here; i++) {
+        const uint4 a = st[2 * i], b = st[2 * i + 1];
+        if ((plain >> i) & 1u) add(a.w, (int32_t)PlainStage<P>::eval(ds, a, b, pa), (int32_t)PlainStage<P>::eval(ds, a, b, pb));
+        else add(a.w, (int32_t)S::eval(ds, a, b, ca), (int32_t)S::eval(ds, a, b, cb));
+      }
+    }
+    __syncwarp();  // the words are read before the next batch overwrites them
+  }
+}
+
+// The samples of a tile through the plugin's staged form where every candidate of
+// the tile allows it, else through the plain one.  row_of(class): the class's block
+// of the histogram.
+template <class P, int SPI, int NT, class RowOf>
+PD_D void hist_samples_tile(const DevSet &ds, const SampleRec *__restrict__ rec, const WorkItem &w,
+                            const typename P::feat_t *__restrict__ feat, uint32_t F, uint32_t f0, uint32_t *sh_hist,
+                            const RankTab &rt, uint32_t T, RowOf row_of) {
+  char *hb = reinterpret_cast<char *>(sh_hist);
+  uint4 *st = reinterpret_cast<uint4 *>(rt.tab + rt.words * 64);
+  if constexpr (P::kId == PD_PLUGIN_USER) {
+    hist_samples_rank<P, PlainStage<P>, SPI, NT>(ds, rec, w, feat, F, f0, hb, rt, st, T, row_of);
+  } else {
+    const uint32_t c = f0 + (threadIdx.x & (kTileF - 1));
+    if (__syncthreads_and(P::fast(tile_candidate<P, PlainStage<P>>(feat, F, c))))
+      hist_samples_rank<P, FastStage<P>, SPI, NT>(ds, rec, w, feat, F, f0, hb, rt, st, T, row_of);
+    else
+      hist_samples_rank<P, PlainStage<P>, 2, NT>(ds, rec, w, feat, F, f0, hb, rt, st, T, row_of);
+  }
+}
+
 // Split of a node whose samples all went through one work item, fused into the
 // histogram CTA: the tile histogram (packed pairs of 16-bit counters) is
 // prefix-summed in place over the ranks, so word (l, j, lane) holds the left
@@ -898,7 +1169,85 @@ PD_D void fused_split(const FusedSplit &fs, const WorkItem &w, uint32_t *sh_hist
   fs.out[slot] = o;
 }
 
-// One work item of the histogram kernel (the whole CTA).
+// Brings the rows of the tile's threshold permutation and column order to L2: the
+// fused split reads them at the end.
+PD_D void prefetch_fused(const FusedSplit &fs, const WorkItem &w, uint32_t f0, uint32_t F, uint32_t T) {
+  const uint32_t last = min(F - 1, f0 + kTileF - 1);  // the tile's last column
+  for (uint32_t t = threadIdx.x; t < T + 2; t += blockDim.x) {
+    if (t < T) {
+      const uint8_t *r = fs.perm + ((size_t)w.slot * T + t) * F;
+      prefetch_l2(r + f0);
+      prefetch_l2(r + last);
+    } else if (fs.ord) {
+      prefetch_l2(fs.ord + (size_t)w.slot * F + (t == T ? f0 : last));
+    }
+  }
+}
+
+// Zeroes the tile histogram; of a fused item only the rows of the classes present
+// in the node, which alone are counted and read.
+PD_D void zero_hist(const FusedSplit &fs, const WorkItem &w, uint32_t *sh_hist, uint32_t T, uint32_t K) {
+  if (w.multi == 2) {
+    for (uint32_t l = 0; l < K; l++)
+      if (fs.class_tot[(size_t)w.slot * K + l])
+        for (uint32_t j = threadIdx.x; j < (T + 1) * 32; j += blockDim.x) sh_hist[l * (T + 1) * 32 + j] = 0u;
+  } else {
+    for (uint32_t j = threadIdx.x; j < K * (T + 1) * 32; j += blockDim.x) sh_hist[j] = 0u;
+  }
+}
+
+// Adds (MULTI) or stores a packed count pair to columns f0 + c and f0 + 32 + c.
+PD_D void flush_pair(uint32_t *dst, uint32_t f0, uint32_t c, uint32_t F, bool multi, uint32_t va, uint32_t vb) {
+  if (f0 + c < F) {
+    if (!multi) *dst = va;
+    else if (va) atomicAdd(dst, va);
+  }
+  if (f0 + 32 + c < F) {
+    if (!multi) dst[32] = vb;
+    else if (vb) atomicAdd(dst + 32, vb);
+  }
+}
+
+// One tile of a work item of the rank-table form (the whole CTA).  Dynamic shared
+// memory: the histogram [K][T+1][32], the `first` bits, the table, the warps'
+// staged words.
+template <class P, int SPI>
+__device__ __forceinline__ void rank_item(const DevSet &ds, const SampleRec *__restrict__ rec, const WorkItem w,
+                                          const typename P::feat_t *__restrict__ cand_feat,
+                                          const typename P::feat_t *__restrict__ cand_thr, uint32_t *__restrict__ hist,
+                                          uint32_t F, uint32_t T, uint32_t K, int32_t lo, uint32_t span) {
+  using FeatT = typename P::feat_t;
+  constexpr int NT = kRankThreads;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint32_t *sh_hist = reinterpret_cast<uint32_t *>(smem_raw);
+  const uint32_t f0 = w.tile * kTileF;
+  const RankTab rt = rank_tab(sh_hist + (size_t)K * (T + 1) * 32, T, lo, span);
+  for (uint32_t j = threadIdx.x; j < K * (T + 1) * 32; j += NT) sh_hist[j] = 0u;
+  build_rank_tab<NT>(rt, cand_thr + (size_t)w.slot * T * F, F, T, f0);
+  hist_samples_tile<P, SPI, NT>(ds, rec, w, cand_feat + (size_t)w.slot * P::kFeatDim * F, F, f0, sh_hist, rt, T,
+                                [](uint32_t l) { return l; });
+  __syncthreads();
+  // rows of distinct thresholds -> sorted positions; a duplicate's row is empty
+  for (uint32_t q = threadIdx.x; q < T * 32; q += NT) {
+    const uint32_t j = q >> 5, c = q & 31, m = 0xffffffffu >> (31 - (j & 31));
+    const uint32_t *fa = rt.first + c * rt.first_words, *fb = fa + 32 * rt.first_words;
+    const uint32_t wa = fa[j >> 5] & m, wb = fb[j >> 5] & m;
+    uint32_t da = __popc(wa), db = __popc(wb);
+    for (uint32_t k = 0; k < j >> 5; k++) {
+      da += __popc(fa[k]);
+      db += __popc(fb[k]);
+    }
+    const bool oa = (wa >> (j & 31)) & 1u, ob = (wb >> (j & 31)) & 1u;
+    const uint32_t *ra = sh_hist + (oa ? da - 1 : 0u) * 32 + c, *rb = sh_hist + (ob ? db - 1 : 0u) * 32 + c;
+    uint32_t *dst = hist + ((size_t)w.slot * K * T + j) * F + f0 + c;
+    for (uint32_t l = 0; l < K; l++)
+      flush_pair(dst + (size_t)l * T * F, f0, c, F, w.multi != 0, oa ? ra[l * (T + 1) * 32] & 0xffffu : 0u,
+                 ob ? rb[l * (T + 1) * 32] >> 16 : 0u);
+  }
+}
+
+// One work item of the search form (the whole CTA): threshold ranges above the
+// rank table's, and shapes whose shared memory it does not fit.
 template <class P, uint32_t TP, int SPI>
 __device__ __forceinline__ void hist_item(const DevSet &ds, const SampleRec *__restrict__ rec, const WorkItem w,
                                           const typename P::feat_t *__restrict__ cand_feat,
@@ -906,7 +1255,6 @@ __device__ __forceinline__ void hist_item(const DevSet &ds, const SampleRec *__r
                                           uint32_t *__restrict__ hist, uint32_t F, uint32_t T, uint32_t K,
                                           const FusedSplit &fs) {
   using FeatT = typename P::feat_t;
-  using ImgT = typename P::img_t;
   constexpr int D = P::kFeatDim;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint32_t *sh_hist = reinterpret_cast<uint32_t *>(smem_raw);                   // [K][T+1][32] packed
@@ -915,7 +1263,7 @@ __device__ __forceinline__ void hist_item(const DevSet &ds, const SampleRec *__r
   // sh_g [T][64] gains, sh_nl [T][32] packed left totals
   float *sh_g = reinterpret_cast<float *>(sh_thr);
   uint32_t *sh_nl = reinterpret_cast<uint32_t *>(sh_g + (size_t)T * kTileF);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   const uint32_t f0 = w.tile * kTileF;
   const uint32_t fa = f0 + lane, fb = f0 + 32 + lane;
   const bool va = fa < F, vb = fb < F;
@@ -927,26 +1275,8 @@ __device__ __forceinline__ void hist_item(const DevSet &ds, const SampleRec *__r
     sh_thr[(c >> 5) * (TP * 32) + t * 32 + (c & 31)] =
         (t < T && ff < F) ? cand_thr[((size_t)w.slot * T + t) * F + ff] : max_of<FeatT>();
   }
-  if (w.multi == 2) {
-    // a fused item: only the rows of the classes present in the node are counted and read
-    for (uint32_t l = 0; l < K; l++)
-      if (fs.class_tot[(size_t)w.slot * K + l])
-        for (uint32_t j = threadIdx.x; j < (T + 1) * 32; j += blockDim.x) sh_hist[l * (T + 1) * 32 + j] = 0u;
-  } else {
-    for (uint32_t j = threadIdx.x; j < K * (T + 1) * 32; j += blockDim.x) sh_hist[j] = 0u;
-  }
-  if (w.multi == 2) {
-    // the fused split reads the tile's threshold permutation and column order
-    // at the end; bring them to L2 now
-    const uint32_t last = min(F - 1, f0 + kTileF - 1);  // the tile's last column
-    if (threadIdx.x < T) {
-      const uint8_t *r = fs.perm + ((size_t)w.slot * T + threadIdx.x) * F;
-      prefetch_l2(r + f0);
-      prefetch_l2(r + last);
-    } else if (fs.ord && threadIdx.x < T + 2) {
-      prefetch_l2(fs.ord + (size_t)w.slot * F + (threadIdx.x == T ? f0 : last));
-    }
-  }
+  zero_hist(fs, w, sh_hist, T, K);
+  if (w.multi == 2) prefetch_fused(fs, w, f0, F, T);
   typename P::Cand ca, cb;
   {
     FeatT fva[D], fvb[D];
@@ -972,39 +1302,33 @@ __device__ __forceinline__ void hist_item(const DevSet &ds, const SampleRec *__r
     for (uint32_t q = threadIdx.x; q < T * 32; q += blockDim.x) {
       const uint32_t v = sh_hist[l * (T + 1) * 32 + q];
       const uint32_t c = q & 31;
-      uint32_t *dst = hist + ((size_t)w.slot * K * T + l * T + (q >> 5)) * F + f0 + c;
-      if (f0 + c < F) {
-        if (w.multi) {
-          if (v & 0xffffu) atomicAdd(dst, v & 0xffffu);
-        } else {
-          *dst = v & 0xffffu;
-        }
-      }
-      if (f0 + 32 + c < F) {
-        if (w.multi) {
-          if (v >> 16) atomicAdd(dst + 32, v >> 16);
-        } else {
-          dst[32] = v >> 16;
-        }
-      }
+      flush_pair(hist + ((size_t)w.slot * K * T + l * T + (q >> 5)) * F + f0 + c, f0, c, F, w.multi != 0, v & 0xffffu,
+                 v >> 16);
     }
   }
 }
 
-// The histogram kernel over a work list.  queue == null: one CTA per item
-// (blockIdx.x).  Otherwise a persistent grid (a few CTAs per SM) whose CTAs
-// take items k = 0, 1, ... in list order from the counter *queue (an atomic
-// add, no wait), so a list sorted largest first keeps every SM busy to the end.
+// The histogram kernel over a work list (every tile of every item, tiles of an item
+// side by side).  queue == null: one CTA per tile (blockIdx.x).  Otherwise a
+// persistent grid (a few CTAs per SM) whose CTAs take tiles k = 0, 1, ... in list
+// order from the counter *queue (an atomic add, no wait), so a list sorted largest
+// first keeps every SM busy to the end.
+// TP = 0: the rank-table form, for thresholds in [lo, lo + span].
 template <class P, uint32_t TP, int SPI>
-__global__ void __launch_bounds__(kHistThreads, SPI <= 2 ? 3 : 2) k_hist(DevSet ds, const SampleRec *__restrict__ rec,
-                                                       const WorkItem *__restrict__ items, uint32_t n_items,
-                                                       unsigned *__restrict__ queue,
-                                                       const typename P::feat_t *__restrict__ cand_feat,
-                                                       const typename P::feat_t *__restrict__ cand_thr,
-                                                       uint32_t *__restrict__ hist, uint32_t F,
-                                                       uint32_t T, uint32_t K, FusedSplit fs) {
+__global__ void __launch_bounds__(hist_threads(TP), TP == 0 ? kRankCtas : SPI <= 2 ? 3 : 2)
+    k_hist(DevSet ds, const SampleRec *__restrict__ rec, const WorkItem *__restrict__ items, uint32_t n_items,
+           unsigned *__restrict__ queue, const typename P::feat_t *__restrict__ cand_feat,
+           const typename P::feat_t *__restrict__ cand_thr, uint32_t *__restrict__ hist, uint32_t F, uint32_t T,
+           uint32_t K, FusedSplit fs, int32_t lo, uint32_t span) {
+  const uint32_t tiles = (F + kTileF - 1) / kTileF;
+  auto item = [&](uint32_t k) {
+    WorkItem w = items[k / tiles];
+    w.tile = k % tiles;
+    if constexpr (TP == 0) rank_item<P, SPI>(ds, rec, w, cand_feat, cand_thr, hist, F, T, K, lo, span);
+    else hist_item<P, TP, SPI>(ds, rec, w, cand_feat, cand_thr, hist, F, T, K, fs);
+  };
   if (queue == nullptr) {
-    hist_item<P, TP, SPI>(ds, rec, items[blockIdx.x], cand_feat, cand_thr, hist, F, T, K, fs);
+    item(blockIdx.x);
     return;
   }
   __shared__ uint32_t s_next;
@@ -1013,10 +1337,332 @@ __global__ void __launch_bounds__(kHistThreads, SPI <= 2 ? 3 : 2) k_hist(DevSet 
     __syncthreads();
     const uint32_t k = s_next;
     __syncthreads();  // read by every thread before thread 0 takes the next item
-    if (k >= n_items) return;
-    hist_item<P, TP, SPI>(ds, rec, items[k], cand_feat, cand_thr, hist, F, T, K, fs);
+    if (k >= n_items * tiles) return;
+    item(k);
     __syncthreads();  // the item's shared memory is free again
   }
+}
+
+// The winner over the tiles of a node (one warp; every tile's part is visible).
+PD_D void pick_tiles(const FusedSplit &fs, uint32_t slot, uint32_t F, uint32_t K) {
+  const uint32_t lane = threadIdx.x & 31;
+  const SplitPart *pb = fs.part_best + (size_t)slot * fs.tiles;
+  double g = -DBL_MAX;
+  long long idx = LLONG_MAX;
+  uint32_t at = 0;
+  for (uint32_t i = lane; i < fs.tiles; i += 32) {
+    const double gi = __ldcg(&pb[i].gain);
+    const long long ii = __ldcg(&pb[i].idx);
+    if (gi > g || (gi == g && ii < idx)) {
+      g = gi;
+      idx = ii;
+      at = i;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double og = __shfl_xor_sync(0xffffffffu, g, o);
+    const long long oi = __shfl_xor_sync(0xffffffffu, idx, o);
+    const uint32_t oa = __shfl_xor_sync(0xffffffffu, at, o);
+    if (og > g || (og == g && oi < idx)) {
+      g = og;
+      idx = oi;
+      at = oa;
+    }
+  }
+  SplitOut o;
+  o.t = o.f = o.j = o.col = -1;
+  o.gain = 0.0;
+  if (idx != LLONG_MAX) {
+    o.t = (int32_t)(idx / F);
+    o.f = (int32_t)(idx % F);
+    o.j = __ldcg(&pb[at].j);
+    o.col = __ldcg(&pb[at].col);
+    o.gain = g;
+    for (uint32_t l = lane; l < K; l += 32)
+      fs.out_cl[(size_t)slot * K + l] = __ldcg(fs.part_cl + ((size_t)slot * fs.tiles + at) * K + l);
+  }
+  if (lane == 0) fs.out[slot] = o;
+}
+
+// Histogram and split of one tile of a small node (at most NC classes present, all
+// samples in one item): the rank-table sample loop into [NC][T+1][32] counters of
+// the classes present, then the split from them.
+//
+// Thread (column c, half of its distinct thresholds) walks its rows with the class
+// counts in registers: no prefix pass, no gain or total arrays.  The FP32 filter is
+// fused_split's (same table, same order of additions, same window); a thread keeps
+// its best position with its counts and its second best, so that one exact FP64
+// evaluation settles it unless the second lies in the window too, and then the
+// thread walks again.
+template <class P, int NC>
+__global__ void __launch_bounds__(small_threads(NC), small_ctas(NC))
+    k_hist_small(DevSet ds, const SampleRec *__restrict__ rec, const WorkItem *__restrict__ items,
+                 const typename P::feat_t *__restrict__ cand_feat, const typename P::feat_t *__restrict__ cand_thr,
+                 uint32_t F, uint32_t T, uint32_t K, FusedSplit fs, int32_t lo, uint32_t span) {
+  constexpr int kSmallThreads = small_threads(NC);
+  constexpr uint32_t kParts = kSmallThreads / kTileF;  // threads per candidate column
+  constexpr bool kPrefix = kParts > 2;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ uint32_t s_tot[NC];
+  __shared__ uint8_t s_map[PD_MAX_CLASSES], s_cls[NC];
+  __shared__ uint32_t s_nc;
+  __shared__ float s_max[kSmallThreads / 32];
+  __shared__ unsigned long long s_key, s_idx;
+  __shared__ double s_gain;
+  __shared__ int s_j, s_col;
+  __shared__ bool s_last;
+  uint32_t *sh_hist = reinterpret_cast<uint32_t *>(smem_raw);
+  WorkItem w = items[blockIdx.x / fs.tiles];
+  w.tile = blockIdx.x % fs.tiles;
+  const uint32_t slot = w.slot, f0 = w.tile * kTileF, TS = T + 1;
+  const uint32_t lane = threadIdx.x & 31;
+  const RankTab rt = rank_tab(sh_hist + (size_t)NC * TS * 32, T, lo, span);
+  if (threadIdx.x < 32) {
+    // the classes present, in class order
+    uint32_t nc = 0;
+    for (uint32_t l0 = 0; l0 < K; l0 += 32) {
+      const uint32_t l = l0 + lane, tot = l < K ? fs.class_tot[(size_t)slot * K + l] : 0u;
+      const uint32_t m = __ballot_sync(0xffffffffu, tot != 0u);
+      const uint32_t i = nc + __popc(m & ((1u << lane) - 1u));
+      if (tot != 0u && i < NC) {
+        s_map[l] = (uint8_t)i;
+        s_cls[i] = (uint8_t)l;
+        s_tot[i] = tot;
+      }
+      nc += __popc(m);
+    }
+    if (lane >= nc && lane < NC) s_tot[lane] = 0u;
+    if (lane == 0) {
+      s_nc = nc;
+      s_key = 0ull;
+      s_idx = ~0ull;
+    }
+  }
+  for (uint32_t j = threadIdx.x; j < NC * TS * 32; j += kSmallThreads) sh_hist[j] = 0u;
+  prefetch_fused(fs, w, f0, F, T);
+  build_rank_tab<kSmallThreads>(rt, cand_thr + (size_t)slot * T * F, F, T, f0);
+  hist_samples_tile<P, kSmallSpi, kSmallThreads>(ds, rec, w, cand_feat + (size_t)slot * P::kFeatDim * F, F, f0, sh_hist, rt, T,
+                                         [&](uint32_t l) { return (uint32_t)s_map[l]; });
+  __syncthreads();
+
+  const uint32_t nc = s_nc, N = w.end - w.begin;
+  const uint32_t c = threadIdx.x & (kTileF - 1), part = threadIdx.x / kTileF;
+  const uint32_t *fw = rt.first + c * rt.first_words;
+  uint32_t D = 0;  // distinct thresholds of the column (0 past the last column)
+  for (uint32_t k = 0; k < rt.first_words; k++) D += __popc(fw[k]);
+  const bool ok = (uint64_t)N < fs.L_len;
+  if constexpr (kPrefix) {
+    // cumulative counts in place, a thread per (class, packed column)
+    for (uint32_t q = threadIdx.x; q < nc * 32; q += kSmallThreads) {
+      uint32_t *p = sh_hist + (q >> 5) * TS * 32 + (q & 31);
+      uint32_t run = 0, j = 0;
+      for (; j + 8 <= T; j += 8) {
+        uint32_t v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = p[(j + k) * 32];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          run += v[k];
+          p[(j + k) * 32] = run;
+        }
+      }
+      for (; j < T; j++) {
+        run += p[j * 32];
+        p[j * 32] = run;
+      }
+    }
+    __syncthreads();
+  }
+  // counts of row j, compact class i, at h[(i * TS + j) * 64]
+  const uint16_t *h = reinterpret_cast<const uint16_t *>(sh_hist) + (c & 31) * 2 + (c >> 5);
+  double best = -DBL_MAX;
+  long long best_idx = LLONG_MAX;
+  int best_j = -1;
+  uint32_t n_checked = 0;
+  if (ok && nc == 1) {
+    // A pure node: every exact gain is 0, so the lowest index t*F + f wins: the
+    // original threshold 0 of the tile's lowest original candidate.
+    const uint32_t f = f0 + c;
+    if (part == 0 && f < F)
+      atomicMin(&s_idx, ((unsigned long long)(fs.ord ? fs.ord[(size_t)slot * F + f] : f) << 8) | c);
+    __syncthreads();
+    const unsigned long long low = s_idx;
+    __syncthreads();
+    if (threadIdx.x == 0) s_idx = ~0ull;
+    __syncthreads();
+    if (part == 0 && c == (uint32_t)(low & 0xffu)) {
+      int row = -1;
+      for (uint32_t t = 0; t < T; t++) {
+        row += (fw[t >> 5] >> (t & 31)) & 1u;
+        if (fs.perm[((size_t)slot * T + t) * F + f] == 0) best_j = row;
+      }
+      best = 0.0;
+      best_idx = (long long)(low >> 8);
+    }
+  } else if (ok) {
+    const float *X = fs.xlog2;
+    const uint32_t per = (D + kParts - 1) / kParts, jb = min(D, part * per), je = min(D, jb + per);
+    uint32_t tot[NC];
+#pragma unroll
+    for (int l = 0; l < NC; l++) tot[l] = s_tot[l];
+    // walks rows [jb, je): visit(j, counts, left total, gain) at every row whose counts differ from the row before
+    auto walk = [&](auto visit) {
+      uint32_t cnt[NC], nL = 0;
+#pragma unroll
+      for (int l = 0; l < NC; l++) cnt[l] = 0u;
+      if constexpr (kPrefix) {
+        if (jb > 0 && jb < je) {
+#pragma unroll
+          for (int l = 0; l < NC; l++) nL += h[(l * TS + jb - 1) * 64];
+        }
+      } else {
+        for (uint32_t j = 0; j < jb; j++) {
+#pragma unroll
+          for (int l = 0; l < NC; l++) cnt[l] += h[(l * TS + j) * 64];
+        }
+#pragma unroll
+        for (int l = 0; l < NC; l++) nL += cnt[l];
+      }
+      for (uint32_t j = jb; j < je; j++) {
+        const uint32_t before = nL;
+        if constexpr (kPrefix) {
+          nL = 0;
+#pragma unroll
+          for (int l = 0; l < NC; l++) {
+            cnt[l] = h[(l * TS + j) * 64];
+            nL += cnt[l];
+          }
+        } else {
+#pragma unroll
+          for (int l = 0; l < NC; l++) {
+            const uint32_t x = h[(l * TS + j) * 64];
+            cnt[l] += x;
+            nL += x;
+          }
+        }
+        if (nL != before || j == 0) {
+          float sl = __ldg(X + nL), sr = __ldg(X + (N - nL));
+#pragma unroll
+          for (int l = 0; l < NC; l++) {
+            sl -= __ldg(X + cnt[l]);
+            sr -= __ldg(X + (tot[l] - cnt[l]));
+          }
+          visit(j, cnt, nL, -(sl + sr));
+        }
+      }
+    };
+    float g1 = -FLT_MAX, g2 = -FLT_MAX;
+    uint32_t j1 = 0, n1 = 0, cnt1[NC];
+    walk([&](uint32_t j, const uint32_t *cnt, uint32_t nL, float g) {
+      if (g > g1) {
+        g2 = g1;
+        g1 = g;
+        j1 = j;
+        n1 = nL;
+#pragma unroll
+        for (int l = 0; l < NC; l++) cnt1[l] = cnt[l];
+      } else {
+        g2 = fmaxf(g2, g);
+      }
+    });
+    float m = g1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) s_max[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSmallThreads / 32; i++) m = fmaxf(m, s_max[i]);
+    const float cut = m - fused_window(K, N);
+    if (g1 >= cut && j1 < je) {
+      const double *L = fs.L;
+      const double hp64 = fs.parent[slot];
+      auto recheck = [&](uint32_t j, const uint32_t *cnt, uint32_t nL) {
+        n_checked++;
+        const uint32_t nR = N - nL;
+        // both sides in one loop (two independent chains; each sums in class order)
+        const double Ll = L[nL], Lr = L[nR];
+        double sl = 0.0, sr = 0.0;
+#pragma unroll
+        for (int l = 0; l < NC; l++) {
+          const uint32_t cl = cnt[l], cr = tot[l] - cl;
+          if (cl != 0u && (uint64_t)cl * 1000000ull > nL) sl = dadd(sl, dmul((double)cl, dsub(Ll, L[cl])));
+          if (cr != 0u && (uint64_t)cr * 1000000ull > nR) sr = dadd(sr, dmul((double)cr, dsub(Lr, L[cr])));
+        }
+        const double g = dsub(hp64, ddiv(dadd(sl, sr), (double)N));
+        if (g < best) return;
+        // rows j..end-1 share these counts: the lowest original threshold of their
+        // sorted positions wins
+        uint32_t end = j + 1;
+        for (; end < D; end++) {
+          uint32_t x = 0;  // what row `end` adds
+          for (uint32_t l = 0; l < nc; l++) x += h[(l * TS + end) * 64];
+          if (x != (kPrefix ? nL : 0u)) break;
+        }
+        const uint32_t f = f0 + c;
+        uint32_t t = 0xffu, row = 0;  // row: rows begun up to position p
+        for (uint32_t p = 0; p < T; p++) {
+          row += (fw[p >> 5] >> (p & 31)) & 1u;
+          if (row > end) break;
+          if (row > j) t = min(t, (uint32_t)fs.perm[((size_t)slot * T + p) * F + f]);
+        }
+        const long long idx = (long long)t * F + (fs.ord ? fs.ord[(size_t)slot * F + f] : f);
+        if (g > best || idx < best_idx) {
+          best = g;
+          best_idx = idx;
+          best_j = (int)j;
+        }
+      };
+      if (g2 >= cut)
+        walk([&](uint32_t j, const uint32_t *cnt, uint32_t nL, float g) {
+          if (g >= cut) recheck(j, cnt, nL);
+        });
+      else
+        recheck(j1, cnt1, n1);
+    }
+  }
+  if (n_checked) atomicAdd(fs.rechecked, (unsigned long long)n_checked);
+  // the tile's best: largest gain (as an ordered integer), then the lowest index
+  const unsigned long long key = (unsigned long long)gain_order_key(best) ^ 0x8000000000000000ull;
+  const bool have = best_idx != LLONG_MAX;
+  if (have) atomicMax(&s_key, key);
+  __syncthreads();
+  const bool top = have && key == s_key;
+  if (top) atomicMin(&s_idx, (unsigned long long)best_idx);
+  __syncthreads();
+  const unsigned long long win = s_idx;
+  if (top && (unsigned long long)best_idx == win) {
+    s_gain = best;
+    s_j = best_j;
+    s_col = (int)c;
+  }
+  __syncthreads();
+  const size_t pi = (size_t)slot * fs.tiles + w.tile;
+  if (win != ~0ull)  // left counts of the winner, by original class
+    for (uint32_t l = threadIdx.x; l < K; l += kSmallThreads) {
+      uint32_t n = 0;
+      for (uint32_t i = 0; i < nc; i++)
+        if (s_cls[i] == l) {
+          const uint16_t *q = reinterpret_cast<const uint16_t *>(sh_hist) + (s_col & 31) * 2 + (s_col >> 5);
+          for (int j = kPrefix ? s_j : 0; j <= s_j; j++) n += q[(i * TS + j) * 64];
+        }
+      fs.part_cl[pi * K + l] = n;
+    }
+  if (threadIdx.x == 0) {
+    SplitPart pb;
+    pb.gain = win != ~0ull ? s_gain : -DBL_MAX;
+    pb.idx = win != ~0ull ? (long long)win : LLONG_MAX;
+    pb.j = s_j;
+    pb.col = win != ~0ull ? (int)(f0 + (uint32_t)s_col) : -1;
+    fs.part_best[pi] = pb;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(fs.done + slot, 1u) == fs.tiles - 1;
+  __syncthreads();
+  if (!s_last || threadIdx.x >= 32) return;
+  __threadfence();
+  pick_tiles(fs, slot, F, K);
 }
 
 static __global__ void k_zero_slots(uint32_t *__restrict__ hist, const uint32_t *__restrict__ slots, uint32_t n,

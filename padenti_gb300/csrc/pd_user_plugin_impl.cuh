@@ -72,6 +72,10 @@ struct UserPlugin {
   template <bool FAST = false>
   static PD_D feat_t eval_train(const Prep &p, const Cand &c) { return eval<FAST>(p, c); }
   static PD_D feat_t eval(const Prep &p, const feat_t *f) { return call(p, f); }
+  // The histogram kernel takes a user feature through its plain staged words
+  // (PlainStage, pd_train_kernels.cuh).
+  static constexpr bool kFastAlways = true;
+  static constexpr bool kSmallResp = false;  // a response may be any value of feat_t
 };
 
 }  // namespace pd
