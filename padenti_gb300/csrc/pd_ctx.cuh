@@ -88,7 +88,8 @@ struct pd_ctx {
   std::vector<float> h_post;
   bool forest_dirty = true;
   pd::DevBuf f_lc, f_feat, f_thr, f_post, f_meta;
-  pd::DevBuf f_cand;                   // NodeRec of every forest node (k_forest_nodes)
+  pd::DevBuf f_cand;                   // FastNode or NodeRec of every forest node
+  pd::DevBuf f_post4;                  // posteriors padded to four classes a word (k_pad_posteriors)
   uint64_t cand_version = ~0ull;       // forest_version f_cand was built for
   bool forest_fast = false;            // every node takes the plugin's fast path (built-in plugins)
   pd::DevBuf f_fast;                   // its device flag

@@ -10,12 +10,13 @@
 //   eval_train(prep, cand)   the same on the trainer's copy of the images, which
 //                            kTrainMapsZero plugins store with 0 replaced by the
 //                            background depth (equal responses, one test fewer);
-// and the histogram kernel's form of the same response, from per-sample words
-// that a warp stages in shared memory (word 3 is the kernel's):
-//   fast_candidate(f)        the constants of a candidate whose P::fast holds;
-//   fast_stage(im, x, y, pre, w)  fills the words of a sample; false where the
-//                            form does not hold (the sample takes eval_train);
-//   eval_fast(a, b, cand)    the response from words a = w[0..3], b = w[4..7];
+// and the form of the same response that the histogram and prediction kernels take
+// for candidates whose P::fast holds, from eight words per pixel (word 3 is the
+// kernel's; the histogram kernel stages them in shared memory):
+//   fast_candidate(f)        the constants of a candidate;
+//   fast_words(im, x, y, pre, w)  the words of a pixel;
+//   eval_fast<MAPPED>(a, b, cand)  the response from words a = w[0..3], b = w[4..7];
+//                            MAPPED: on the trainer's copy of the images;
 // and kOrderDim, the feature dims (kOrderDim, kOrderDim + 1) of its first probe
 // offset, by which the trainer orders a node's candidates.
 // eval(prep, f) runs all of it for a single evaluation.
@@ -128,7 +129,7 @@ struct OffsetConst {
 
 // The same rounding in one fused multiply-add.  With i = fl(1/d), u' = u + 1/4
 // sgn(u) and M = 3*2^22, fl(u' i + (M + x)) - M is x + round_half_away(u / d) for
-// |u| <= 2^21, d in [1, 65535] and 0 <= x < 2^16: floats in [2^23, 2^24) are the
+// |u| <= 2^21, |d| in [1, 65535] and 0 <= x < 2^16: floats in [2^23, 2^24) are the
 // integers, so the fused operation rounds the exact u' i + M + x once, to the
 // nearest integer.  |u|/d + 1/2 lies a multiple of 1/(2d) above an integer; the
 // quarter moves it to at least 1/(4d) from both ends of its unit interval, so no
@@ -149,7 +150,7 @@ PD_D uint32_t fast_coord(float u, float inv_d, float base) {
   return 0u;
 #endif
 }
-PD_D float inv_depth(uint32_t d) {
+PD_D float inv_depth(int32_t d) {
 #if defined(__CUDA_ARCH__)
   return __frcp_rn((float)d);
 #else
@@ -255,8 +256,7 @@ struct DepthDiff2 {
   template <bool FAST = false>
   static PD_D int32_t eval_train(const Prep &p, const Cand &c) { return eval<FAST, true>(p, c); }
   static PD_D int32_t eval(const Prep &p, const int32_t *f) { return eval(p, candidate(f)); }
-  // ---- staged form (on the trainer's copy): words 1/d, M + x, M + y, -, image, w, h ----
-  static constexpr bool kFastAlways = true;   // fast_stage never fails
+  // ---- words 1/d, M + x, M + y, -, image, w, h ----
   static constexpr bool kSmallResp = true;    // |response| < 2^17
   struct FastCand {
     float o[4];
@@ -267,26 +267,27 @@ struct DepthDiff2 {
     for (int k = 0; k < 4; k++) c.o[k] = fast_offset(f[k]);
     return c;
   }
-  static PD_D bool fast_stage(const ImageRef<uint16_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint32_t *w) {
+  static PD_D void fast_words(const ImageRef<uint16_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint32_t *w) {
     const uint64_t p = (uint64_t)im.data;
-    w[0] = float_bits(inv_depth(pre[0]));
+    w[0] = float_bits(inv_depth((int32_t)pre[0]));
     w[1] = float_bits(kRoundMagic + (float)x);
     w[2] = float_bits(kRoundMagic + (float)y);
     w[4] = (uint32_t)p;
     w[5] = (uint32_t)(p >> 32);
     w[6] = (uint32_t)im.w;
     w[7] = (uint32_t)im.h;
-    return true;
   }
+  template <bool MAPPED>
   static PD_D int32_t fast_probe(const uint4 &a, const uint4 &b, float u, float v) {
     const float inv = bits_float(a.x);
     const uint32_t x = fast_coord(u, inv, bits_float(a.y)), y = fast_coord(v, inv, bits_float(a.z));
-    uint32_t r = (uint32_t)kBgDepth;
+    uint32_t r = MAPPED ? (uint32_t)kBgDepth : 0u;
     if (x < b.z && y < b.w) r = ldg(staged_ptr<uint16_t>(b.x, b.y) + (y * b.z + x));
-    return (int32_t)r;
+    return MAPPED || r ? (int32_t)r : kBgDepth;
   }
+  template <bool MAPPED>
   static PD_D int32_t eval_fast(const uint4 &a, const uint4 &b, const FastCand &c) {
-    return fast_probe(a, b, c.o[0], c.o[1]) - fast_probe(a, b, c.o[2], c.o[3]);
+    return fast_probe<MAPPED>(a, b, c.o[0], c.o[1]) - fast_probe<MAPPED>(a, b, c.o[2], c.o[3]);
   }
 };
 
@@ -369,10 +370,9 @@ struct DepthDiff1 {
   template <bool FAST = false>
   static PD_D int16_t eval_train(const Prep &p, const Cand &c) { return eval<FAST>(p, c); }
   static PD_D int16_t eval(const Prep &p, const int16_t *f) { return eval(p, candidate(f)); }
-  // ---- staged form: words 1/d, M + x, M + y, -, image, w | h << 16, d.  A zero
-  // centre depth reads every probe as outside (w = 0); a negative one (a depth
-  // above 32767 read as short) takes eval_train. ----
-  static constexpr bool kFastAlways = false;
+  // ---- words 1/d, M + x, M + y, -, image, w | h << 16, d.  A zero centre depth
+  // reads every probe as outside (w = 0); the rounding is odd in d, so a negative
+  // one (a depth above 32767 read as short) needs no other form. ----
   static constexpr bool kSmallResp = true;
   struct FastCand {
     float o[2];
@@ -383,18 +383,18 @@ struct DepthDiff1 {
     c.o[1] = fast_offset(500 * (int32_t)f[1]);
     return c;
   }
-  static PD_D bool fast_stage(const ImageRef<uint16_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint32_t *w) {
+  static PD_D void fast_words(const ImageRef<uint16_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint32_t *w) {
     const uint64_t p = (uint64_t)im.data;
     const int32_t d = (int16_t)(int32_t)pre[0];
-    w[0] = float_bits(inv_depth(d > 0 ? (uint32_t)d : 1u));
+    w[0] = float_bits(inv_depth(d ? d : 1));
     w[1] = float_bits(kRoundMagic + (float)x);
     w[2] = float_bits(kRoundMagic + (float)y);
     w[4] = (uint32_t)p;
     w[5] = (uint32_t)(p >> 32);
     w[6] = (d ? (uint32_t)im.w : 0u) | ((uint32_t)im.h << 16);
     w[7] = (uint32_t)d;
-    return d >= 0;
   }
+  template <bool MAPPED>
   static PD_D int16_t eval_fast(const uint4 &a, const uint4 &b, const FastCand &c) {
     const float inv = bits_float(a.x);
     const uint32_t x = fast_coord(c.o[0], inv, bits_float(a.y)), y = fast_coord(c.o[1], inv, bits_float(a.z));
@@ -461,15 +461,13 @@ struct ChannelDiff {
   template <bool FAST = false>
   static PD_D int32_t eval_train(const Prep &p, const Cand &c) { return eval<FAST>(p, c); }
   static PD_D int32_t eval(const Prep &p, const int32_t *f) { return eval(p, candidate(f)); }
-  // ---- staged form: words 3w, x, y, -, the pixel's address, w, h.  A probe is
-  // uy * 3w + (3 ux + c) bytes from the pixel, in 32 bits (images of fewer than
-  // 2^31 bytes; an offset that leaves the image loads nothing, whatever it
-  // wraps to). ----
-  static constexpr bool kFastAlways = false;
+  // ---- words 3w, x, y, -, the pixel's address, w, h.  A probe is uy * 3w + (3 ux +
+  // c) bytes from the pixel (an offset that leaves the image loads nothing, whatever
+  // 3 ux wraps to). ----
   static constexpr bool kSmallResp = true;
   struct FastCand {
     int32_t ux, uy, vx, vy;
-    uint32_t o1, o2;
+    int32_t o1, o2;
   };
   static PD_D FastCand fast_candidate(const int32_t *f) {
     const Cand c = candidate(f);
@@ -478,11 +476,11 @@ struct ChannelDiff {
     r.uy = c.uy;
     r.vx = c.vx;
     r.vy = c.vy;
-    r.o1 = 3u * (uint32_t)c.ux + (uint32_t)c.c1;
-    r.o2 = 3u * (uint32_t)c.vx + (uint32_t)c.c2;
+    r.o1 = (int32_t)(3u * (uint32_t)c.ux + (uint32_t)c.c1);
+    r.o2 = (int32_t)(3u * (uint32_t)c.vx + (uint32_t)c.c2);
     return r;
   }
-  static PD_D bool fast_stage(const ImageRef<uint8_t> &im, int32_t x, int32_t y, const uint32_t *, uint32_t *w) {
+  static PD_D void fast_words(const ImageRef<uint8_t> &im, int32_t x, int32_t y, const uint32_t *, uint32_t *w) {
     const uint64_t p = (uint64_t)im.data + ((uint64_t)((uint32_t)y * (uint32_t)im.w + (uint32_t)x)) * 3u;
     w[0] = 3u * (uint32_t)im.w;
     w[1] = (uint32_t)x;
@@ -491,14 +489,14 @@ struct ChannelDiff {
     w[5] = (uint32_t)(p >> 32);
     w[6] = (uint32_t)im.w;
     w[7] = (uint32_t)im.h;
-    return 3ull * (uint64_t)im.w * (uint64_t)im.h < (1ull << 31);
   }
-  static PD_D int32_t fast_read(const uint4 &a, const uint4 &b, int32_t ux, int32_t uy, uint32_t o) {
+  static PD_D int32_t fast_read(const uint4 &a, const uint4 &b, int32_t ux, int32_t uy, int32_t o) {
     uint32_t r = 0u;
     if (a.y + (uint32_t)ux < b.z && a.z + (uint32_t)uy < b.w)
-      r = ldg(staged_ptr<uint8_t>(b.x, b.y) + (int32_t)((uint32_t)uy * a.x + o));
+      r = ldg(staged_ptr<uint8_t>(b.x, b.y) + ((int64_t)uy * (int32_t)a.x + o));
     return (int32_t)r;
   }
+  template <bool MAPPED>
   static PD_D int32_t eval_fast(const uint4 &a, const uint4 &b, const FastCand &c) {
     return fast_read(a, b, c.ux, c.uy, c.o1) - fast_read(a, b, c.vx, c.vy, c.o2);
   }

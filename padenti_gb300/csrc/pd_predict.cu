@@ -73,6 +73,12 @@ static int ensure_forest_nodes(pd_ctx *ctx) {
   const FeatT *ft = ctx->f_feat.as<FeatT>(), *th = ctx->f_thr.as<FeatT>();
   const int32_t *lc = ctx->f_lc.as<int32_t>();
   const dim3 grid((unsigned)((nodes + 255) / 256 + (nodes == 0)));
+  const uint32_t K = (uint32_t)ctx->cfg.n_classes, KP = (K + 3) / 4 * 4;
+  PD_TRY(ctx->f_post4.ensure(nodes * KP * 4 + 16));
+  k_pad_posteriors<<<(unsigned)((nodes * KP + 255) / 256 + (nodes == 0)), 256, 0, ctx->stream>>>(
+      ctx->f_post.as<float>(), nodes, K, ctx->f_post4.as<float>());
+  PD_CUDA(cudaGetLastError());
+  ctx->launches++;
   if (is_user_plugin(ctx)) {
     const RtcKernels *rk = nullptr;
     PD_TRY(rtc_kernels(ctx, &rk));
@@ -80,18 +86,23 @@ static int ensure_forest_nodes(pd_ctx *ctx) {
     void *args[] = {&ft, &th, &lc, &nodes, &out};
     PD_TRY(rtc_launch(ctx, rk->forest_nodes, grid, dim3(256), 0, args));
   } else if constexpr (!P::kRtcOnly) {
-    k_forest_nodes<P><<<grid, 256, 0, ctx->stream>>>(ft, th, lc, nodes, ctx->f_cand.as<NodeRec<P>>());
-    PD_CUDA(cudaGetLastError());
-    // whether every node takes the fast path: the prediction kernels then carry no slow path
+    // the fast form's records, and whether every node takes it; else the general ones
+    static_assert(sizeof(FastNode<P>) <= sizeof(NodeRec<P>), "both forms fit f_cand");
     PD_TRY(ctx->f_fast.ensure(16));
     int all = 1;
     PD_CUDA(h2d(ctx, ctx->f_fast.ptr, &all, 4));
-    k_forest_fast<P><<<grid, 256, 0, ctx->stream>>>(ctx->f_cand.as<NodeRec<P>>(), nodes, ctx->f_fast.as<int>());
+    k_forest_fast<P><<<grid, 256, 0, ctx->stream>>>(ft, th, lc, nodes, ctx->f_cand.as<FastNode<P>>(),
+                                                    ctx->f_fast.as<int>());
     PD_CUDA(cudaGetLastError());
     PD_CUDA(d2h(ctx, &all, ctx->f_fast.ptr, 4));
     PD_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->forest_fast = all != 0;
-    ctx->launches += 2;
+    ctx->launches++;
+    if (!ctx->forest_fast) {
+      k_forest_nodes<P><<<grid, 256, 0, ctx->stream>>>(ft, th, lc, nodes, ctx->f_cand.as<NodeRec<P>>());
+      PD_CUDA(cudaGetLastError());
+      ctx->launches++;
+    }
   }
   ctx->cand_version = ctx->forest_version;
   return PD_OK;
@@ -114,19 +125,23 @@ static int launch_posterior(pd_ctx *ctx, uint32_t n, const void *images, uint32_
     uint64_t ib = img_bytes;
     uint32_t w_ = W, h_ = H, nt_ = nt, k_ = (uint32_t)ctx->cfg.n_classes;
     const void *nd = ctx->f_cand.ptr;
-    const float *po = ctx->f_post.as<float>();
+    const float *po = ctx->f_post4.as<float>();
     const TreeMeta *me = ctx->f_meta.as<TreeMeta>();
     const uint32_t *mg = ctx->magic_tab.as<uint32_t>();
     void *args[] = {&im, &ib, &w_, &h_, &masks, &out, &nd, &po, &me, &nt_, &k_, &mg};
     return rtc_launch(ctx, rk->predict_posterior, grid, dim3(kPredX, kPredY), smem, args);
   }
   if constexpr (!P::kRtcOnly) {
-    auto kern = ctx->forest_fast ? k_predict_posterior<P, true> : k_predict_posterior<P, false>;
-    PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, dim3(kPredX, kPredY), smem, ctx->stream>>>(
-        static_cast<const uint8_t *>(images), img_bytes, W, H, masks, out, ctx->f_cand.as<NodeRec<P>>(),
-        ctx->f_post.as<float>(), ctx->f_meta.as<TreeMeta>(), nt, (uint32_t)ctx->cfg.n_classes,
-        ctx->magic_tab.as<uint32_t>());
+    auto launch = [&]<bool AF>() -> int {
+      auto kern = k_predict_posterior<P, AF>;
+      PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<grid, dim3(kPredX, kPredY), smem, ctx->stream>>>(
+          static_cast<const uint8_t *>(images), img_bytes, W, H, masks, out, ctx->f_cand.as<Node<P, AF>>(),
+          ctx->f_post4.as<float4>(), ctx->f_meta.as<TreeMeta>(), nt, (uint32_t)ctx->cfg.n_classes,
+          ctx->magic_tab.as<uint32_t>());
+      return PD_OK;
+    };
+    PD_TRY(ctx->forest_fast ? launch.template operator()<true>() : launch.template operator()<false>());
     PD_CUDA(cudaGetLastError());
     ctx->launches++;
   }
@@ -380,7 +395,7 @@ extern "C" int pd_predict_posterior_batch(pd_ctx *ctx, uint32_t n, const void *c
       const BatchImage *bd = ctx->b_desc.as<BatchImage>();
       uint32_t n_ = n, nt_ = nt, k_ = K;
       const void *nd = ctx->f_cand.ptr;
-      const float *po = ctx->f_post.as<float>();
+      const float *po = ctx->f_post4.as<float>();
       const TreeMeta *me = ctx->f_meta.as<TreeMeta>();
       const uint32_t *mg = ctx->magic_tab.as<uint32_t>();
       void *args[] = {&im, &mk, &o, &bd, &n_, &nd, &po, &me, &nt_, &k_, &mg};
@@ -391,9 +406,8 @@ extern "C" int pd_predict_posterior_batch(pd_ctx *ctx, uint32_t n, const void *c
         PD_TRY(rtc_set_smem(ctx, rk->predict_batch, smem));
         fn = (const void *)rk->predict_batch;
       } else if constexpr (!P::kRtcOnly) {
-        auto kern = ctx->forest_fast ? k_predict_batch<P, true> : k_predict_batch<P, false>;
-        fn = (const void *)kern;
-        PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        fn = ctx->forest_fast ? (const void *)k_predict_batch<P, true> : (const void *)k_predict_batch<P, false>;
+        PD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       }
       cudaGraph_t g = nullptr;
       PD_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -465,10 +479,13 @@ extern "C" int pd_predict_leaf(pd_ctx *ctx, uint32_t tree, const void *image, ui
       return rtc_launch(ctx, rk->predict_leaf, grid, dim3(kPredX, kPredY), 0, args);
     }
     if constexpr (!P::kRtcOnly) {
-      auto kern = ctx->forest_fast ? k_predict_leaf<P, true> : k_predict_leaf<P, false>;
-      kern<<<grid, dim3(kPredX, kPredY), 0, st>>>(
-          ctx->p_img.as<uint8_t>(), width, height, mask ? ctx->p_mask.as<uint8_t>() : nullptr,
-          ctx->p_out.as<int32_t>(), ctx->f_cand.as<NodeRec<P>>() + off, depth, ctx->magic_tab.as<uint32_t>());
+      auto launch = [&]<bool AF>() {
+        k_predict_leaf<P, AF><<<grid, dim3(kPredX, kPredY), 0, st>>>(
+            ctx->p_img.as<uint8_t>(), width, height, mask ? ctx->p_mask.as<uint8_t>() : nullptr,
+            ctx->p_out.as<int32_t>(), ctx->f_cand.as<Node<P, AF>>() + off, depth, ctx->magic_tab.as<uint32_t>());
+      };
+      if (ctx->forest_fast) launch.template operator()<true>();
+      else launch.template operator()<false>();
       PD_CUDA(cudaGetLastError());
     }
     return PD_OK;

@@ -23,27 +23,73 @@ struct __align__(16) NodeRec {
   int32_t lc;
 };
 
+// The record of a forest all of whose nodes take the plugin's fast form: its
+// constants there (one word per offset), threshold and left child, in one 16- or
+// 32-byte record, so that a visit fetches one sector.
+template <class P>
+struct __align__(sizeof(typename P::FastCand) <= 8 ? 16 : 32) FastNode {
+  typename P::FastCand c;
+  int32_t thr, lc;
+};
+// What a kernel reads per node: a FastNode (AF) or a NodeRec.
+template <class P, bool AF>
+struct NodeOf {
+  using type = NodeRec<P>;
+};
+template <class P>
+struct NodeOf<P, true> {
+  using type = FastNode<P>;
+};
+template <class P, bool AF>
+using Node = typename NodeOf<P, AF>::type;
+
 constexpr int kPredX = 32, kPredY = 8, kPredThreads = kPredX * kPredY;
-// Tree walks interleaved per pixel.  On the 3-tree, depth-16 forest of 640x480
-// depth maps, 1 measures fastest (7.07e9 pixels/s; 2: 6.91e9, 3: 7.08e9): the
-// wider walks cost registers and occupancy.
-#ifndef PD_PRED_GROUP
-#define PD_PRED_GROUP 1
-#endif
-constexpr int kPredGroup = PD_PRED_GROUP;
+
+// A record by 16-byte read-only loads (one 32-byte load was 6 % slower: L1 returns
+// 128 bytes a cycle, and the last 8 of a FastNode are not wanted).
+template <class N>
+PD_D N load_node(const N *p) {
+  static_assert(sizeof(N) % 16 == 0, "whole 16-byte words");
+  N n;
+  uint4 *d = reinterpret_cast<uint4 *>(&n);
+#pragma unroll
+  for (uint32_t i = 0; i < sizeof(N) / 16; i++) d[i] = ldg(reinterpret_cast<const uint4 *>(p) + i);
+  return n;
+}
+
+// One pixel as the walks read it.
+// AF: every node of the forest takes the plugin's fast form (P::fast, checked once
+// per forest upload): the walk evaluates it from the pixel's words, with no
+// per-visit test or slow path.
+template <class P, bool AF>
+struct Pixel {
+  typename P::Prep prep;
+  PD_D Pixel(const ImageRef<typename P::img_t> &im, int32_t x, int32_t y) : prep(P::prepare(im, x, y)) {}
+  PD_D typename P::feat_t eval(const NodeRec<P> &n) const {
+    return P::fast(n.c) ? P::template eval<true>(prep, n.c) : P::template eval<false>(prep, n.c);
+  }
+};
+template <class P>
+struct Pixel<P, true> {
+  uint4 a, b;
+  PD_D Pixel(const ImageRef<typename P::img_t> &im, int32_t x, int32_t y) {
+    uint32_t pre[2] = {0u, 0u}, w[8];
+    P::preload(im, x, y, pre);
+    P::fast_words(im, x, y, pre, w);
+    a = make_uint4(w[0], w[1], w[2], 0u);
+    b = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+  PD_D typename P::feat_t eval(const FastNode<P> &n) const { return P::template eval_fast<false>(a, b, n.c); }
+};
 
 // Leaf reached by one tree from the root (nodes: the tree's records).
-// AF: every node of the forest takes the plugin's fast path (P::fast, checked
-// once per forest upload), so the walk carries no per-visit test or slow path.
-template <class P, bool AF = false>
-PD_D int32_t walk(const typename P::Prep &prep, const NodeRec<P> *__restrict__ nodes, uint32_t depth) {
-  using FeatT = typename P::feat_t;
+template <class P, bool AF>
+PD_D int32_t walk(const Pixel<P, AF> &px, const Node<P, AF> *__restrict__ nodes, uint32_t depth) {
   int32_t node = 0;
   for (uint32_t d = 1; d < depth; d++) {
-    const NodeRec<P> nr = nodes[node];
-    if (nr.lc < 0) break;  // leaf (-1); an untrained root (-2) also stops
-    const FeatT r = (AF || P::fast(nr.c)) ? P::template eval<true>(prep, nr.c) : P::template eval<false>(prep, nr.c);
-    node = nr.lc + (r <= nr.thr ? 0 : 1);
+    const Node<P, AF> n = load_node(nodes + node);
+    if (n.lc < 0) break;  // leaf (-1); an untrained root (-2) also stops
+    node = n.lc + (px.eval(n) <= n.thr ? 0 : 1);
   }
   return node;
 }
@@ -63,84 +109,83 @@ __global__ void k_forest_nodes(const typename P::feat_t *__restrict__ feat, cons
   }
 }
 
-// Clears *all_fast when a node of the forest needs the plugin's slow path.
+// The FastNode of every forest node; clears *all_fast when a node needs the
+// plugin's slow path (the NodeRec form is built then).
 template <class P>
-__global__ void k_forest_fast(const NodeRec<P> *__restrict__ nodes, unsigned long long n_nodes,
+__global__ void k_forest_fast(const typename P::feat_t *__restrict__ feat, const typename P::feat_t *__restrict__ thr,
+                              const int32_t *__restrict__ lc, unsigned long long n_nodes, FastNode<P> *__restrict__ out,
                               int *__restrict__ all_fast) {
   const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-  if (i < n_nodes && !P::fast(nodes[i].c)) *all_fast = 0;
+  if (i >= n_nodes) return;
+  const typename P::feat_t *f = feat + i * P::kFeatDim;
+  FastNode<P> n;
+  n.c = P::fast_candidate(f);
+  n.thr = (int32_t)thr[i];
+  n.lc = lc[i];
+  out[i] = n;
+  if (!P::fast(P::candidate(f))) *all_fast = 0;
 }
 
-// The leaves of trees t0 .. t0+G-1 (those below n_trees) for one pixel, the G
-// walks interleaved level by level so that their loads overlap; each walk is
-// the one walk() does.
-template <class P, int G, bool AF = false>
-PD_D void walk_group(const typename P::Prep &prep, const NodeRec<P> *__restrict__ nodes,
-                     const TreeMeta *__restrict__ meta, uint32_t t0, uint32_t n_trees, int32_t *leaf_s,
-                     uint32_t tid) {
-  using FeatT = typename P::feat_t;
-  int32_t node[G];
-  size_t off[G];
-  uint32_t depth[G];
-#pragma unroll
-  for (int g = 0; g < G; g++) {
-    node[g] = 0;
-    const bool have = t0 + g < n_trees;
-    off[g] = have ? meta[t0 + g].off : 0;
-    depth[g] = have ? meta[t0 + g].depth : 0;  // depth 0: no step
-  }
-  uint32_t live = 0;
-#pragma unroll
-  for (int g = 0; g < G; g++) live |= (depth[g] > 1 ? 1u : 0u) << g;
-  for (uint32_t d = 1; live; d++) {
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-      if (!((live >> g) & 1u)) continue;
-      const NodeRec<P> nr = nodes[off[g] + node[g]];
-      if (nr.lc < 0) {  // leaf (-1); an untrained root (-2) also stops
-        live &= ~(1u << g);
-        continue;
-      }
-      const FeatT r = (AF || P::fast(nr.c)) ? P::template eval<true>(prep, nr.c) : P::template eval<false>(prep, nr.c);
-      node[g] = nr.lc + (r <= nr.thr ? 0 : 1);
-      if (d + 1 >= depth[g]) live &= ~(1u << g);
-    }
-  }
-#pragma unroll
-  for (int g = 0; g < G; g++)
-    if (t0 + g < n_trees) leaf_s[(t0 + g) * kPredThreads + tid] = node[g];
-}
-
-// The forest posterior of pixel (x, y): the leaf of every tree (kept in the
-// CTA's leaf_s, [tree][thread]), then the leaf posteriors summed in tree order
-// and divided by the tree count, written planar with stride plane.
+// What bounds it (60 640x480 maps, 3 trees of depth 16, 9 classes): the L1 data pipe
+// (90 %, 15 wavefronts per node visit: 24 bytes of record per lane, and probes that
+// scatter once the lanes' nodes differ), then issue (81 %, 50 instructions per visit;
+// 81 with the general records).  160 maps: 5.88 -> 3.97 ms.  CTA rows of 32 pixels:
+// warps of 16x2 and 8x4 pixels were 9 and 28 % slower (a probe's pixels lie in one
+// image row).
+//
+// The forest posterior of pixel (x, y): the leaf of every tree (its index in the
+// forest, kept in the CTA's leaf_s, [tree][thread]), then the leaf posteriors summed
+// in tree order and divided by the tree count, written planar with stride plane.
+// post: rows of K4 float4 (the classes padded to a multiple of four), so that four
+// classes of a leaf are one load; the planes are written with the streaming hint
+// (they are not read here, and the images and records stay in L2).
 template <class P, bool AF = false>
 PD_D void predict_pixel(const ImageRef<typename P::img_t> &im, uint32_t x, uint32_t y, bool masked_out, float *o,
-                        size_t plane, const NodeRec<P> *__restrict__ nodes, const float *__restrict__ post,
+                        size_t plane, const Node<P, AF> *__restrict__ nodes, const float4 *__restrict__ post,
                         const TreeMeta *__restrict__ meta, uint32_t n_trees, uint32_t K, int32_t *leaf_s,
                         uint32_t tid) {
   if (masked_out) {
     for (uint32_t l = 0; l < K; l++) o[l * plane] = 0.0f;
     return;
   }
-  const auto prep = P::prepare(im, (int32_t)x, (int32_t)y);
-  for (uint32_t t = 0; t < n_trees; t += kPredGroup)
-    walk_group<P, kPredGroup, AF>(prep, nodes, meta, t, n_trees, leaf_s, tid);
-  const float nt = (float)n_trees;
-  for (uint32_t l = 0; l < K; l++) {
-    float acc = 0.0f;
-    for (uint32_t t = 0; t < n_trees; t++)
-      acc = acc + ldg(post + (meta[t].off + (size_t)leaf_s[t * kPredThreads + tid]) * K + l);
-    o[l * plane] = fdiv(acc, nt);
+  const Pixel<P, AF> px(im, (int32_t)x, (int32_t)y);
+  for (uint32_t t = 0; t < n_trees; t++) {
+    const unsigned long long off = meta[t].off;
+    leaf_s[t * kPredThreads + tid] = (int32_t)off + walk<P, AF>(px, nodes + off, meta[t].depth);
   }
+  const float nt = (float)n_trees;
+  const uint32_t K4 = (K + 3) / 4;
+  for (uint32_t q = 0; q < K4; q++) {
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (uint32_t t = 0; t < n_trees; t++) {
+      const float4 p = ldg(post + (size_t)(uint32_t)leaf_s[t * kPredThreads + tid] * K4 + q);
+      acc[0] = acc[0] + p.x;
+      acc[1] = acc[1] + p.y;
+      acc[2] = acc[2] + p.z;
+      acc[3] = acc[3] + p.w;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++)
+      if (4 * q + i < K) __stcs(o + (4 * q + i) * plane, fdiv(acc[i], nt));
+  }
+}
+
+// post [n][K] -> out [n][4 ceil(K / 4)], padded with zeros.
+static __global__ void k_pad_posteriors(const float *__restrict__ post, unsigned long long n, uint32_t K,
+                                        float *__restrict__ out) {
+  const uint32_t KP = (K + 3) / 4 * 4;
+  const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+  if (i >= n * KP) return;
+  const uint32_t l = (uint32_t)(i % KP);
+  out[i] = l < K ? post[i / KP * K + l] : 0.0f;
 }
 
 // grid (ceil(W/32), ceil(H/8), n_images); dynamic smem n_trees*256 int32.
 template <class P, bool AF = false>
 __global__ void __launch_bounds__(kPredThreads) k_predict_posterior(
     const uint8_t *__restrict__ images, uint64_t img_bytes, uint32_t W, uint32_t H,
-    const uint8_t *__restrict__ masks, float *__restrict__ out, const NodeRec<P> *__restrict__ nodes,
-    const float *__restrict__ post, const TreeMeta *__restrict__ meta, uint32_t n_trees, uint32_t K,
+    const uint8_t *__restrict__ masks, float *__restrict__ out, const Node<P, AF> *__restrict__ nodes,
+    const float4 *__restrict__ post, const TreeMeta *__restrict__ meta, uint32_t n_trees, uint32_t K,
     const uint32_t *__restrict__ magic) {
   using ImgT = typename P::img_t;
   extern __shared__ int32_t leaf_s[];
@@ -170,8 +215,8 @@ struct BatchImage {
 template <class P, bool AF = false>
 __global__ void __launch_bounds__(kPredThreads) k_predict_batch(
     const uint8_t *__restrict__ images, const uint8_t *__restrict__ masks, uint8_t *__restrict__ out,
-    const BatchImage *__restrict__ batch, uint32_t n, const NodeRec<P> *__restrict__ nodes,
-    const float *__restrict__ post, const TreeMeta *__restrict__ meta, uint32_t n_trees, uint32_t K,
+    const BatchImage *__restrict__ batch, uint32_t n, const Node<P, AF> *__restrict__ nodes,
+    const float4 *__restrict__ post, const TreeMeta *__restrict__ meta, uint32_t n_trees, uint32_t K,
     const uint32_t *__restrict__ magic) {
   using ImgT = typename P::img_t;
   extern __shared__ int32_t leaf_s[];
@@ -201,7 +246,7 @@ template <class P, bool AF = false>
 __global__ void __launch_bounds__(kPredThreads) k_predict_leaf(const uint8_t *__restrict__ image, uint32_t W,
                                                                uint32_t H, const uint8_t *__restrict__ mask,
                                                                int32_t *__restrict__ out,
-                                                               const NodeRec<P> *__restrict__ nodes,
+                                                               const Node<P, AF> *__restrict__ nodes,
                                                                uint32_t depth, const uint32_t *__restrict__ magic) {
   using ImgT = typename P::img_t;
   const uint32_t x = blockIdx.x * kPredX + threadIdx.x, y = blockIdx.y * kPredY + threadIdx.y;
@@ -216,7 +261,7 @@ __global__ void __launch_bounds__(kPredThreads) k_predict_leaf(const uint8_t *__
   im.w = (int32_t)W;
   im.h = (int32_t)H;
   im.magic = magic;
-  out[pix] = walk<P, AF>(P::prepare(im, (int32_t)x, (int32_t)y), nodes, depth);
+  out[pix] = walk<P, AF>(Pixel<P, AF>(im, (int32_t)x, (int32_t)y), nodes, depth);
 }
 
 // One step of the per-pixel node map of features that read the tree

@@ -705,13 +705,12 @@ PD_D uint32_t rank_offset(int32_t r, int32_t lo, int32_t cap, const uint2 *col) 
   return e.y + (uint32_t)__popc(e.x & low_mask(v)) * 128u;
 }
 
-// Staged words of a plugin without its own form, and of samples or tiles that
-// do not take it: position, preload words, size, image pointer, map offset.
+// Staged words of a plugin without its own form, and of tiles that do not take it: position, preload words, size, image pointer, map offset.
 template <class P>
 struct PlainStage {
   using Cand = typename P::Cand;
   static PD_D Cand candidate(const typename P::feat_t *f) { return P::candidate(f); }
-  static PD_D bool stage(const ImageRef<typename P::img_t> &im, int32_t x, int32_t y, const uint32_t *pre,
+  static PD_D void stage(const ImageRef<typename P::img_t> &im, int32_t x, int32_t y, const uint32_t *pre,
                          uint64_t moff, uint32_t *w) {
     const uint64_t p = (uint64_t)im.data;
     w[0] = (uint32_t)x | ((uint32_t)y << 16);
@@ -726,7 +725,6 @@ struct PlainStage {
       w[6] = P::kPreWords > 1 ? pre[P::kPreWords - 1] : 0u;
       w[7] = 0u;
     }
-    return true;
   }
   static PD_D typename P::feat_t eval(const DevSet &ds, const uint4 &a, const uint4 &b, const Cand &c) {
     ImageRef<typename P::img_t> im;
@@ -744,12 +742,12 @@ template <class P>
 struct FastStage {
   using Cand = typename P::FastCand;
   static PD_D Cand candidate(const typename P::feat_t *f) { return P::fast_candidate(f); }
-  static PD_D bool stage(const ImageRef<typename P::img_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint64_t,
+  static PD_D void stage(const ImageRef<typename P::img_t> &im, int32_t x, int32_t y, const uint32_t *pre, uint64_t,
                          uint32_t *w) {
-    return P::fast_stage(im, x, y, pre, w);
+    P::fast_words(im, x, y, pre, w);
   }
   static PD_D typename P::feat_t eval(const DevSet &, const uint4 &a, const uint4 &b, const Cand &c) {
-    return P::eval_fast(a, b, c);
+    return P::template eval_fast<true>(a, b, c);
   }
 };
 
@@ -797,7 +795,6 @@ PD_D void hist_samples_rank(const DevSet &ds, const SampleRec *__restrict__ rec,
   const uint32_t bs = share >= 32u ? 32u : (share + SPI - 1) / SPI * SPI;
   for (uint32_t base = w.begin + warp * bs; base < w.end; base += bs * kWarps) {
     const uint32_t n_here = min(bs, w.end - base);
-    bool ok = true;
     if (lane < n_here) {
       const uint4 r = ldg(reinterpret_cast<const uint4 *>(rec + base + lane));
       const uint32_t imi = r.y & 0xffffffu;
@@ -810,14 +807,11 @@ PD_D void hist_samples_rank(const DevSet &ds, const SampleRec *__restrict__ rec,
       uint64_t moff = 0;
       if constexpr (P::kUsesTree) moff = ds.map_off ? ds.map_off[imi] : 0ull;
       uint32_t v[8];
-      ok = S::stage(im, (int32_t)(r.x & 0xffffu), (int32_t)(r.x >> 16), pre, moff, v);
-      if (!P::kFastAlways && !ok) ok = !PlainStage<P>::stage(im, (int32_t)(r.x & 0xffffu), (int32_t)(r.x >> 16), pre, moff, v);
+      S::stage(im, (int32_t)(r.x & 0xffffu), (int32_t)(r.x >> 16), pre, moff, v);
       v[3] = row_of(r.y >> 24) * class_bytes;
       st[2 * lane] = make_uint4(v[0], v[1], v[2], v[3]);
       st[2 * lane + 1] = make_uint4(v[4], v[5], v[6], v[7]);
     }
-    // samples whose words are plain ones (none for most plugins)
-    const uint32_t plain = P::kFastAlways ? 0u : __ballot_sync(0xffffffffu, !ok);
     __syncwarp();
     auto add = [&](uint32_t row, int32_t ra, int32_t rb) {
       // Rank T (no threshold >= r) and the columns past F (no bits: rank 0) land in
@@ -825,33 +819,23 @@ PD_D void hist_samples_rank(const DevSet &ds, const SampleRec *__restrict__ rec,
       atomicAdd(reinterpret_cast<uint32_t *>(sh_hist + row + rank_offset<P::kSmallResp>(ra, lo, cap, ta)), 1u);
       atomicAdd(reinterpret_cast<uint32_t *>(sh_hist + row + rank_offset<P::kSmallResp>(rb, lo, cap, tb)), 0x10000u);
     };
-    if (P::kFastAlways || plain == 0u) {
-      uint32_t i = 0;
-      for (; i + SPI <= n_here; i += SPI) {
-        int32_t ra[SPI], rb[SPI];
-        uint32_t row[SPI];
+    uint32_t i = 0;
+    for (; i + SPI <= n_here; i += SPI) {
+      int32_t ra[SPI], rb[SPI];
+      uint32_t row[SPI];
 #pragma unroll
-        for (int k = 0; k < SPI; k++) {
-          const uint4 a = st[2 * (i + k)], b = st[2 * (i + k) + 1];
-          row[k] = a.w;
-          ra[k] = (int32_t)S::eval(ds, a, b, ca);
-          rb[k] = (int32_t)S::eval(ds, a, b, cb);
-        }
+      for (int k = 0; k < SPI; k++) {
+        const uint4 a = st[2 * (i + k)], b = st[2 * (i + k) + 1];
+        row[k] = a.w;
+        ra[k] = (int32_t)S::eval(ds, a, b, ca);
+        rb[k] = (int32_t)S::eval(ds, a, b, cb);
+      }
 #pragma unroll
-        for (int k = 0; k < SPI; k++) add(row[k], ra[k], rb[k]);
-      }
-      for (; i < n_here; i++) {
-        const uint4 a = st[2 * i], b = st[2 * i + 1];
-        add(a.w, (int32_t)S::eval(ds, a, b, ca), (int32_t)S::eval(ds, a, b, cb));
-      }
-    } else {
-      const auto pa = tile_candidate<P, PlainStage<P>>(feat, F, f0 + lane);
-      const auto pb = tile_candidate<P, PlainStage<P>>(feat, F, f0 + 32 + lane);
-      for (uint32_t i = 0; i < n_here; i++) {
-        const uint4 a = st[2 * i], b = st[2 * i + 1];
-        if ((plain >> i) & 1u) add(a.w, (int32_t)PlainStage<P>::eval(ds, a, b, pa), (int32_t)PlainStage<P>::eval(ds, a, b, pb));
-        else add(a.w, (int32_t)S::eval(ds, a, b, ca), (int32_t)S::eval(ds, a, b, cb));
-      }
+      for (int k = 0; k < SPI; k++) add(row[k], ra[k], rb[k]);
+    }
+    for (; i < n_here; i++) {
+      const uint4 a = st[2 * i], b = st[2 * i + 1];
+      add(a.w, (int32_t)S::eval(ds, a, b, ca), (int32_t)S::eval(ds, a, b, cb));
     }
     __syncwarp();  // the words are read before the next batch overwrites them
   }

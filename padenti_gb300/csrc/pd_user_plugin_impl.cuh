@@ -74,7 +74,6 @@ struct UserPlugin {
   static PD_D feat_t eval(const Prep &p, const feat_t *f) { return call(p, f); }
   // The histogram kernel takes a user feature through its plain staged words
   // (PlainStage, pd_train_kernels.cuh).
-  static constexpr bool kFastAlways = true;
   static constexpr bool kSmallResp = false;  // a response may be any value of feat_t
 };
 
