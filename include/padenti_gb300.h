@@ -405,11 +405,12 @@ typedef struct {
   uint64_t images;
   uint64_t data_bytes;       /* image bytes checksummed */
   uint64_t label_bytes;      /* label bytes read */
-  uint64_t kernel_launches;
+  uint64_t kernel_launches;  /* two per group of images: the scan and the drawing phase (which may be
+                                several kernels) */
   uint64_t h2d_bytes;
   uint64_t d2h_bytes;
   double ms_scan;            /* checksum + labelled-pixel count kernel */
-  double ms_draw;            /* per-image drawing / reservoir kernel */
+  double ms_draw;            /* drawing / reservoir kernels */
   double ms_total;           /* wall time of the call */
 } pd_sample_stats;
 

@@ -113,6 +113,9 @@ extern "C" int pd_ctx_destroy(pd_ctx *ctx) {
   ctx->sm_lab.release();
   ctx->sm_desc.release();
   ctx->sm_out.release();
+  ctx->sm_counts.release();
+  ctx->sm_draws.release();
+  ctx->sm_slots.release();
   ctx->h_sm.release();
   ctx->h_sm_desc.release();
   for (auto &sl : ctx->samp) {

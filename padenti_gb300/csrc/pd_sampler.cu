@@ -9,16 +9,20 @@
 //     image as the XOR of per-thread checksums of its bytes, each moved to its
 //     place by a multiplication modulo the CRC polynomial, and the number of
 //     labelled pixels.
-//  2. one CTA per image: MT19937 blocks of 624 words, each twisted in three
-//     parallel phases, then
-//     - k_sample_uniform: Boost's bucket method on every draw (accepted draws
-//       keep their order by a block scan), a bitonic sort of the drawn ranks,
-//       one pass over the labels that maps ranks to pixel indices;
-//     - k_sample_class_weighted: the per-class reservoir in scan order, 1024
-//       pixels per step: a pixel's count within its class and its draw index
-//       come from warp matches and block scans; a write lands by atomicMax on
-//       its slot (pixel order is scan order, so the last writer of the
-//       sequential loop wins); the buckets are then gathered and sorted.
+//  2. uniform: one CTA per image (k_sample_uniform): MT19937 blocks of 624 words,
+//     each twisted in three parallel phases, Boost's bucket method on every draw
+//     (accepted draws keep their order by a block scan), a bitonic sort of the
+//     drawn ranks, one pass over the labels that maps ranks to pixel indices.
+//  3. class-weighted: the per-class reservoir in scan order, in parallel over
+//     segments of 512 pixels.  A pixel's count within its class and its draw's
+//     index depend only on the class counts before it, so
+//     - k_class_counts counts every segment's classes, k_class_prefix turns the
+//       counts of an image into each segment's counts and first draw;
+//     - k_mt_draws writes each image's MT19937 outputs (the one serial chain left);
+//     - k_reservoir takes a warp per segment: ranks from ballots, draws by index; a
+//       write lands by atomicMax on its slot (pixel order is scan order, so the
+//       last writer of the sequential loop wins);
+//     - k_bucket_samples gathers and sorts the buckets.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -48,7 +52,6 @@ constexpr uint32_t kSliceBytes = kRegion * kSmWarps;         // 256 KiB per chec
 constexpr uint32_t kGap = 2 * kBlock - kPiece;               // from one piece of a chain to its next
 constexpr uint32_t kLabVecsPerItem = 16 * kSmThreads;        // 64 KiB of labels per count work item
 constexpr uint32_t kMtN = 624;
-constexpr uint32_t kWindow = 4 * kSmThreads;                  // pixels per reservoir step
 constexpr uint32_t kNoError = 0xFFFFFFFFu;
 
 // One image of a sampled batch.  Offsets are into the batch's data, label and
@@ -63,7 +66,8 @@ struct SampImage {
   uint32_t n_slices;  // checksum work items (kSliceBytes each, counted from data_end)
   uint32_t crc0;      // its first checksum work item (checksum items come first)
   uint32_t lab0;      // its first label work item
-  uint32_t pad;
+  uint32_t seg0;      // its first segment (class-weighted: kSeg pixels each)
+  uint64_t draw_off;  // its first draw in the group's draws (class-weighted)
 };
 
 // ---- arithmetic modulo the CRC-32 polynomial (reflected: bit 31 is x^0) ----
@@ -450,140 +454,316 @@ __global__ void __launch_bounds__(kSmThreads) k_sample_uniform(const uint8_t *__
   if (t == 0) out_count[im] = n_samples;
 }
 
-// ClassWeightedImageSampler::sample, one CTA per image.  Dynamic shared
-// memory: n_slots bucket slots (pixel + 1, 0 = empty) then sort_n words.
-// Step layout: warp w, round j, lane l holds pixel win + 128 w + 32 j + l, so
-// (w, j, l) order is scan order.
-__global__ void __launch_bounds__(kSmThreads) k_sample_class_weighted(
-    const uint8_t *__restrict__ labels, const SampImage *__restrict__ imgs, const uint32_t *__restrict__ crc,
-    const uint32_t *__restrict__ bucket_size, uint32_t n_classes, uint32_t n_slots, uint32_t seed, uint32_t sort_n,
-    uint32_t *__restrict__ out, uint32_t *__restrict__ out_count, uint32_t *__restrict__ err) {
-  extern __shared__ uint32_t dyn[];
-  uint32_t *slots = dyn, *keys = dyn + n_slots;
-  __shared__ uint32_t ring[3][kMtN];  // MT block b in ring[b % 3]; the seeded state is block -1
-  __shared__ uint32_t bsz[256], boff[256], seen[256];
-  __shared__ uint32_t wcnt[kSmWarps][256];
-  __shared__ uint32_t wd[kSmWarps];
-  __shared__ uint32_t bad;
-  const uint32_t im = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const uint32_t lt = (1u << lane) - 1;
+// ---- ClassWeightedImageSampler::sample ----
+// 500 maps of 640x480, 2000 samples, 9 classes: one CTA walking each image in
+// 1024-pixel steps (three barriers per 624 draws, four per step) took 1.07 ms.  The
+// kernels below take 0.09 (counts), 0.02 (prefix), 0.20 (draws), 0.38 (reservoir) and
+// 0.02 ms (samples), and the checksum scan no longer reads the labels (0.129 -> 0.119).
+constexpr uint32_t kSeg = 512;  // pixels of a segment (16 per lane of a warp)
+constexpr uint32_t kSegRun = 2;    // segments of a k_reservoir warp, one after the other
+constexpr uint32_t kSegGroup = 4;  // its rows of 32 pixels in flight together
+constexpr int kResCtas = 5;
+
+// Class counts of every segment: class k of segment s of an image at
+// counts[seg0 * n_classes + k * segs + s].  A warp per segment; 32 classes at a time
+// in counters of the lane's own ([class][lane], no conflicts): one shared add per
+// label, then a warp sum per class.  Labels above n_classes are errors (err: the
+// lowest image).
+// Grid: (segments of the largest image / kSmWarps, images).
+__global__ void __launch_bounds__(kSmThreads) k_class_counts(const uint8_t *__restrict__ labels,
+                                                             const SampImage *__restrict__ imgs, uint32_t first,
+                                                             uint32_t n_classes, uint32_t *__restrict__ counts,
+                                                             uint32_t *__restrict__ err) {
+  extern __shared__ uint32_t cnt_all[];  // [warps][min(n_classes, 32) + 1][32]; row 0: every other label
+  const uint32_t rows = min(n_classes, 32u) + 1;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, im = first + blockIdx.y;
+  uint32_t *mine = cnt_all + warp * rows * 32 + lane;
   const SampImage g = imgs[im];
-  for (uint32_t k = t; k < n_classes; k += kSmThreads) {
-    bsz[k] = bucket_size[k];
-    seen[k] = 0;
+  const uint32_t s = blockIdx.x * kSmWarps + warp, segs = (g.n_pix + kSeg - 1) / kSeg;
+  if (s >= segs) return;
+  // 16 labels a lane (zeros past the image), in any order
+  const uint32_t p = s * kSeg + 16 * lane;
+  const uint4 q = p < g.lab_vecs * 16u ? __ldg(reinterpret_cast<const uint4 *>(labels + g.lab_off + p)) : make_uint4(0, 0, 0, 0);
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+  uint32_t bad = 0;
+  for (uint32_t k0 = 0; k0 < n_classes; k0 += 32) {
+    const uint32_t nk = min(n_classes - k0, 32u);
+    for (uint32_t k = 0; k <= nk; k++) mine[k * 32] = 0u;
+#pragma unroll
+    for (uint32_t i = 0; i < 16; i++) {
+      const uint32_t l = (w[i >> 2] >> (8 * (i & 3))) & 0xFFu, k = l - k0;
+      bad |= l > n_classes;
+      atomicAdd(&mine[(k <= nk ? k : 0u) * 32], 1u);  // the lane's own word: no wait between the adds
+    }
+    uint32_t out = 0;  // lane k: class k0 + k
+    for (uint32_t k = 0; k < nk; k++) {
+      const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, mine[(k + 1) * 32]);
+      if (lane == k) out = sum;
+    }
+    if (lane < nk) counts[(size_t)g.seg0 * n_classes + (size_t)(k0 + lane) * segs + s] = out;
   }
-  for (uint32_t k = t; k < kSmWarps * 256; k += kSmThreads) (&wcnt[0][0])[k] = 0;
-  for (uint32_t i = t; i < n_slots; i += kSmThreads) slots[i] = 0;
-  if (t == 0) {
-    uint32_t o = 0;
+  if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicMin(err, im);
+}
+
+// counts of an image's segments -> the pixels of each class before the segment (in
+// place), the class totals, and the index of each segment's first draw: a pixel
+// draws when its class's bucket is full.  One CTA per image, a warp per class.
+__global__ void __launch_bounds__(kSmThreads) k_class_prefix(const SampImage *__restrict__ imgs, uint32_t n_classes,
+                                                             const uint32_t *__restrict__ bucket_size,
+                                                             uint32_t *__restrict__ counts, uint32_t *__restrict__ draw0,
+                                                             uint32_t *__restrict__ class_tot,
+                                                             uint32_t *__restrict__ n_draws) {
+  const SampImage g = imgs[blockIdx.x];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t segs = (g.n_pix + kSeg - 1) / kSeg;
+  uint32_t *c = counts + (size_t)g.seg0 * n_classes;
+  for (uint32_t k = warp; k < n_classes; k += kSmWarps) {
+    uint32_t *ck = c + (size_t)k * segs, run = 0;
+    uint32_t nxt = lane < segs ? ck[lane] : 0u;
+    for (uint32_t s0 = 0; s0 < segs; s0 += 32) {
+      const uint32_t s = s0 + lane, v = nxt;
+      nxt = s + 32 < segs ? ck[s + 32] : 0u;  // the next step's, ahead
+      uint32_t x = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+      }
+      if (s < segs) ck[s] = run + x - v;
+      run += __shfl_sync(0xFFFFFFFFu, x, 31);
+    }
+    if (lane == 0) class_tot[(size_t)blockIdx.x * n_classes + k] = run;
+  }
+  __syncthreads();
+  for (uint32_t s = threadIdx.x; s <= segs; s += kSmThreads) {
+    uint32_t d = 0;
+#pragma unroll 8
     for (uint32_t k = 0; k < n_classes; k++) {
-      boff[k] = o;
-      o += bucket_size[k];
+      const uint32_t seen = s < segs ? c[(size_t)k * segs + s] : class_tot[(size_t)blockIdx.x * n_classes + k];
+      d += seen > bucket_size[k] ? seen - bucket_size[k] : 0u;
     }
-    bad = 0;
-    mt_seed(ring[2], crc[im] ^ seed);
+    if (s < segs) draw0[g.seg0 + s] = d;
+    else n_draws[blockIdx.x] = d;
+  }
+}
+
+// The first n_draws MT19937 outputs of every image of a group, at draws + g.draw_off.
+// One CTA of 112 threads per image: word n + 624 needs words n, n + 1 and n + 397, so
+// 224 words go at a time, two a thread (64-bit shared accesses), one barrier each; the
+// words run through a linear array (fixed offsets from one pointer) whose last 624
+// move to its start at the end of a lap.  A step's words are tempered and stored
+// while the next step's loads are in flight, off the chain.  ALU-bound when an SM
+// holds four images (64 % of the pipe), the chain's latency below that; one word a
+// thread in 8 warps 0.22 ms for 500 images, four in 2 warps 0.21, this 0.20.  Every
+// thread of the CTA works in every step: the barriers see whole warps.
+constexpr uint32_t kMtStep = 224, kMtThreads = kMtStep / 2, kMtLap = 15;
+constexpr uint32_t kMtWords = kMtN + kMtLap * kMtStep;
+__global__ void __launch_bounds__(kMtThreads) k_mt_draws(const SampImage *__restrict__ imgs, uint32_t first,
+                                                         const uint32_t *__restrict__ crc, uint32_t seed,
+                                                         const uint32_t *__restrict__ n_draws,
+                                                         uint32_t *__restrict__ draws) {
+  __shared__ __align__(16) uint32_t x[kMtWords];
+  const uint32_t im = first + blockIdx.x, t = threadIdx.x, n = n_draws[im];
+  if (n == 0) return;
+  uint32_t *out = draws + imgs[im].draw_off + 2 * t;  // 8-byte aligned; whole pairs are kept
+  if (t == 0) mt_seed(x, crc[im] ^ seed);
+  __syncthreads();
+  uint2 v = make_uint2(0, 0);
+  for (uint32_t d0 = 0; d0 < n;) {
+    uint32_t *p = x + 2 * t;
+    for (uint32_t lap = 0; lap < kMtLap && d0 < n; lap++, d0 += kMtStep, p += kMtStep) {
+      const uint2 a = *reinterpret_cast<const uint2 *>(p), b = *reinterpret_cast<const uint2 *>(p + 396),
+                  c = *reinterpret_cast<const uint2 *>(p + 398);
+      const uint32_t a2 = p[2];
+      if (d0) {  // the step before: draws d0 - kMtStep + 2 t (all below n: n > d0)
+        *reinterpret_cast<uint2 *>(out) = make_uint2(mt_temper(v.x), mt_temper(v.y));
+        out += kMtStep;
+      }
+      v = make_uint2(b.y ^ mt_mix(a.x, a.y), c.x ^ mt_mix(a.y, a2));
+      *reinterpret_cast<uint2 *>(p + kMtN) = v;
+      __syncthreads();
+    }
+    if (d0 >= n) break;
+    for (uint32_t i = t; i < kMtN; i += kMtThreads) x[i] = x[kMtLap * kMtStep + i];  // the two ranges are apart
+    __syncthreads();
+  }
+  // the last step: its draws below n
+  const uint32_t i = (n - 1) / kMtStep * kMtStep + 2 * t;
+  if (i < n) *reinterpret_cast<uint2 *>(out) = make_uint2(mt_temper(v.x), mt_temper(v.y));
+}
+static_assert(kMtLap * kMtStep >= kMtN, "a lap's end does not overlap its start");
+
+// The reservoir, a warp per kSegRun segments (grid as k_class_counts).  Pixel p of
+// class k with c pixels of its class before it takes slot c while the bucket has
+// room; else its draw v picks slot roundf(v 2^-32 c), which counts if it lies in the
+// bucket.  c and the draw's index come from the segment's prefix and the ballots of
+// the rows before it.  floor(v c 2^-32) >= the bucket's size settles nearly every
+// draw (the rounding is monotone, and the size a float).
+// BITS: of a label, n_classes < 2^BITS; up to 32 classes are counted a lane each (a
+// row's mask of class k is lane k's, and goes to the pixels of class k by a shuffle);
+// BITS = 8: more classes, counted in shared memory.
+// Issue-bound (62 instructions per row of 32 pixels, 50 % issue-active at 24 warps,
+// waiting for the draws); eight rows in flight with four CTAs 0.386 ms, four rows with
+// five 0.378; all rows of a segment unrolled 0.48-0.74 (instruction cache).
+template <int BITS>
+__global__ void __launch_bounds__(kSmThreads, kResCtas) k_reservoir(const uint8_t *__restrict__ labels,
+                                                          const SampImage *__restrict__ imgs, uint32_t first,
+                                                          uint32_t n_classes,
+                                                          const uint32_t *__restrict__ bucket_size,
+                                                          const uint32_t *__restrict__ bucket_off,
+                                                          const uint32_t *__restrict__ counts,
+                                                          const uint32_t *__restrict__ draw0,
+                                                          const uint32_t *__restrict__ draws, uint32_t stride,
+                                                          uint32_t *__restrict__ slots) {
+  constexpr bool WIDE = BITS == 8;
+  __shared__ uint32_t s_cnt[WIDE ? kSmWarps : 1][WIDE ? 256 : 1];  // by label
+  __shared__ uint32_t bsz[257], boff[257];  // by label; label 0 never fills its bucket
+  for (uint32_t k = threadIdx.x; k <= n_classes; k += kSmThreads) {
+    bsz[k] = k ? bucket_size[k - 1] : 0xFFFFFFFFu;
+    boff[k] = k ? bucket_off[k - 1] : 0u;
   }
   __syncthreads();
-  const uint8_t *lab = labels + g.lab_off;
-  uint32_t gen = 0, d_base = 0;
-  uint32_t nxt[4];  // the labels of the next step, loaded ahead
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+  const uint32_t im = first + blockIdx.y;
+  const SampImage g = imgs[im];
+  const uint32_t segs = (g.n_pix + kSeg - 1) / kSeg;
+  const uint32_t s_beg = (blockIdx.x * kSmWarps + warp) * kSegRun, s_end = min(segs, s_beg + kSegRun);
+  if (s_beg >= segs) return;
+  const uint8_t *lp = labels + g.lab_off;
+  // groups of kSegGroup rows of 32 pixels (row i: pixels p + 32 i + lane), the next
+  // group's labels loaded ahead; the loop over them stays a loop (unrolled, it
+  // outgrows the instruction cache)
+  const uint32_t p_beg = s_beg * kSeg, p_end = min(g.n_pix, s_end * kSeg);
+  uint32_t nxt[kSegGroup];
+  auto load_rows = [&](uint32_t p0) {
 #pragma unroll
-  for (uint32_t j = 0; j < 4; j++) {
-    const uint32_t p = warp * 128 + j * 32 + lane;
-    nxt[j] = p < g.n_pix ? lab[p] : 0u;
-  }
-  for (uint32_t win = 0; win < g.n_pix; win += kWindow) {
-    uint32_t cls[4], rank[4];
-    bool valid[4];
-#pragma unroll
-    for (uint32_t j = 0; j < 4; j++) {
-      cls[j] = nxt[j];
-      const uint32_t p = win + kWindow + warp * 128 + j * 32 + lane;
-      nxt[j] = p < g.n_pix ? lab[p] : 0u;
+    for (uint32_t i = 0; i < kSegGroup; i++) {
+      const uint32_t p = p0 + 32 * i + lane;
+      nxt[i] = p < p_end ? (uint32_t)__ldg(lp + p) : 0u;
     }
+  };
+  load_rows(p_beg);
+  const uint32_t *c0 = counts + (size_t)g.seg0 * n_classes + s_beg;
+  uint32_t cnt = 0, flip[BITS];  // lane k: pixels of class k so far; the inverted bits of label k + 1
 #pragma unroll
-    for (uint32_t j = 0; j < 4; j++) {
-      const uint32_t k = cls[j] - 1u;
-      valid[j] = cls[j] != 0 && k < n_classes;
-      if (cls[j] != 0 && k >= n_classes) atomicOr(&bad, 1u);
-      cls[j] = valid[j] ? k : 0xFFFFFFFFu;
-      const uint32_t peers = __match_any_sync(0xFFFFFFFFu, cls[j]);
-      rank[j] = valid[j] ? wcnt[warp][cls[j]] + __popc(peers & lt) : 0u;
-      __syncwarp();
-      if (valid[j] && lane == (uint32_t)(__ffs(peers) - 1)) wcnt[warp][cls[j]] += __popc(peers);
-      __syncwarp();
-    }
-    __syncthreads();
-    // per class: the count before each warp's pixels (in place), and the running count
-    for (uint32_t k = t; k < n_classes; k += kSmThreads) {
-      uint32_t acc = seen[k];
-#pragma unroll
-      for (uint32_t w = 0; w < kSmWarps; w++) {
-        const uint32_t c = wcnt[w][k];
-        wcnt[w][k] = acc;
-        acc += c;
-      }
-      seen[k] = acc;
-    }
-    __syncthreads();
-    uint32_t didx[4], dcount = 0;
-    bool draw[4];
-#pragma unroll
-    for (uint32_t j = 0; j < 4; j++) {
-      const uint32_t p = win + warp * 128 + j * 32 + lane;
-      draw[j] = false;
-      if (valid[j]) {
-        rank[j] += wcnt[warp][cls[j]];  // pixels of this class before p
-        if (rank[j] < bsz[cls[j]]) atomicMax(&slots[boff[cls[j]] + rank[j]], p + 1);
-        else draw[j] = true;
-      }
-      const uint32_t m = __ballot_sync(0xFFFFFFFFu, draw[j]);
-      didx[j] = dcount + __popc(m & lt);
-      dcount += __popc(m);
-    }
-    if (lane == 0) wd[warp] = dcount;
-    __syncthreads();
-    uint32_t before = 0, total = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kSmWarps; w++) {
-      before += w < warp ? wd[w] : 0;
-      total += wd[w];
-    }
-    if (total) {
-      const uint32_t need = (d_base + total - 1) / kMtN;  // last block this step reads
-      while (gen <= need) {
-        mt_twist(ring[(gen + 2) % 3], ring[gen % 3]);
-        gen++;
-      }
-#pragma unroll
-      for (uint32_t j = 0; j < 4; j++)
-        if (draw[j]) {
-          const uint32_t d = d_base + before + didx[j];
-          const uint32_t v = mt_temper(ring[(d / kMtN) % 3][d % kMtN]);
-          const uint32_t s = reservoir_slot(v, rank[j]);
-          if (s < bsz[cls[j]]) atomicMax(&slots[boff[cls[j]] + s], win + warp * 128 + j * 32 + lane + 1);
-        }
-      d_base += total;
-    }
+  for (int b = 0; b < BITS; b++) flip[b] = ((lane + 1u) >> b) & 1u ? 0u : 0xFFFFFFFFu;
+  if constexpr (WIDE) {
+    for (uint32_t l = lane; l <= n_classes; l += 32) s_cnt[warp][l] = l ? c0[(size_t)(l - 1) * segs] : 0u;
     __syncwarp();
-    for (uint32_t k = lane; k < n_classes; k += 32) wcnt[warp][k] = 0;
-    __syncthreads();
+  } else {
+    cnt = lane < n_classes ? c0[(size_t)lane * segs] : 0u;
   }
-  // gather the buckets in class order, sort, write
-  uint32_t pos = 0;
-  for (uint32_t k = 0; k < n_classes; k++) {
-    const uint32_t f = min(seen[k], bsz[k]);
-    for (uint32_t s = t; s < f; s += kSmThreads) keys[pos + s] = slots[boff[k] + s] - 1;
-    pos += f;
+  const uint32_t *dr = draws + g.draw_off + draw0[g.seg0 + s_beg];
+  uint32_t *sl = slots + (size_t)im * stride;
+  // The few pixels that may take a slot queue up, and are settled 32 at a time.
+  __shared__ __align__(16) uint4 s_q[kSmWarps][64];  // label, rank, draw, pixel + 1
+  uint4 *q = s_q[warp];
+  uint32_t nq = 0;
+  auto take = [&](uint32_t count) {
+    if (lane < count) {
+      const uint4 e = q[lane];
+      const uint32_t size = bsz[e.x], slot = e.y < size ? e.y : reservoir_slot(e.z, e.y);
+      if (slot < size) atomicMax(&sl[boff[e.x] + slot], e.w);
+    }
+  };
+#pragma unroll 1
+  for (uint32_t p0 = p_beg; p0 < p_end; p0 += 32 * kSegGroup) {
+    uint32_t rows[kSegGroup], rank[kSegGroup], v[kSegGroup];
+#pragma unroll
+    for (uint32_t i = 0; i < kSegGroup; i++) rows[i] = nxt[i] <= n_classes ? nxt[i] : 0u;  // a larger label is an error
+    load_rows(p0 + 32 * kSegGroup);
+    // ranks and draws, the draws loaded together
+#pragma unroll
+    for (uint32_t i = 0; i < kSegGroup; i++) {
+      const uint32_t lab = rows[i];
+      uint32_t c;
+      if constexpr (WIDE) {
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, lab);
+        c = s_cnt[warp][lab] + __popc(peers & lt);
+        __syncwarp();
+        if ((peers & lt) == 0u) s_cnt[warp][lab] += __popc(peers);
+        __syncwarp();
+      } else {
+        uint32_t row = 0xFFFFFFFFu;  // lane k: the row's pixels of class k
+#pragma unroll
+        for (int b = 0; b < BITS; b++) row &= __ballot_sync(0xFFFFFFFFu, lab & (1u << b)) ^ flip[b];
+        c = __shfl_sync(0xFFFFFFFFu, cnt, lab - 1u) + __popc(__shfl_sync(0xFFFFFFFFu, row, lab - 1u) & lt);
+        cnt += __popc(row);
+      }
+      const bool draw = c >= bsz[lab];
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, draw);
+      rank[i] = c;
+      v[i] = draw ? __ldg(dr + __popc(m & lt)) : 0u;  // 0: takes slot c
+      dr += __popc(m);
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kSegGroup; i++) {
+      const uint32_t lab = rows[i];
+      const bool may = lab != 0u && __umulhi(v[i], rank[i]) < bsz[lab];
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, may);
+      if (m == 0u) continue;
+      if (may) q[nq + __popc(m & lt)] = make_uint4(lab, rank[i], v[i], p0 + 32 * i + lane + 1);
+      nq += __popc(m);
+      if (nq >= 32) {
+        __syncwarp();
+        take(32);
+        nq -= 32;
+        const uint4 e = q[32 + lane];  // the rest moves down
+        __syncwarp();
+        if (lane < nq) q[lane] = e;
+        __syncwarp();
+      }
+    }
   }
-  for (uint32_t i = pos + t; i < sort_n; i += kSmThreads) keys[i] = 0xFFFFFFFFu;
-  __syncthreads();
-  bitonic_sort(keys, sort_n);
+  __syncwarp();
+  take(nq);
+}
+
+// The filled slots of an image, sorted (its samples), one CTA per image.  A pixel
+// fills at most one slot, so images of up to kBitmapPixels are sorted by a bitmap in
+// shared memory (set the pixels' bits, list them in order); larger ones by the
+// bitonic sort.  Dynamic shared memory: the bitmap, or sort_n words.
+constexpr uint32_t kBitmapPixels = 1u << 20;  // 128 KB
+template <bool BITMAP>
+__global__ void __launch_bounds__(kSmThreads) k_bucket_samples(const SampImage *__restrict__ imgs,
+                                                               const uint32_t *__restrict__ bucket_size,
+                                                               const uint32_t *__restrict__ class_tot,
+                                                               uint32_t n_classes, const uint32_t *__restrict__ slots,
+                                                               uint32_t stride, uint32_t sort_n,
+                                                               uint32_t *__restrict__ out,
+                                                               uint32_t *__restrict__ out_count) {
+  extern __shared__ __align__(16) uint32_t keys[];
+  __shared__ uint32_t wtot[kSmWarps];
+  const uint32_t im = blockIdx.x, t = threadIdx.x;
+  const SampImage g = imgs[im];
+  const uint32_t *sl = slots + (size_t)im * stride;
   uint32_t *o = out + g.out_off;
-  for (uint32_t i = t; i < pos; i += kSmThreads) o[i] = keys[i];
-  if (t == 0) {
-    out_count[im] = pos;
-    if (bad) atomicMin(err, im);
+  if constexpr (BITMAP) {
+    const uint32_t words = (g.n_pix + 31) / 32, per = ((words + kSmThreads - 1) / kSmThreads + 3) / 4 * 4;
+    for (uint32_t i = t; i < (words + 3) / 4; i += kSmThreads) reinterpret_cast<uint4 *>(keys)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    for (uint32_t i = t; i < stride; i += kSmThreads) {
+      const uint32_t p = sl[i] - 1u;  // an empty slot holds 0
+      if (p < g.n_pix) atomicOr(&keys[p >> 5], 1u << (p & 31));
+    }
+    __syncthreads();
+    const uint32_t b = min(words, t * per), e = min(words, b + per);
+    uint32_t mine = 0, total;
+    for (uint32_t i = b; i < e; i++) mine += __popc(keys[i]);
+    uint32_t pos = block_scan(mine, wtot, &total);
+    for (uint32_t i = b; i < e; i++)
+      for (uint32_t m = keys[i]; m; m &= m - 1) o[pos++] = 32 * i + (uint32_t)__ffs((int)m) - 1;
+    if (t == 0) out_count[im] = total;
+  } else {
+    uint32_t mine = 0, total;
+    for (uint32_t k = t; k < n_classes; k += kSmThreads)
+      mine += min(class_tot[(size_t)im * n_classes + k], bucket_size[k]);
+    block_scan(mine, wtot, &total);
+    for (uint32_t i = t; i < sort_n; i += kSmThreads) keys[i] = (i < stride ? sl[i] : 0u) - 1u;  // empty: last
+    __syncthreads();
+    bitonic_sort(keys, sort_n);
+    for (uint32_t i = t; i < total; i += kSmThreads) o[i] = keys[i];
+    if (t == 0) out_count[im] = total;
   }
 }
 
@@ -640,7 +820,7 @@ struct DescLayout {
     count = crc + 4ull * n;
     err = count + 4ull * n;
     bucket = err + 16;  // err[0], err[1]: errors; err[2]: the scan's work counter
-    bytes = bucket + 4ull * n_classes;
+    bytes = bucket + 8ull * n_classes;  // sizes, then offsets
     this->n_items = n_items;
   }
 };
@@ -667,7 +847,63 @@ const uint32_t *shift_constants() {
   return tab.data();
 }
 
-// Uploads the descriptor block and launches the two kernels on a batch that is
+// The class-weighted sampler's kernels on a batch (images and checksums in place).
+// Its scratch -- segment counts, draws, slots -- belongs to the context, like its
+// stream: calls on one context are serialised.
+int launch_class_weighted(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32_t n, const uint8_t *host_desc,
+                          const DescLayout &lay, const uint8_t *labels, const SampImage *imgs, const uint32_t *crc,
+                          const uint32_t *bucket, uint32_t *out, uint32_t *counts, uint32_t *err, uint64_t *launched) {
+  cudaStream_t st = ctx->stream;
+  const uint32_t K = s->n_classes;
+  const SampImage *h = reinterpret_cast<const SampImage *>(host_desc + lay.imgs);
+  auto segs_of = [&](uint32_t i) { return (h[i].n_pix + kSeg - 1) / kSeg; };
+  const uint32_t segs = h[n - 1].seg0 + segs_of(n - 1);
+  uint64_t draw_words = 0;
+  for (uint32_t i = 0; i < n; i++) draw_words = std::max(draw_words, h[i].draw_off + ((uint64_t)h[i].n_pix + 3) / 4 * 4);
+  const size_t slot_bytes = (size_t)n * std::max(1u, pl.stride) * 4;
+  PD_TRY(ctx->sm_counts.ensure(((size_t)segs * (K + 1) + (size_t)n * (K + 1)) * 4));
+  PD_TRY(ctx->sm_draws.ensure(draw_words * 4));
+  PD_TRY(ctx->sm_slots.ensure(slot_bytes));
+  uint32_t *c = ctx->sm_counts.as<uint32_t>(), *draw0 = c + (size_t)segs * K, *tot = draw0 + segs,
+           *n_draws = tot + (size_t)n * K, *draws = ctx->sm_draws.as<uint32_t>(), *slots = ctx->sm_slots.as<uint32_t>();
+  const uint32_t *bsz = bucket, *boff = bucket + K;
+  PD_CUDA(cudaMemsetAsync(slots, 0, slot_bytes, st));
+  *launched = 2;
+  // CTAs of images [first, last): the segments of the largest, up to 65535 images a grid
+  auto grid_of = [&](uint32_t first, uint32_t last, uint32_t per_warp) {
+    uint32_t most = 0;
+    for (uint32_t i = first; i < last; i++) most = std::max(most, segs_of(i));
+    return dim3((most + kSmWarps * per_warp - 1) / (kSmWarps * per_warp), last - first);
+  };
+  const size_t count_smem = (size_t)kSmWarps * (std::min(K, 32u) + 1) * 128;
+  for (uint32_t first = 0; first < n; first += 65535, ++*launched)
+    k_class_counts<<<grid_of(first, std::min(n, first + 65535), 1), kSmThreads, count_smem, st>>>(labels, imgs, first, K, c,
+                                                                                               err);
+  k_class_prefix<<<n, kSmThreads, 0, st>>>(imgs, K, bsz, c, draw0, tot, n_draws);
+  PD_CUDA(cudaGetLastError());
+  for (uint32_t first = 0; first < n;) {
+    uint32_t last = first + 1;  // a group: up to the next image whose draws start over
+    while (last < n && last - first < 65535 && h[last].draw_off != 0) last++;
+    k_mt_draws<<<last - first, kMtThreads, 0, st>>>(imgs, first, crc, s->seed, n_draws, draws);
+    auto res = K < 16 ? k_reservoir<4> : K <= 32 ? k_reservoir<6> : k_reservoir<8>;
+    res<<<grid_of(first, last, kSegRun), kSmThreads, 0, st>>>(labels, imgs, first, K, bsz, boff, c, draw0, draws, pl.stride, slots);
+    PD_CUDA(cudaGetLastError());
+    *launched += 2;
+    first = last;
+  }
+  uint32_t most = 0;
+  for (uint32_t i = 0; i < n; i++) most = std::max(most, h[i].n_pix);
+  const bool bitmap = most <= kBitmapPixels;
+  const size_t smem = bitmap ? ((size_t)most + 127) / 128 * 16 : (size_t)pl.sort_n * 4;
+  auto bucket_samples = bitmap ? k_bucket_samples<true> : k_bucket_samples<false>;
+  PD_CUDA(cudaFuncSetAttribute(bucket_samples, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  bucket_samples<<<n, kSmThreads, smem, st>>>(imgs, bsz, tot, K, slots, pl.stride, pl.sort_n, out, counts);
+  PD_CUDA(cudaGetLastError());
+  *launched += 1;
+  return PD_OK;
+}
+
+// Uploads the descriptor block and launches the kernels on a batch that is
 // in device memory.  counts/err stay on the device.
 int launch_batch(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32_t n, const uint8_t *data, const uint8_t *labels, uint32_t *out, uint32_t *counts, const DescLayout &lay,
                  uint8_t *dev_desc, const void *host_desc, cudaEvent_t *ev) {
@@ -681,34 +917,38 @@ int launch_batch(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32
   int sms = 0, per_sm = 0;
   PD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sample_scan, kSmThreads, 0));
-  const uint32_t grid = std::max(1u, std::min<uint32_t>(lay.n_items, (uint32_t)(sms * std::max(per_sm, 1))));
   PD_CUDA(cudaEventRecord(ev[0], st));
-  k_sample_scan<<<grid, kSmThreads, 0, st>>>(data, labels, imgs, item_img, lay.n_items, lay.n_crc_items,
+  // the class-weighted sampler does not need the labelled-pixel counts: checksums only
+  const uint32_t n_items = s->kind == PD_SAMPLER_UNIFORM ? lay.n_items : lay.n_crc_items;
+  const uint32_t grid = std::max(1u, std::min<uint32_t>(n_items, (uint32_t)(sms * std::max(per_sm, 1))));
+  k_sample_scan<<<grid, kSmThreads, 0, st>>>(data, labels, imgs, item_img, n_items, lay.n_crc_items,
                                              reinterpret_cast<const uint32_t *>(dev_desc + lay.shifts), crc, cnt,
                                              err + 2);
   PD_CUDA(cudaGetLastError());
   PD_CUDA(cudaEventRecord(ev[1], st));
+  uint64_t launched = 2;
   if (s->kind == PD_SAMPLER_UNIFORM) {
     const size_t smem = (size_t)pl.sort_n * 4;
     PD_CUDA(cudaFuncSetAttribute(k_sample_uniform, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_sample_uniform<<<n, kSmThreads, smem, st>>>(labels, imgs, crc, cnt, s->n_samples, s->seed, pl.sort_n, out,
                                                   counts, err);
   } else {
-    const size_t smem = ((size_t)pl.stride + pl.sort_n) * 4;
-    PD_CUDA(cudaFuncSetAttribute(k_sample_class_weighted, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_sample_class_weighted<<<n, kSmThreads, smem, st>>>(labels, imgs, crc,
-                                                         reinterpret_cast<const uint32_t *>(dev_desc + lay.bucket),
-                                                         s->n_classes, pl.stride, s->seed, pl.sort_n, out, counts, err);
+    PD_TRY(launch_class_weighted(ctx, s, pl, n, static_cast<const uint8_t *>(host_desc), lay, labels, imgs, crc,
+                                 reinterpret_cast<const uint32_t *>(dev_desc + lay.bucket), out, counts, err, &launched));
   }
   PD_CUDA(cudaGetLastError());
   PD_CUDA(cudaEventRecord(ev[2], st));
-  ctx->launches += 2;
-  ctx->sample_stats.kernel_launches += 2;
+  ctx->launches += launched;
+  ctx->sample_stats.kernel_launches += 2;  // the two phases
   return PD_OK;
 }
 
 // Fills the pinned descriptor block for images described by (data_lo, data
 // bytes, lab_off, n_pix, out_off) and returns the item count.
+// Words of MT19937 outputs kept at a time by the class-weighted sampler (images are
+// taken in groups of at most that many pixels, one image at least).
+constexpr uint64_t kDrawGroup = 1ull << 29;
+
 struct ImagePlace {
   uint64_t data_lo, data_end, lab_off, out_off;
   uint64_t data_bytes;
@@ -735,9 +975,16 @@ int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> 
   uint32_t *crc = reinterpret_cast<uint32_t *>(h + lay.crc);
   uint32_t *cnt = reinterpret_cast<uint32_t *>(h + lay.count);
   uint32_t ic = 0, il = (uint32_t)n_crc;
+  uint64_t segs = 0, draws = 0;
   for (uint32_t i = 0; i < n; i++) {
     const ImagePlace &p = place[i];
-    im[i] = SampImage{p.data_lo, p.data_end, p.lab_off, p.out_off, p.n_pix, (p.n_pix + 15) / 16, slices[i], ic, il, 0};
+    // draws are kept for kDrawGroup words of images at a time (one image at least)
+    const uint64_t dw = ((uint64_t)p.n_pix + 3) / 4 * 4;
+    if (draws && draws + dw > kDrawGroup) draws = 0;
+    im[i] = SampImage{p.data_lo, p.data_end, p.lab_off, p.out_off, p.n_pix, (p.n_pix + 15) / 16, slices[i], ic, il,
+                      (uint32_t)segs, draws};
+    segs += (p.n_pix + kSeg - 1) / kSeg;
+    draws += dw;
     for (uint32_t k = 0; k < slices[i]; k++) item_img[ic++] = i;
     for (uint32_t k = 0; k < chunks[i]; k++) item_img[il++] = i;
     // the initial value 0xFFFFFFFF carried past the image bytes, and the final XOR
@@ -748,11 +995,19 @@ int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> 
       crc[i] = crc[i - 1];
     cnt[i] = 0;
   }
+  PD_CHECK(segs < (1ull << 31), PD_ERR_UNSUPPORTED, "batch too large");
   std::memcpy(h + lay.shifts, shift_constants(), 4ull * kShiftWords);
   reinterpret_cast<uint32_t *>(h + lay.err)[0] = kNoError;  // first image with a label above nClasses
   reinterpret_cast<uint32_t *>(h + lay.err)[1] = kNoError;  // first image whose draws hit the block limit
   reinterpret_cast<uint32_t *>(h + lay.err)[2] = 0;         // next work item of the scan
-  if (!pl.bucket.empty()) std::memcpy(h + lay.bucket, pl.bucket.data(), pl.bucket.size() * 4);
+  if (!pl.bucket.empty()) {
+    uint32_t *b = reinterpret_cast<uint32_t *>(h + lay.bucket), *off = b + pl.bucket.size(), o = 0;
+    for (size_t k = 0; k < pl.bucket.size(); k++) {
+      b[k] = pl.bucket[k];
+      off[k] = o;
+      o += pl.bucket[k];
+    }
+  }
   *lay_out = lay;
   return PD_OK;
 }
