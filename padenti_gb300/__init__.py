@@ -313,6 +313,13 @@ class _Ctx:
             self.h = None
 
 
+def _store_tree(tree: Tree, n: int, lc, ft, th, po) -> None:
+    """The trained arrays back into the tree (which holds them already where they are views of its own)."""
+    for dst, src in ((tree.left_child, lc), (tree.features, ft), (tree.thresholds, th), (tree.posteriors, po)):
+        if dst.ctypes.data != src.ctypes.data:
+            dst[:n] = src
+
+
 class TreeTrainer(_Ctx):
     """CLTreeTrainer (cl_tree_trainer.hpp:115-120) on one GB300."""
 
@@ -359,7 +366,7 @@ class TreeTrainer(_Ctx):
         prior = np.ascontiguousarray(ts.priors, np.float32)
         check(lib().pd_train_tree(self.h, C.byref(params.c()), tree.id, start_depth, end_depth, _ptr(prior),
                                   _ptr(lc), _ptr(ft), _ptr(th), _ptr(po)))
-        tree.left_child[:n], tree.features[:n], tree.thresholds[:n], tree.posteriors[:n] = lc, ft, th, po
+        _store_tree(tree, n, lc, ft, th, po)
 
     def train_proposed(self, tree: Tree, ts: TrainingSet, params: TreeTrainerParameters, proposer: "ProposalNetwork",
                        n_proposed: int, end_depth: int | None = None) -> None:
@@ -375,7 +382,7 @@ class TreeTrainer(_Ctx):
         prior = np.ascontiguousarray(ts.priors, np.float32)
         check(lib().pd_train_tree_proposed(self.h, proposer.h, C.byref(params.c()), n_proposed, tree.id, 1, end_depth,
                                            _ptr(prior), _ptr(lc), _ptr(ft), _ptr(th), _ptr(po)))
-        tree.left_child[:n], tree.features[:n], tree.thresholds[:n], tree.posteriors[:n] = lc, ft, th, po
+        _store_tree(tree, n, lc, ft, th, po)
 
     def train_sharded(self, tree: Tree, ts: TrainingSet, params: TreeTrainerParameters, f_begin: int, f_end: int,
                       exchange, end_depth: int | None = None) -> None:
@@ -398,7 +405,7 @@ class TreeTrainer(_Ctx):
         check(lib().pd_train_tree_sharded(self.h, C.byref(params.c()), f_begin, f_end, C.cast(cb, C.c_void_p), None,
                                           tree.id, 1, end_depth, _ptr(prior), _ptr(lc), _ptr(ft), _ptr(th),
                                           _ptr(po)))
-        tree.left_child[:n], tree.features[:n], tree.thresholds[:n], tree.posteriors[:n] = lc, ft, th, po
+        _store_tree(tree, n, lc, ft, th, po)
 
     def records(self) -> np.ndarray:
         """The records (one per split node) of the last training call; set_tuning("records", 1)

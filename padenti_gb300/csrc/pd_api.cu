@@ -95,9 +95,9 @@ extern "C" int pd_ctx_destroy(pd_ctx *ctx) {
   cudaStreamSynchronize(ctx->stream);
   DevBuf *bufs[] = {&ctx->pixels, &ctx->img_off, &ctx->img_wh, &ctx->s_xy, &ctx->s_img, &ctx->s_label,
                     &ctx->log2_tab, &ctx->magic_tab, &ctx->snode, &ctx->act[0], &ctx->act[1], &ctx->act_rec[0], &ctx->act_rec[1], &ctx->s_rec, &ctx->act_slot[0],
-                    &ctx->act_slot[1], &ctx->flags, &ctx->scan_blocks, &ctx->slot_adj, &ctx->scatter_err,
-                    &ctx->cand_feat, &ctx->cand_thr, &ctx->cand_perm, &ctx->cand_ord, &ctx->parent, &ctx->xlog2_tab, &ctx->split_par, &ctx->hist, &ctx->g32, &ctx->items, &ctx->hist_queue,
-                    &ctx->zero_slots, &ctx->split_out, &ctx->split_cl, &ctx->recheck, &ctx->split_scratch, &ctx->fused_scratch, &ctx->t_lc,
+                    &ctx->act_slot[1], &ctx->flags, &ctx->scan_blocks, &ctx->slot_adj, 
+                    &ctx->cand_feat, &ctx->cand_thr, &ctx->cand_perm, &ctx->cand_ord, &ctx->parent, &ctx->xlog2_tab, &ctx->hist, &ctx->g32, &ctx->items, &ctx->hist_queue,
+                    &ctx->split_res, &ctx->d_pre, &ctx->d_splits, &ctx->split_scratch, &ctx->fused_scratch, &ctx->t_lc,
                     &ctx->t_feat, &ctx->t_thr, &ctx->t_post, &ctx->f_lc, &ctx->f_feat, &ctx->f_thr,
                     &ctx->f_post, &ctx->f_meta, &ctx->f_cand, &ctx->p_img, &ctx->p_mask, &ctx->p_out,
                     &ctx->nm_map[0], &ctx->nm_map[1], &ctx->nm_off, &ctx->nm_label, &ctx->np_map[0],
@@ -134,6 +134,10 @@ extern "C" int pd_ctx_destroy(pd_ctx *ctx) {
   ctx->h_lab.release();
   ctx->h_stage.release();
   ctx->h_items.release();
+  ctx->h_pre.release();
+  ctx->h_splits.release();
+  ctx->h_res.release();
+  ctx->h_chk.release();
   for (auto &ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
   cudaStreamDestroy(ctx->stream);

@@ -47,11 +47,14 @@ struct pd_ctx {
   std::vector<uint32_t> root_class_tot;  // samples per class (the root's class totals)
   pd_upload_stats upload_stats{};        // of the last pd_dataset_upload
   pd::HostBuf h_stage;           // pinned staging of the per-sample upload arrays
-  pd::HostBuf h_items;           // pinned staging of a histogram launch's work list
+  pd::HostBuf h_items;           // pinned staging of a histogram launch's work list, zero and split slots
+  // pinned staging of a frontier slice (nodes, class totals) and of a level's splits
+  // (SlotNext, parameters), the results of a slice, the reassignment's check
+  pd::HostBuf h_pre, h_splits, h_res, h_chk;
+  pd::DevBuf d_pre, d_splits;
   pd::DevBuf log2_tab;  // double log2(n), n < log2_len
   pd::DevBuf xlog2_tab; // float c*log2(c), c < min(log2_len, 65536): the fused split's filter
   pd::DevBuf parent;    // [slots] parent term of the exact gain, for the fused split
-  pd::DevBuf split_par; // [slots][D + 1] feature values and threshold of each winner
   pd::DevBuf magic_tab; // uint32 RoundDiv multiplier by depth value (65536)
   uint64_t log2_len = 0;
 
@@ -63,12 +66,19 @@ struct pd_ctx {
   pd::DevBuf flags;                  // uint8 per active sample
   pd::DevBuf scan_blocks;            // uint64 per scan block
   pd::DevBuf slot_adj;               // int64 [4] per slot: adjL, adjR, kL, kR
-  pd::DevBuf scatter_err;            // uint32 error counter
   pd::DevBuf cand_feat, cand_thr, cand_perm;
   pd::DevBuf cand_ord;       // [slots][F] original candidate index of each column
   pd::DevBuf hist, g32;
-  pd::DevBuf items, zero_slots, hist_queue;
-  pd::DevBuf split_out, split_cl, recheck, split_scratch, fused_scratch;
+  pd::DevBuf items, hist_queue;  // work list, slots to zero, slots to split
+  // Results of a slice in one buffer, for one copy back: SplitOut [n], left class
+  // counts [n][K], feature values and threshold [n][D + 1], rechecked candidates
+  // (set_results).
+  pd::DevBuf split_res;
+  void *res_out = nullptr, *res_par = nullptr;
+  uint32_t *res_cl = nullptr;
+  unsigned long long *res_recheck = nullptr;
+  size_t res_bytes = 0;
+  pd::DevBuf split_scratch, fused_scratch;
   pd::DevBuf t_lc, t_feat, t_thr, t_post;  // device copy of the tree being trained
   // ---- node map of features that read the tree (tree_feature) ----
   pd::DevBuf nm_map[2];   // int32 node per pixel of every training image, this depth's and the next

@@ -507,12 +507,15 @@ __global__ void __launch_bounds__(kSmThreads) k_class_counts(const uint8_t *__re
 
 // counts of an image's segments -> the pixels of each class before the segment (in
 // place), the class totals, and the index of each segment's first draw: a pixel
-// draws when its class's bucket is full.  One CTA per image, a warp per class.
+// draws when its class's bucket is full.  One CTA per image, a warp per class; it also
+// empties the image's slots.
 __global__ void __launch_bounds__(kSmThreads) k_class_prefix(const SampImage *__restrict__ imgs, uint32_t n_classes,
                                                              const uint32_t *__restrict__ bucket_size,
                                                              uint32_t *__restrict__ counts, uint32_t *__restrict__ draw0,
                                                              uint32_t *__restrict__ class_tot,
-                                                             uint32_t *__restrict__ n_draws) {
+                                                             uint32_t *__restrict__ n_draws,
+                                                             uint32_t *__restrict__ slots, uint32_t stride) {
+  for (uint32_t i = threadIdx.x; i < stride; i += kSmThreads) slots[(size_t)blockIdx.x * stride + i] = 0u;
   const SampImage g = imgs[blockIdx.x];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t segs = (g.n_pix + kSeg - 1) / kSeg;
@@ -867,7 +870,6 @@ int launch_class_weighted(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &p
   uint32_t *c = ctx->sm_counts.as<uint32_t>(), *draw0 = c + (size_t)segs * K, *tot = draw0 + segs,
            *n_draws = tot + (size_t)n * K, *draws = ctx->sm_draws.as<uint32_t>(), *slots = ctx->sm_slots.as<uint32_t>();
   const uint32_t *bsz = bucket, *boff = bucket + K;
-  PD_CUDA(cudaMemsetAsync(slots, 0, slot_bytes, st));
   *launched = 2;
   // CTAs of images [first, last): the segments of the largest, up to 65535 images a grid
   auto grid_of = [&](uint32_t first, uint32_t last, uint32_t per_warp) {
@@ -879,7 +881,7 @@ int launch_class_weighted(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &p
   for (uint32_t first = 0; first < n; first += 65535, ++*launched)
     k_class_counts<<<grid_of(first, std::min(n, first + 65535), 1), kSmThreads, count_smem, st>>>(labels, imgs, first, K, c,
                                                                                                err);
-  k_class_prefix<<<n, kSmThreads, 0, st>>>(imgs, K, bsz, c, draw0, tot, n_draws);
+  k_class_prefix<<<n, kSmThreads, 0, st>>>(imgs, K, bsz, c, draw0, tot, n_draws, slots, pl.stride);
   PD_CUDA(cudaGetLastError());
   for (uint32_t first = 0; first < n;) {
     uint32_t last = first + 1;  // a group: up to the next image whose draws start over

@@ -177,6 +177,21 @@ static int check_params(const pd_ctx *ctx, const pd_train_params *p) {
   return PD_OK;
 }
 
+// Lays the results of a slice of n nodes out in one buffer (kept; grown as needed).
+static int set_results(pd_ctx *ctx, uint32_t n) {
+  auto up = [](size_t v) { return (v + 15) / 16 * 16; };
+  const size_t K = ctx->cfg.n_classes, par = up((size_t)n * (ctx->cfg.feat_dim + 1) * feat_size(ctx->cfg.feat_type));
+  const size_t out = up((size_t)n * sizeof(SplitOut)), cl = up((size_t)n * K * 4);
+  PD_TRY(ctx->split_res.ensure(out + cl + par + 16));
+  uint8_t *b = ctx->split_res.as<uint8_t>();
+  ctx->res_out = b;
+  ctx->res_cl = reinterpret_cast<uint32_t *>(b + out);
+  ctx->res_par = b + out + cl;
+  ctx->res_recheck = reinterpret_cast<unsigned long long *>(b + out + cl + par);
+  ctx->res_bytes = out + cl + par + 8;
+  return PD_OK;
+}
+
 // Scratch sized for `slots` frontier nodes.
 static int ensure_slice(pd_ctx *ctx, const pd_train_params *p, uint32_t slots) {
   const uint64_t F = p->n_features, T = p->n_thresholds, K = ctx->cfg.n_classes;
@@ -187,11 +202,7 @@ static int ensure_slice(pd_ctx *ctx, const pd_train_params *p, uint32_t slots) {
   PD_TRY(ctx->cand_ord.ensure(slots * F * 4));
   PD_TRY(ctx->hist.ensure(slots * K * T * F * 4));
   PD_TRY(ctx->g32.ensure(slots * T * F * 4));
-  PD_TRY(ctx->split_out.ensure(slots * sizeof(SplitOut)));
-  PD_TRY(ctx->split_par.ensure(slots * (ctx->cfg.feat_dim + 1) * fs));
-  PD_TRY(ctx->split_cl.ensure(slots * K * 4));
-  PD_TRY(ctx->recheck.ensure(sizeof(unsigned long long) + slots * K * 4 + slots * 4));
-  return PD_OK;
+  return set_results(ctx, slots);
 }
 
 static uint64_t slot_bytes(const pd_ctx *ctx, const pd_train_params *p) {
@@ -272,13 +283,15 @@ static int launch_candidates(pd_ctx *ctx, const pd_train_params *p, uint32_t tre
 // and launches the histogram kernels.  With `split_slots` non-null, nodes whose
 // samples fit one work item get their split fused into the histogram kernel (multi
 // = 2, rows never written) and the other slots are returned for the split kernels;
-// h_class_tot: their class totals [n][K] on the host.
+// h_class_tot: their class totals [n][K] on the host; *d_split_list: those slots on the
+// device.
 template <class P>
 static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *off, uint32_t n,
                        const SampleRec *d_rec, uint64_t *n_items_out, cudaEvent_t ev_before = nullptr,
                        cudaEvent_t ev_after = nullptr, std::vector<uint32_t> *split_slots = nullptr,
                        const uint32_t *d_class_tot = nullptr, const uint32_t *h_class_tot = nullptr,
-                       const uint32_t *d_ord = nullptr, const PropSrc *prop = nullptr) {
+                       const uint32_t *d_ord = nullptr, const PropSrc *prop = nullptr,
+                       const uint32_t **d_split_list = nullptr) {
   using FeatT = typename P::feat_t;
   const uint32_t F = p->n_features, T = p->n_thresholds, K = ctx->cfg.n_classes;
   const uint32_t tiles = (F + kTileF - 1) / kTileF;
@@ -334,7 +347,7 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
     at[b] = n_items;
     n_items += n_small[b];
   }
-  PD_TRY(ctx->h_items.ensure(std::max<uint64_t>(1, n_items) * sizeof(WorkItem)));
+  PD_TRY(ctx->h_items.ensure(n_items * sizeof(WorkItem) + (size_t)n * 8 + 16));
   WorkItem *items = ctx->h_items.as<WorkItem>();
   uint64_t ni = 0;
   std::vector<uint32_t> zero;
@@ -369,22 +382,31 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
     }
   }
   *n_items_out = n_items * tiles;
-  PD_TRY(ctx->items.ensure(std::max<size_t>(1, n_items) * sizeof(WorkItem)));
-  PD_TRY(ctx->zero_slots.ensure(std::max<size_t>(1, zero.size()) * 4));
+  // one copy: the work list, the slots whose rows are added to (zeroed first), the
+  // slots for the split kernels
+  uint32_t *lists = reinterpret_cast<uint32_t *>(items + n_items);
+  size_t n_lists = zero.size();
+  if (!zero.empty()) memcpy(lists, zero.data(), zero.size() * 4);
+  if (split_slots && !split_slots->empty()) {
+    memcpy(lists + n_lists, split_slots->data(), split_slots->size() * 4);
+    n_lists += split_slots->size();
+  }
+  const size_t list_bytes = n_items * sizeof(WorkItem) + n_lists * 4;
+  PD_TRY(ctx->items.ensure(list_bytes + 16));
+  if (list_bytes) PD_CUDA(h2d(ctx, ctx->items.ptr, items, list_bytes));
+  const uint32_t *d_lists = reinterpret_cast<const uint32_t *>(ctx->items.as<WorkItem>() + n_items);
+  if (d_split_list) *d_split_list = d_lists + zero.size();
   const uint64_t per_slot = (uint64_t)K * T * F;
   if (!zero.empty()) {
-    PD_CUDA(h2d(ctx, ctx->zero_slots.ptr, zero.data(), zero.size() * 4));
-    k_zero_slots<<<1216, 256, 0, ctx->stream>>>(ctx->hist.as<uint32_t>(), ctx->zero_slots.as<uint32_t>(),
-                                                (uint32_t)zero.size(), per_slot);
+    k_zero_slots<<<1216, 256, 0, ctx->stream>>>(ctx->hist.as<uint32_t>(), d_lists, (uint32_t)zero.size(), per_slot);
     PD_CUDA(cudaGetLastError());
+    ctx->launches++;
   }
-  if (!zero.empty()) ctx->launches++;
   if (!n_items) {
     if (ev_before) PD_CUDA(cudaEventRecord(ev_before, ctx->stream));
     if (ev_after) PD_CUDA(cudaEventRecord(ev_after, ctx->stream));
     return PD_OK;
   }
-  PD_CUDA(h2d(ctx, ctx->items.ptr, items, n_items * sizeof(WorkItem)));
   FusedSplit fs;
   memset(&fs, 0, sizeof(fs));
   if (split_slots) {
@@ -405,9 +427,9 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
     ctx->launches++;
     fs.parent = ctx->parent.as<double>();
     fs.tiles = tiles;
-    fs.out = ctx->split_out.as<SplitOut>();
-    fs.out_cl = ctx->split_cl.as<uint32_t>();
-    fs.rechecked = ctx->recheck.as<unsigned long long>();
+    fs.out = static_cast<SplitOut *>(ctx->res_out);
+    fs.out_cl = ctx->res_cl;
+    fs.rechecked = ctx->res_recheck;
     fs.ord = d_ord;
   }
   HistGrid g;
@@ -497,9 +519,9 @@ static int launch_split(pd_ctx *ctx, const pd_train_params *p, uint32_t n, const
   a.part_best = reinterpret_cast<SplitPart *>(ctx->split_scratch.as<uint8_t>() + (size_t)all * 8);
   a.slot_list = d_slot_list;
   a.ord = d_ord;
-  a.out = ctx->split_out.as<SplitOut>();
-  a.out_cl = ctx->split_cl.as<uint32_t>();
-  a.rechecked = ctx->recheck.as<unsigned long long>();
+  a.out = static_cast<SplitOut *>(ctx->res_out);
+  a.out_cl = ctx->res_cl;
+  a.rechecked = ctx->res_recheck;
   const dim3 grid(parts, n);
   auto run = [&]<int KM>() -> int {
     k_split_g32<KM, CUM><<<grid, kSplitCols, 0, ctx->stream>>>(a);
@@ -593,16 +615,19 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
   ctx->records.clear();
 
   PD_TRY(ensure_log2_table(ctx, S + 2));
-  PD_TRY(ctx->t_lc.ensure(n_nodes * 4));
-  PD_TRY(ctx->t_feat.ensure(n_nodes * D * sizeof(FeatT)));
-  PD_TRY(ctx->t_thr.ensure(n_nodes * sizeof(FeatT)));
-  PD_TRY(ctx->t_post.ensure(n_nodes * K * 4));
   memcpy(posts, root_prior, sizeof(float) * K);
-  // The tree as the caller holds it goes to the device (init:33-50).
-  PD_CUDA(h2d(ctx, ctx->t_lc.ptr, lc, n_nodes * 4));
-  PD_CUDA(h2d(ctx, ctx->t_feat.ptr, feats, n_nodes * D * sizeof(FeatT)));
-  PD_CUDA(h2d(ctx, ctx->t_thr.ptr, thrs, n_nodes * sizeof(FeatT)));
-  PD_CUDA(h2d(ctx, ctx->t_post.ptr, posts, n_nodes * K * 4));
+  if (ctx->tree_feature) {
+    // A feature that reads the tree needs it on the device, as the caller holds it
+    // (init:33-50); the trainer itself reads splits by frontier slot.
+    PD_TRY(ctx->t_lc.ensure(n_nodes * 4));
+    PD_TRY(ctx->t_feat.ensure(n_nodes * D * sizeof(FeatT)));
+    PD_TRY(ctx->t_thr.ensure(n_nodes * sizeof(FeatT)));
+    PD_TRY(ctx->t_post.ensure(n_nodes * K * 4));
+    PD_CUDA(h2d(ctx, ctx->t_lc.ptr, lc, n_nodes * 4));
+    PD_CUDA(h2d(ctx, ctx->t_feat.ptr, feats, n_nodes * D * sizeof(FeatT)));
+    PD_CUDA(h2d(ctx, ctx->t_thr.ptr, thrs, n_nodes * sizeof(FeatT)));
+    PD_CUDA(h2d(ctx, ctx->t_post.ptr, posts, n_nodes * K * 4));
+  }
 
   PD_TRY(ctx->snode.ensure(S * 4 + 4));
   for (int b = 0; b < 2; b++) {
@@ -611,9 +636,15 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
     PD_TRY(ctx->act_rec[b].ensure(S * sizeof(SampleRec) + sizeof(SampleRec)));
   }
   PD_TRY(ctx->flags.ensure(S + 16));
-  PD_TRY(ctx->scan_blocks.ensure((S / kScanItems + 2) * 8 + 16));
-  PD_TRY(ctx->scatter_err.ensure(16));
+  PD_TRY(ctx->scan_blocks.ensure((S / kScanItems + 4) * 8));
+  PD_TRY(ctx->h_chk.ensure(16));
   PD_CUDA(cudaMemsetAsync(ctx->snode.ptr, 0, S * 4, st));
+  // the regrouping of a level is checked at the next level's synchronisation: until
+  // then a position it missed (a feature that is no function of its inputs) reads
+  // sample 0
+  PD_CUDA(cudaMemsetAsync(ctx->act[1].ptr, 0, S * 4, st));
+  PD_CUDA(cudaMemsetAsync(ctx->act_slot[1].ptr, 0, S * 4, st));
+  PD_CUDA(cudaMemsetAsync(ctx->act_rec[1].ptr, 0, S * sizeof(SampleRec), st));
   if (ctx->tree_feature) {
     // every pixel starts at the root (traverse_ts.hpp:146-163 fills the node image with 0)
     PD_CHECK(ctx->nm_pixels, PD_ERR_STATE, "the training set was uploaded before the plugin was compiled");
@@ -629,89 +660,113 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
   }
   PD_CUDA(cudaGetLastError());
 
-  std::vector<uint32_t> node_tot(n_nodes, 0u), class_tot(n_nodes * K, 0u);
-  node_tot[0] = (uint32_t)S;
-  std::vector<int32_t> frontier{0};
-  std::vector<uint64_t> cur_off{0, S};
+  // the frontier: nodes, class totals [slot][K], and their ranges of active samples
+  std::vector<int32_t> frontier{0}, next;
+  std::vector<uint32_t> tot(ctx->root_class_tot), next_tot;
+  std::vector<uint64_t> cur_off{0, S}, next_off;
   int cur = 0;
-  uint64_t n_act = S;
+  uint64_t n_act = S, pending = ~0ull;  // pending: samples the last regrouping must have placed (~0: none to check)
+  uint32_t pending_depth = 0;
   // slices are sized for all F_total candidates when sharded, so every rank cuts the same slices
   pd_train_params p_all = *p;
   if (shard) p_all.n_features = shard->F_total;
   const uint64_t per_slot = slot_bytes(ctx, &p_all);
   const uint32_t max_slots = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(ctx->hist_budget / per_slot, 1u << 30));
-  DevBuf d_nodes, d_ctot, d_next, d_split_list;
   std::vector<SplitOut> h_out;
-  std::vector<uint32_t> h_cl;
-  std::vector<FeatT> h_par;
-  std::vector<uint32_t> cl(K), cr(K);
+  std::vector<uint32_t> cr(K);
+  std::vector<uint8_t> split_now;
+  std::vector<uint32_t> left_cnt;  // left class counts of every slot of the level
+  std::vector<FeatT> level_par;    // feature values and threshold of every slot of the level
   cudaEvent_t *ev = ctx->ev;
+  // after a synchronisation: the last regrouping's counts, and its time
+  auto check_regroup = [&]() -> int {
+    if (pending == ~0ull) return PD_OK;
+    const unsigned long long *chk = ctx->h_chk.as<unsigned long long>();
+    const uint64_t want = pending, got = (chk[0] & 0xffffffffull) + (chk[0] >> 32);
+    pending = ~0ull;
+    PD_CHECK(chk[1] == 0 && got == want, PD_ERR_STATE,
+             "reassignment disagrees with the split counts at depth %u (%llu vs %llu samples, %u misplaced)",
+             pending_depth, (unsigned long long)got, (unsigned long long)want, (uint32_t)chk[1]);
+    return PD_OK;
+  };
+  bool timed_reassign = false;
+  auto after_sync = [&]() -> int {
+    if (timed_reassign) stats.ms_reassign += elapsed(ev[4], ev[5]);
+    timed_reassign = false;
+    return check_regroup();
+  };
 
   for (uint32_t depth = 1; depth < end_depth; depth++) {
-    if (depth == 1) {
-      for (uint32_t l = 0; l < K; l++) class_tot[l] = ctx->root_class_tot[l];
-    }
     ctx->nm_level = (int32_t)depth - 1;  // the node map's level: the frontier's
     const uint32_t nf = (uint32_t)frontier.size();
     if (nf == 0) break;
-    for (uint32_t i = 0; i < nf; i++) stats.evals += (uint64_t)node_tot[frontier[i]] * F;
+    stats.evals += cur_off.back() * F;
     stats.nodes_trained += nf;
     const uint32_t cap = std::min(nf, max_slots);
     PD_TRY(ensure_slice(ctx, p, cap));
-    PD_TRY(d_nodes.ensure((size_t)cap * 4));
-    PD_TRY(d_ctot.ensure((size_t)cap * K * 4));
-    PD_TRY(d_split_list.ensure((size_t)cap * 4));
-    std::vector<uint8_t> split_now(nf, 0);
+    split_now.assign(nf, 0);
+    left_cnt.assign((size_t)nf * K, 0u);
+    level_par.assign((size_t)nf * (D + 1), (FeatT)0);
 
     for (uint32_t s0 = 0; s0 < nf; s0 += cap) {
       const uint32_t ns = std::min(cap, nf - s0);
-      std::vector<uint32_t> ctot((size_t)ns * K);
-      for (uint32_t i = 0; i < ns; i++)
-        memcpy(&ctot[(size_t)i * K], &class_tot[(size_t)frontier[s0 + i] * K], K * 4);
-      PD_CUDA(h2d(ctx, d_nodes.ptr, &frontier[s0], (size_t)ns * 4));
-      PD_CUDA(h2d(ctx, d_ctot.ptr, ctot.data(), (size_t)ns * K * 4));
-      PD_CUDA(cudaMemsetAsync(ctx->recheck.ptr, 0, sizeof(unsigned long long), st));
+      // nodes and class totals of the slice, in one copy
+      const size_t node_bytes = ((size_t)ns * 4 + 15) / 16 * 16;
+      PD_TRY(ctx->h_pre.ensure(node_bytes + (size_t)ns * K * 4));
+      PD_TRY(ctx->d_pre.ensure(node_bytes + (size_t)ns * K * 4));
+      const uint32_t *ctot = &tot[(size_t)s0 * K];
+      memcpy(ctx->h_pre.ptr, &frontier[s0], (size_t)ns * 4);
+      memcpy(ctx->h_pre.as<uint8_t>() + node_bytes, ctot, (size_t)ns * K * 4);
+      PD_CUDA(h2d(ctx, ctx->d_pre.ptr, ctx->h_pre.ptr, node_bytes + (size_t)ns * K * 4));
+      const int32_t *d_nodes = ctx->d_pre.as<int32_t>();
+      const uint32_t *d_ctot = reinterpret_cast<const uint32_t *>(ctx->d_pre.as<uint8_t>() + node_bytes);
+      PD_TRY(set_results(ctx, ns));
+      PD_CUDA(cudaMemsetAsync(ctx->res_recheck, 0, sizeof(unsigned long long), st));
       std::vector<uint64_t> off(cur_off.begin() + s0, cur_off.begin() + s0 + ns + 1);
       PD_CUDA(cudaEventRecord(ev[0], st));
       const uint32_t *d_ord = nullptr;
       PropSrc src;
       if (prop) {
         // the network's mixture for every node of the slice, then the table drawn from it
-        PD_TRY(proposer_infer(prop, d_ctot.as<uint32_t>(), ns, depth, n_prop, &src));
-        PD_TRY(launch_candidates<P>(ctx, p, tree_id, d_nodes.as<int32_t>(), ns, ctx->cand_order, &d_ord, &src));
+        PD_TRY(proposer_infer(prop, d_ctot, ns, depth, n_prop, &src));
+        PD_TRY(launch_candidates<P>(ctx, p, tree_id, d_nodes, ns, ctx->cand_order, &d_ord, &src));
       } else {
-        PD_TRY(launch_candidates<P>(ctx, p, tree_id, d_nodes.as<int32_t>(), ns, ctx->cand_order, &d_ord, nullptr,
+        PD_TRY(launch_candidates<P>(ctx, p, tree_id, d_nodes, ns, ctx->cand_order, &d_ord, nullptr,
                                     shard ? shard->f_base : 0u));
       }
       PD_CUDA(cudaEventRecord(ev[1], st));
       uint64_t n_items = 0;
       std::vector<uint32_t> split_slots;
+      const uint32_t *d_split_list = nullptr;
       PD_TRY(launch_hist<P>(ctx, p, off.data(), ns, ctx->act_rec[cur].as<SampleRec>(), &n_items, ev[6], ev[2],
-                            &split_slots, d_ctot.as<uint32_t>(), ctot.data(), d_ord, prop ? &src : nullptr));
+                            &split_slots, d_ctot, ctot, d_ord, prop ? &src : nullptr, &d_split_list));
       stats.hist_launches++;
       stats.hist_bytes += hist_algorithmic_bytes(ctx, p, off.back() - off.front(), ns, (uint32_t)split_slots.size(),
                                                  image_bytes);
-      if (!split_slots.empty())
-        PD_CUDA(h2d(ctx, d_split_list.ptr, split_slots.data(), split_slots.size() * 4));
       PD_TRY(launch_split<false>(ctx, p, (uint32_t)split_slots.size(), ctx->hist.as<uint32_t>(),
-                                 ctx->cand_perm.as<uint8_t>(), d_ctot.as<uint32_t>(), d_split_list.as<uint32_t>(),
-                                 ns, d_ord));
+                                 ctx->cand_perm.as<uint8_t>(), d_ctot, d_split_list, ns, d_ord));
       // the winners' feature values and thresholds, from the candidate tables
       k_split_params<FeatT><<<(ns + 127) / 128, 128, 0, st>>>(
-          ctx->split_out.as<SplitOut>(), ns, ctx->cand_feat.as<FeatT>(), ctx->cand_thr.as<FeatT>(),
-          ctx->cand_perm.as<uint8_t>(), p->n_features, p->n_thresholds, D, ctx->split_par.as<FeatT>());
+          static_cast<SplitOut *>(ctx->res_out), ns, ctx->cand_feat.as<FeatT>(), ctx->cand_thr.as<FeatT>(),
+          ctx->cand_perm.as<uint8_t>(), p->n_features, p->n_thresholds, D, static_cast<FeatT *>(ctx->res_par));
       PD_CUDA(cudaGetLastError());
       ctx->launches++;
       PD_CUDA(cudaEventRecord(ev[3], st));
-      h_out.resize(ns);
-      h_cl.resize((size_t)ns * K);
-      h_par.resize((size_t)ns * (D + 1));
-      unsigned long long rechecked = 0;
-      PD_CUDA(d2h(ctx, h_out.data(), ctx->split_out.ptr, ns * sizeof(SplitOut)));
-      PD_CUDA(d2h(ctx, h_cl.data(), ctx->split_cl.ptr, (size_t)ns * K * 4));
-      PD_CUDA(d2h(ctx, h_par.data(), ctx->split_par.ptr, (size_t)ns * (D + 1) * sizeof(FeatT)));
-      PD_CUDA(d2h(ctx, &rechecked, ctx->recheck.ptr, 8));
+      PD_TRY(ctx->h_res.ensure(ctx->res_bytes));
+      PD_CUDA(d2h(ctx, ctx->h_res.ptr, ctx->res_out, ctx->res_bytes));
       PD_CUDA(cudaStreamSynchronize(st));
+      PD_TRY(after_sync());
+      auto host = [&](const void *d) {  // where a result lies in the copy
+        return ctx->h_res.as<uint8_t>() + (static_cast<const uint8_t *>(d) - static_cast<const uint8_t *>(ctx->res_out));
+      };
+      h_out.assign(reinterpret_cast<const SplitOut *>(host(ctx->res_out)),
+                   reinterpret_cast<const SplitOut *>(host(ctx->res_out)) + ns);
+      uint32_t *h_cl = &left_cnt[(size_t)s0 * K];
+      FeatT *h_par = &level_par[(size_t)s0 * (D + 1)];
+      memcpy(h_cl, host(ctx->res_cl), (size_t)ns * K * 4);
+      memcpy(h_par, host(ctx->res_par), (size_t)ns * (D + 1) * sizeof(FeatT));
+      unsigned long long rechecked = 0;
+      memcpy(&rechecked, host(ctx->res_recheck), 8);
       stats.ms_candidates += elapsed(ev[0], ev[1]);
       stats.ms_hist += elapsed(ev[6], ev[2]);
       stats.ms_split += elapsed(ev[2], ev[3]);
@@ -726,7 +781,7 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
           idx[i] = o.t < 0 ? -1 : (int64_t)o.t * shard->F_total + (int64_t)(shard->f_base + (uint32_t)o.f);
           if (o.t < 0) memset(&h_cl[(size_t)i * K], 0, K * 4);
         }
-        PD_CHECK(shard->exchange(shard->user, ns, K, key.data(), idx.data(), h_cl.data()) == 0, PD_ERR_STATE,
+        PD_CHECK(shard->exchange(shard->user, ns, K, key.data(), idx.data(), h_cl) == 0, PD_ERR_STATE,
                  "the exchange of the ranks' best splits failed at depth %u", depth);
         for (uint32_t i = 0; i < ns; i++) {
           SplitOut &o = h_out[i];
@@ -754,20 +809,16 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
         const SplitOut &o = h_out[i];
         if (o.t < 0) continue;
         const uint32_t n = (uint32_t)frontier[s0 + i];
+        const uint32_t *cl = h_cl + (size_t)i * K, *nt = ctot + (size_t)i * K;
         uint32_t lsum = 0, rsum = 0;
         for (uint32_t l = 0; l < K; l++) {
-          cl[l] = h_cl[(size_t)i * K + l];
-          cr[l] = class_tot[(size_t)n * K + l] - cl[l];
+          cr[l] = nt[l] - cl[l];
           lsum += cl[l];
           rsum += cr[l];
         }
         if (!lsum || !rsum) continue;
         const uint64_t L = 2ull * n + 1, R = 2ull * n + 2;
-        node_tot[L] = lsum;
-        node_tot[R] = rsum;
         for (uint32_t l = 0; l < K; l++) {
-          class_tot[L * K + l] = cl[l];
-          class_tot[R * K + l] = cr[l];
           posts[L * K + l] = (float)cl[l] / (float)lsum;
           posts[R * K + l] = (float)cr[l] / (float)rsum;
         }
@@ -783,57 +834,76 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
           pd_record r;
           memset(&r, 0, sizeof(r));
           r.depth = depth;
-          r.count = node_tot[n];
+          r.count = lsum + rsum;
           r.node = n;
           r.tree = tree_id;
           r.gain = o.gain;
           for (int d = 0; d < D; d++) r.feat[d] = (int32_t)feats[(size_t)n * D + d];
           r.thr = (int32_t)thrs[n];
-          for (uint32_t l = 0; l < K; l++) r.class_count[l] = class_tot[(size_t)n * K + l];
+          for (uint32_t l = 0; l < K; l++) r.class_count[l] = nt[l];
           ctx->records.push_back(r);
         }
       }
     }
 
-    // device tree update for the frontier nodes and their children
-    const uint64_t nmin = (uint64_t)frontier.front(), nmax = (uint64_t)frontier.back();
-    const uint64_t cmax = std::min<uint64_t>(n_nodes - 1, 2 * nmax + 2);
-    PD_CUDA(h2d(ctx, ctx->t_lc.as<int32_t>() + nmin, lc + nmin, (cmax - nmin + 1) * 4));
-    PD_CUDA(h2d(ctx, ctx->t_feat.as<FeatT>() + nmin * D, feats + nmin * D, (nmax - nmin + 1) * D * sizeof(FeatT)));
-    PD_CUDA(h2d(ctx, ctx->t_thr.as<FeatT>() + nmin, thrs + nmin, (nmax - nmin + 1) * sizeof(FeatT)));
-    if (2 * nmin + 1 < n_nodes)
-      PD_CUDA(h2d(ctx, ctx->t_post.as<float>() + (2 * nmin + 1) * K, posts + (2 * nmin + 1) * K,
-                              (cmax - (2 * nmin + 1) + 1) * K * 4));
+    if (ctx->tree_feature) {
+      // device tree update for the frontier nodes and their children
+      const uint64_t nmin = (uint64_t)frontier.front(), nmax = (uint64_t)frontier.back();
+      const uint64_t cmax = std::min<uint64_t>(n_nodes - 1, 2 * nmax + 2);
+      PD_CUDA(h2d(ctx, ctx->t_lc.as<int32_t>() + nmin, lc + nmin, (cmax - nmin + 1) * 4));
+      PD_CUDA(h2d(ctx, ctx->t_feat.as<FeatT>() + nmin * D, feats + nmin * D, (nmax - nmin + 1) * D * sizeof(FeatT)));
+      PD_CUDA(h2d(ctx, ctx->t_thr.as<FeatT>() + nmin, thrs + nmin, (nmax - nmin + 1) * sizeof(FeatT)));
+      if (2 * nmin + 1 < n_nodes)
+        PD_CUDA(h2d(ctx, ctx->t_post.as<float>() + (2 * nmin + 1) * K, posts + (2 * nmin + 1) * K,
+                    (cmax - (2 * nmin + 1) + 1) * K * 4));
+    }
 
     // next frontier (init:333-365: leaf children with more than perLeafSamplesThr samples)
-    std::vector<int32_t> next;
-    std::vector<uint64_t> next_off{0};
-    std::vector<SlotNext> sn(nf);
+    next.clear();
+    next_tot.clear();
+    next_off.assign(1, 0);
+    const size_t sn_bytes = (size_t)nf * sizeof(SlotNext), par_bytes = (size_t)nf * (D + 1) * sizeof(FeatT);
+    PD_TRY(ctx->h_splits.ensure(sn_bytes + par_bytes));
+    PD_TRY(ctx->d_splits.ensure(sn_bytes + par_bytes));
+    SlotNext *sn = ctx->h_splits.as<SlotNext>();
     long long base_l = 0, base_r = 0;
     const bool more = depth + 1 < end_depth;
     for (uint32_t i = 0; i < nf; i++) {
-      sn[i].k_l = sn[i].k_r = -1;
-      sn[i].adj_l = sn[i].adj_r = 0;
-      if (!split_now[i]) continue;
-      const uint64_t n = (uint64_t)frontier[i];
-      const uint64_t L = 2 * n + 1, R = 2 * n + 2;
-      if (more && node_tot[L] > p->per_leaf_samples_thr) {
-        sn[i].k_l = (int32_t)next.size();
-        sn[i].adj_l = (long long)next_off.back() - base_l;
-        base_l += node_tot[L];
-        next.push_back((int32_t)L);
-        next_off.push_back(next_off.back() + node_tot[L]);
+      SlotNext x;
+      x.k_l = x.k_r = x.child = -1;
+      x.pad = 0;
+      x.adj_l = x.adj_r = 0;
+      if (split_now[i]) {
+        const uint64_t n = (uint64_t)frontier[i], L = 2 * n + 1, R = 2 * n + 2;
+        const uint32_t *cl = &left_cnt[(size_t)i * K], *nt = &tot[(size_t)i * K];
+        uint64_t lsum = 0;
+        for (uint32_t l = 0; l < K; l++) lsum += cl[l];
+        const uint64_t rsum = cur_off[i + 1] - cur_off[i] - lsum;
+        x.child = (int32_t)L;
+        if (more && lsum > p->per_leaf_samples_thr) {
+          x.k_l = (int32_t)next.size();
+          x.adj_l = (long long)next_off.back() - base_l;
+          base_l += (long long)lsum;
+          next.push_back((int32_t)L);
+          next_off.push_back(next_off.back() + lsum);
+          next_tot.insert(next_tot.end(), cl, cl + K);
+        }
+        if (more && rsum > p->per_leaf_samples_thr) {
+          x.k_r = (int32_t)next.size();
+          x.adj_r = (long long)next_off.back() - base_r;
+          base_r += (long long)rsum;
+          next.push_back((int32_t)R);
+          next_off.push_back(next_off.back() + rsum);
+          for (uint32_t l = 0; l < K; l++) next_tot.push_back(nt[l] - cl[l]);
+        }
       }
-      if (more && node_tot[R] > p->per_leaf_samples_thr) {
-        sn[i].k_r = (int32_t)next.size();
-        sn[i].adj_r = (long long)next_off.back() - base_r;
-        base_r += node_tot[R];
-        next.push_back((int32_t)R);
-        next_off.push_back(next_off.back() + node_tot[R]);
-      }
+      sn[i] = x;
     }
-    PD_TRY(d_next.ensure((size_t)nf * sizeof(SlotNext)));
-    PD_CUDA(h2d(ctx, d_next.ptr, sn.data(), (size_t)nf * sizeof(SlotNext)));
+    // the level's splits by slot, in one copy
+    memcpy(ctx->h_splits.as<uint8_t>() + sn_bytes, level_par.data(), par_bytes);
+    PD_CUDA(h2d(ctx, ctx->d_splits.ptr, ctx->h_splits.ptr, sn_bytes + par_bytes));
+    const SlotNext *d_next = ctx->d_splits.as<SlotNext>();
+    const FeatT *d_par = reinterpret_cast<const FeatT *>(ctx->d_splits.as<uint8_t>() + sn_bytes);
     PD_CUDA(cudaEventRecord(ev[4], st));
     if (n_act && is_user_plugin(ctx)) {
       const RtcKernels *rk = nullptr;
@@ -843,19 +913,15 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
       const SampleRec *r_ = ctx->act_rec[cur].as<SampleRec>();
       uint32_t na = (uint32_t)n_act;
       int32_t *sn_ = ctx->snode.as<int32_t>();
-      const int32_t *lc_ = ctx->t_lc.as<int32_t>();
-      const FeatT *tf = ctx->t_feat.as<FeatT>(), *tt = ctx->t_thr.as<FeatT>();
-      const SlotNext *nx = d_next.as<SlotNext>();
       uint8_t *fl = ctx->flags.as<uint8_t>();
-      void *args[] = {&ds, &a_, &r_, &as_, &na, &sn_, &lc_, &tf, &tt, &nx, &fl};
+      void *args[] = {&ds, &a_, &r_, &as_, &na, &sn_, &d_par, &d_next, &fl};
       PD_TRY(rtc_launch(ctx, rk->reassign, dim3((unsigned)((n_act + 255) / 256)), dim3(256), 0, args));
     } else if constexpr (!P::kRtcOnly) {
       if (n_act) {
         k_reassign<P><<<(unsigned)((n_act + 255) / 256), 256, 0, st>>>(
             devset(ctx), ctx->act[cur].as<uint32_t>(), ctx->act_rec[cur].as<SampleRec>(),
-            ctx->act_slot[cur].as<uint32_t>(), (uint32_t)n_act,
-            ctx->snode.as<int32_t>(), ctx->t_lc.as<int32_t>(), ctx->t_feat.as<FeatT>(), ctx->t_thr.as<FeatT>(),
-            d_next.as<SlotNext>(), ctx->flags.as<uint8_t>());
+            ctx->act_slot[cur].as<uint32_t>(), (uint32_t)n_act, ctx->snode.as<int32_t>(), d_par, d_next,
+            ctx->flags.as<uint8_t>());
         PD_CUDA(cudaGetLastError());
         ctx->launches++;
       }
@@ -870,37 +936,29 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
     if (!next.empty() && n_act) {
       const uint32_t nb = (uint32_t)((n_act + kScanItems - 1) / kScanItems);
       unsigned long long *bs = ctx->scan_blocks.as<unsigned long long>();
-      PD_CUDA(cudaMemsetAsync(ctx->scatter_err.ptr, 0, 4, st));
       k_scan_reduce<<<nb, 256, 0, st>>>(ctx->flags.as<uint8_t>(), (uint32_t)n_act, bs);
       k_scan_blocks<<<1, 1024, 0, st>>>(bs, nb, bs + nb);
       k_scatter<<<nb, 256, 0, st>>>(ctx->flags.as<uint8_t>(), (uint32_t)n_act, bs, ctx->act[cur].as<uint32_t>(),
-                                    ctx->act_slot[cur].as<uint32_t>(), d_next.as<SlotNext>(), (uint32_t)n_next,
+                                    ctx->act_slot[cur].as<uint32_t>(), d_next, (uint32_t)n_next,
                                     ctx->act[1 - cur].as<uint32_t>(), ctx->act_slot[1 - cur].as<uint32_t>(),
                                     ctx->act_rec[cur].as<SampleRec>(), ctx->act_rec[1 - cur].as<SampleRec>(),
-                                    ctx->scatter_err.as<uint32_t>());
+                                    bs + nb + 1);
       PD_CUDA(cudaGetLastError());
       ctx->launches += 3;
-      unsigned long long total = 0;
-      uint32_t err = 0;
-      PD_CUDA(d2h(ctx, &total, bs + nb, 8));
-      PD_CUDA(d2h(ctx, &err, ctx->scatter_err.ptr, 4));
-      PD_CUDA(cudaEventRecord(ev[5], st));
-      PD_CUDA(cudaStreamSynchronize(st));
-      const uint64_t got = (total & 0xffffffffull) + (total >> 32);
-      PD_CHECK(err == 0 && got == n_next, PD_ERR_STATE,
-               "reassignment disagrees with the split counts at depth %u (%llu vs %llu samples, %u misplaced)",
-               depth, (unsigned long long)got, (unsigned long long)n_next, err);
+      PD_CUDA(d2h(ctx, ctx->h_chk.ptr, bs + nb, 16));  // checked after the next synchronisation
+      pending = n_next;
+      pending_depth = depth;
       cur = 1 - cur;
-    } else {
-      PD_CUDA(cudaEventRecord(ev[5], st));
-      PD_CUDA(cudaStreamSynchronize(st));
     }
-    stats.ms_reassign += elapsed(ev[4], ev[5]);
+    PD_CUDA(cudaEventRecord(ev[5], st));
+    timed_reassign = true;
     n_act = n_next;
     frontier.swap(next);
     cur_off.swap(next_off);
+    tot.swap(next_tot);
   }
   PD_CUDA(cudaStreamSynchronize(st));
+  PD_TRY(after_sync());
   stats.ms_total = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
   stats.h2d_bytes = ctx->bytes_h2d - h2d0;
   stats.d2h_bytes = ctx->bytes_d2h - d2h0;
@@ -1108,10 +1166,10 @@ extern "C" int pd_split(pd_ctx *ctx, const pd_train_params *params, const uint32
   PD_TRY(dc.ensure((size_t)n_nodes * K * 4 + 4));
   PD_CUDA(h2d(ctx, dh.ptr, hist, (size_t)n_nodes * K * T * F * 4));
   PD_CUDA(h2d(ctx, dc.ptr, class_tot, (size_t)n_nodes * K * 4));
-  PD_CUDA(cudaMemsetAsync(ctx->recheck.ptr, 0, 8, ctx->stream));
+  PD_CUDA(cudaMemsetAsync(ctx->res_recheck, 0, 8, ctx->stream));
   PD_TRY(launch_split<true>(ctx, params, n_nodes, dh.as<uint32_t>(), nullptr, dc.as<uint32_t>()));
   std::vector<SplitOut> o(n_nodes);
-  PD_CUDA(d2h(ctx, o.data(), ctx->split_out.ptr, n_nodes * sizeof(SplitOut)));
+  PD_CUDA(d2h(ctx, o.data(), ctx->res_out, n_nodes * sizeof(SplitOut)));
   PD_CUDA(cudaStreamSynchronize(ctx->stream));
   for (uint32_t i = 0; i < n_nodes; i++) {
     out_t[i] = o[i].t;

@@ -1969,25 +1969,25 @@ __global__ void __launch_bounds__(kSplitCols) k_split_pick(SplitArgs a) {
 struct SlotNext {
   long long adj_l, adj_r;  // next position base (next offset of child - samples of earlier parents)
   int32_t k_l, k_r;        // next frontier slot of each child or -1
+  int32_t child, pad;      // left child of the slot's node, -1 when it was not split
 };
 
+// par: feature values and threshold of each slot's split [slot][D + 1].  Everything is
+// read by slot, so the trainer uploads a level's frontier, not ranges of the tree.
 template <class P>
 __global__ void k_reassign(DevSet ds, const uint32_t *__restrict__ act, const SampleRec *__restrict__ rec,
-                           const uint32_t *__restrict__ act_slot,
-                           uint32_t n_act, int32_t *__restrict__ snode, const int32_t *__restrict__ lc,
-                           const typename P::feat_t *__restrict__ feat,
-                           const typename P::feat_t *__restrict__ thr, const SlotNext *__restrict__ nxt,
+                           const uint32_t *__restrict__ act_slot, uint32_t n_act, int32_t *__restrict__ snode,
+                           const typename P::feat_t *__restrict__ par, const SlotNext *__restrict__ nxt,
                            uint8_t *__restrict__ flags) {
   using FeatT = typename P::feat_t;
   using ImgT = typename P::img_t;
   constexpr int D = P::kFeatDim;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_act) return;
-  const uint32_t s = act[i];
-  const int32_t n = snode[s];
-  const int32_t c = lc[n];
+  const uint32_t slot = act_slot[i];
+  const SlotNext sn = nxt[slot];
   uint8_t flag = 0;
-  if (c >= 0) {
+  if (sn.child >= 0) {
     const SampleRec r = rec[i];
     const uint32_t xy = r.xy, im_i = r.img_lab & 0xffffffu;
     const uint32_t wh = ds.img_wh[im_i];
@@ -1999,12 +1999,11 @@ __global__ void k_reassign(DevSet ds, const uint32_t *__restrict__ act, const Sa
     if constexpr (P::kUsesTree) attach_tree<P>(im, ds, ds.map_off ? ds.map_off[im_i] : 0ull);
     FeatT fv[D];
 #pragma unroll
-    for (int d = 0; d < D; d++) fv[d] = feat[(size_t)n * D + d];
+    for (int d = 0; d < D; d++) fv[d] = par[(size_t)slot * (D + 1) + d];
     const auto prep = P::prepare(im, (int32_t)(xy & 0xffffu), (int32_t)(xy >> 16), r.pre);
     const FeatT resp = P::eval(prep, fv);
-    const bool right = resp > thr[n];
-    snode[s] = c + (right ? 1 : 0);
-    const SlotNext sn = nxt[act_slot[i]];
+    const bool right = resp > par[(size_t)slot * (D + 1) + D];
+    snode[act[i]] = sn.child + (right ? 1 : 0);
     if (right) flag = sn.k_r >= 0 ? 2 : 0;
     else flag = sn.k_l >= 0 ? 1 : 0;
   }
@@ -2034,6 +2033,7 @@ static __global__ void __launch_bounds__(256) k_scan_reduce(const uint8_t *__res
 // Exclusive scan of the block sums in one CTA (any count).
 static __global__ void __launch_bounds__(1024) k_scan_blocks(unsigned long long *__restrict__ bsum, uint32_t nb,
                                                       unsigned long long *__restrict__ total) {
+  if (threadIdx.x == 0) total[1] = 0ull;  // k_scatter's misplaced samples
   const uint32_t per = (nb + blockDim.x - 1) / blockDim.x;
   const uint32_t b = threadIdx.x * per, e = min(nb, b + per);
   unsigned long long s = 0;
@@ -2069,7 +2069,7 @@ static __global__ void __launch_bounds__(256) k_scatter(const uint8_t *__restric
                                                  uint32_t *__restrict__ slot_out,
                                                  const SampleRec *__restrict__ rec,
                                                  SampleRec *__restrict__ rec_out,
-                                                 uint32_t *__restrict__ err) {
+                                                 unsigned long long *__restrict__ err) {
   constexpr int PER = kScanItems / 256;
   const uint32_t b0 = blockIdx.x * kScanItems + threadIdx.x * PER;
   uint8_t fl[PER];
@@ -2108,7 +2108,7 @@ static __global__ void __launch_bounds__(256) k_scatter(const uint8_t *__restric
       run += 1ull << 32;
     }
     if (pos < 0 || pos >= (long long)n_next) {
-      atomicAdd(err, 1u);
+      atomicAdd(err, 1ull);
       continue;
     }
     act_out[pos] = act[i];
