@@ -259,7 +259,7 @@ static int launch_candidates(pd_ctx *ctx, const pd_train_params *p, uint32_t tre
   if (packed && T <= 64 && ctx->cand_regs) {
     // keys sorted in registers
     auto rk = T <= 16 ? k_candidates_reg<FeatT, 16> : (T <= 32 ? k_candidates_reg<FeatT, 32> : k_candidates_reg<FeatT, 64>);
-    rk<<<grid, kCandThreads, 0, ctx->stream>>>(d_nodes, n, tree, F, T, P::kFeatDim, b, ord, ctx->cand_feat.as<FeatT>(),
+    rk<<<grid, kCandThreads, (size_t)T * kCandThreads * 4, ctx->stream>>>(d_nodes, n, tree, F, T, P::kFeatDim, b, ord, ctx->cand_feat.as<FeatT>(),
                                                ctx->cand_thr.as<FeatT>(), ctx->cand_perm.as<uint8_t>(),
                                                prop ? *prop : PropSrc{});
     PD_CUDA(cudaGetLastError());
