@@ -1835,11 +1835,68 @@ __global__ void __launch_bounds__(kSplitCols) k_split_g32(SplitArgs a) {
   }
 }
 
+// Exact gain of sorted position j of column f, by a whole warp (every lane returns
+// it): the lanes share the row sums and the classes' terms; the terms are added one
+// after the other in class order, as sum64 adds them (a term it skips is 0 here, and
+// the sums are never -0).
+template <int KM, bool CUM>
+PD_D double warp_gain(const SplitArgs &a, const uint32_t *H, const uint32_t *tot, uint32_t N, double hp64, uint32_t j,
+                      uint32_t f) {
+  const uint32_t lane = threadIdx.x & 31, K = a.K, T = a.T, F = a.F;
+  constexpr int R = (KM + 31) / 32;
+  uint32_t mine[R];  // class lane + 32 r
+#pragma unroll
+  for (int r = 0; r < R; r++) mine[r] = 0u;
+  if constexpr (CUM) {
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if (lane + 32u * r < K) mine[r] = H[((size_t)(lane + 32u * r) * T + j) * F + f];
+  } else {
+#pragma unroll
+    for (int l = 0; l < KM; l++) {
+      uint32_t v = 0;
+      if ((uint32_t)l < K)
+        for (uint32_t q = lane; q <= j; q += 32) v += H[((size_t)l * T + q) * F + f];
+      v = __reduce_add_sync(0xffffffffu, v);
+      if (lane == (uint32_t)(l & 31)) mine[l >> 5] = v;
+    }
+  }
+  uint32_t nL = 0;
+#pragma unroll
+  for (int r = 0; r < R; r++) nL += mine[r];
+  nL = __reduce_add_sync(0xffffffffu, nL);
+  const uint32_t nR = N - nL;
+  const double Ll = a.L[nL], Lr = a.L[nR];
+  double tl[R], tr[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const uint32_t l = lane + 32u * r, cl = mine[r], cr = l < K ? tot[l] - cl : 0u;
+    tl[r] = cl != 0u && (uint64_t)cl * 1000000ull > nL ? dmul((double)cl, dsub(Ll, a.L[cl])) : 0.0;
+    tr[r] = cr != 0u && (uint64_t)cr * 1000000ull > nR ? dmul((double)cr, dsub(Lr, a.L[cr])) : 0.0;
+  }
+  double sl = 0.0, sr = 0.0;
+#pragma unroll
+  for (int l = 0; l < KM; l++) {
+    if ((uint32_t)l < K) {
+      sl = dadd(sl, __shfl_sync(0xffffffffu, tl[l >> 5], l & 31));
+      sr = dadd(sr, __shfl_sync(0xffffffffu, tr[l >> 5], l & 31));
+    }
+  }
+  return dsub(hp64, ddiv(dadd(sl, sr), (double)N));
+}
+
 // Pass 2: candidates within delta of the node's FP32 maximum are re-evaluated
 // with the exact FP64 gain S(tot,N)/N - (S(L)+S(R))/N; the largest exact gain
 // wins, ties to the lowest t*F+f (the first-max rule of
 // learn_best_feature.cl:96-101 + std::max_element).  The last part of a node to
 // finish reduces the parts and writes the winner with its left class counts.
+//
+// The candidates cluster in few columns, so they are listed and dealt out over the
+// warps (warp_gain); a thread per column, walking its rows, re-evaluated them one
+// after the other, each waiting for its rows and logarithms.  Lists that overflow
+// (nodes that nothing separates: thousands of equal gains, few different counts) go
+// that way.
+constexpr uint32_t kPickList = 256;
 template <int KM, bool CUM>
 __global__ void __launch_bounds__(kSplitCols) k_split_pick(SplitArgs a) {
   const uint32_t slot = a.slot_list ? a.slot_list[blockIdx.y] : blockIdx.y, part = blockIdx.x;
@@ -1850,6 +1907,9 @@ __global__ void __launch_bounds__(kSplitCols) k_split_pick(SplitArgs a) {
   __shared__ int red_j[kSplitCols / 32];
   __shared__ int red_c[kSplitCols / 32];
   __shared__ bool last;
+  __shared__ uint32_t s_n, s_col[kPickList];
+  __shared__ uint16_t s_row[kPickList];
+  if (threadIdx.x == 0) s_n = 0u;
   uint32_t N;
   load_tot<KM>(a, slot, tot, N);
   if (N == 0 || (uint64_t)N >= a.L_len) {
@@ -1862,43 +1922,77 @@ __global__ void __launch_bounds__(kSplitCols) k_split_pick(SplitArgs a) {
     return;
   }
   const float cut = ord2f(a.node_max[slot]) - a.delta;
-  const double hp64 = ddiv(sum64<KM, false>(tot, tot, K, N, a.L), (double)N);
   const uint32_t *H = a.hist + (size_t)slot * K * T * F;
   const float *G = a.g32 + (size_t)slot * T * F;
   const uint32_t fb = part * a.cols, fe = min(F, fb + a.cols);
+  for (uint32_t f = fb + threadIdx.x; f < fe; f += blockDim.x) {
+#pragma unroll 10
+    for (uint32_t j = 0; j < T; j++)
+      if (G[(size_t)j * F + f] >= cut) {
+        const uint32_t i = atomicAdd(&s_n, 1u);
+        if (i < kPickList) {
+          s_col[i] = f;
+          s_row[i] = (uint16_t)j;
+        }
+      }
+  }
+  __syncthreads();
+  const uint32_t n_list = s_n;
   double best = -DBL_MAX;
   long long best_idx = LLONG_MAX;
   int best_j = -1, best_c = -1;
   unsigned long long n_checked = 0;
-  for (uint32_t f = fb + threadIdx.x; f < fe; f += blockDim.x) {
-    int jmax = -1;
-    for (uint32_t j = 0; j < T; j++)
-      if (G[(size_t)j * F + f] >= cut) jmax = (int)j;
-    if (jmax < 0) continue;
-    uint32_t c[KM];
-#pragma unroll
-    for (int l = 0; l < KM; l++) c[l] = 0u;
-    bool dirty = true;
-    double g = 0.0;
-    for (int j = 0; j <= jmax; j++) {
-      uint32_t nL;
-      dirty |= step_counts<KM, CUM>(H, K, T, F, (uint32_t)j, f, c, nL);
-      if (!(G[(size_t)j * F + f] >= cut)) continue;
-      if (dirty) {
-        n_checked++;
-        const uint32_t nR = N - nL;
-        const double sl = sum64<KM, false>(tot, c, K, nL, a.L);
-        const double sr = sum64<KM, true>(tot, c, K, nR, a.L);
-        g = dsub(hp64, ddiv(dadd(sl, sr), (double)N));
-        dirty = false;
-      }
-      const uint32_t t = a.perm ? a.perm[((size_t)slot * T + j) * F + f] : (uint32_t)j;
+  if (n_list == 0) {
+    // nothing of this part is near the maximum
+  } else if (n_list <= kPickList) {
+    const double hp64 = ddiv(sum64<KM, false>(tot, tot, K, N, a.L), (double)N);
+    for (uint32_t i = threadIdx.x >> 5; i < n_list; i += kSplitCols / 32) {
+      const uint32_t j = s_row[i], f = s_col[i];
+      const uint32_t t = a.perm ? a.perm[((size_t)slot * T + j) * F + f] : j;
       const long long idx = (long long)t * F + (a.ord ? a.ord[(size_t)slot * F + f] : f);
+      const double g = warp_gain<KM, CUM>(a, H, tot, N, hp64, j, f);
+      if ((threadIdx.x & 31) != 0) continue;
+      n_checked++;
       if (g > best || (g == best && idx < best_idx)) {
         best = g;
         best_idx = idx;
-        best_j = j;
+        best_j = (int)j;
         best_c = (int)f;
+      }
+    }
+  } else {
+    const double hp64 = ddiv(sum64<KM, false>(tot, tot, K, N, a.L), (double)N);
+    for (uint32_t f = fb + threadIdx.x; f < fe; f += blockDim.x) {
+      int jmax = -1;
+#pragma unroll 8
+      for (uint32_t j = 0; j < T; j++)
+        if (G[(size_t)j * F + f] >= cut) jmax = (int)j;
+      if (jmax < 0) continue;
+      uint32_t c[KM];
+#pragma unroll
+      for (int l = 0; l < KM; l++) c[l] = 0u;
+      bool dirty = true;
+      double g = 0.0;
+      for (int j = 0; j <= jmax; j++) {
+        uint32_t nL;
+        dirty |= step_counts<KM, CUM>(H, K, T, F, (uint32_t)j, f, c, nL);
+        if (!(G[(size_t)j * F + f] >= cut)) continue;
+        if (dirty) {
+          n_checked++;
+          const uint32_t nR = N - nL;
+          const double sl = sum64<KM, false>(tot, c, K, nL, a.L);
+          const double sr = sum64<KM, true>(tot, c, K, nR, a.L);
+          g = dsub(hp64, ddiv(dadd(sl, sr), (double)N));
+          dirty = false;
+        }
+        const uint32_t t = a.perm ? a.perm[((size_t)slot * T + j) * F + f] : (uint32_t)j;
+        const long long idx = (long long)t * F + (a.ord ? a.ord[(size_t)slot * F + f] : f);
+        if (g > best || (g == best && idx < best_idx)) {
+          best = g;
+          best_idx = idx;
+          best_j = j;
+          best_c = (int)f;
+        }
       }
     }
   }
@@ -1946,35 +2040,63 @@ __global__ void __launch_bounds__(kSplitCols) k_split_pick(SplitArgs a) {
     last = atomicAdd(a.done + slot, 1u) == a.parts - 1;
   }
   __syncthreads();
-  if (!last || threadIdx.x != 0) return;
+  if (!last) return;
   __threadfence();
-  SplitPart b = a.part_best[(size_t)slot * a.parts];
-  for (uint32_t i = 1; i < a.parts; i++) {
-    const SplitPart q = a.part_best[(size_t)slot * a.parts + i];
-    if (q.gain > b.gain || (q.gain == b.gain && q.idx < b.idx)) b = q;
-  }
-  SplitOut o;
-  if (b.idx == LLONG_MAX) {
-    o.t = o.f = o.j = o.col = -1;
-    o.gain = 0.0;
-  } else {
-    o.t = (int32_t)(b.idx / F);
-    o.f = (int32_t)(b.idx % F);
-    o.j = b.j;
-    o.col = b.col;
-    o.gain = b.gain;
-    const uint32_t col = (uint32_t)b.col;
-    for (uint32_t l = 0; l < K; l++) {
-      uint32_t c = 0;
-      if (CUM) {
-        c = H[((size_t)l * T + o.j) * F + col];
-      } else {
-        for (int j = 0; j <= o.j; j++) c += H[((size_t)l * T + j) * F + col];
+  // the node's winner over its parts (the first warp), then its left class counts: a
+  // sum over the rows up to it, dealt out over the CTA (one thread alone waited for
+  // K * T loads a few at a time, most of the kernel's time)
+  __shared__ SplitOut s_out;
+  __shared__ uint32_t s_cl[KM];
+  for (uint32_t l = threadIdx.x; l < KM; l += blockDim.x) s_cl[l] = 0u;
+  if (threadIdx.x < 32) {
+    const SplitPart *pb = a.part_best + (size_t)slot * a.parts;
+    double g = -DBL_MAX;
+    long long idx = LLONG_MAX;
+    uint32_t at = 0;
+    for (uint32_t i = threadIdx.x; i < a.parts; i += 32) {
+      const double gi = __ldcg(&pb[i].gain);
+      const long long ii = __ldcg(&pb[i].idx);
+      if (gi > g || (gi == g && ii < idx)) {
+        g = gi;
+        idx = ii;
+        at = i;
       }
-      a.out_cl[(size_t)slot * K + l] = c;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double og = __shfl_xor_sync(0xffffffffu, g, o);
+      const long long oi = __shfl_xor_sync(0xffffffffu, idx, o);
+      const uint32_t oa = __shfl_xor_sync(0xffffffffu, at, o);
+      if (og > g || (og == g && oi < idx)) {
+        g = og;
+        idx = oi;
+        at = oa;
+      }
+    }
+    if (threadIdx.x == 0) {
+      SplitOut o;
+      o.t = o.f = o.j = o.col = -1;
+      o.gain = 0.0;
+      if (idx != LLONG_MAX) {
+        o.t = (int32_t)(idx / F);
+        o.f = (int32_t)(idx % F);
+        o.j = __ldcg(&pb[at].j);
+        o.col = __ldcg(&pb[at].col);
+        o.gain = g;
+      }
+      s_out = o;
+      a.out[slot] = o;
     }
   }
-  a.out[slot] = o;
+  __syncthreads();
+  if (s_out.t < 0) return;
+  const uint32_t col = (uint32_t)s_out.col, rows = CUM ? 1u : (uint32_t)s_out.j + 1u, j0 = CUM ? (uint32_t)s_out.j : 0u;
+  for (uint32_t q = threadIdx.x; q < K * rows; q += blockDim.x) {
+    const uint32_t l = q / rows, j = j0 + q % rows;
+    atomicAdd(&s_cl[l], H[((size_t)l * T + j) * F + col]);
+  }
+  __syncthreads();
+  for (uint32_t l = threadIdx.x; l < K; l += blockDim.x) a.out_cl[(size_t)slot * K + l] = s_cl[l];
 }
 
 // ------------------------------------------------------------ reassign ----
