@@ -38,7 +38,7 @@ static size_t hist_smem(const pd_ctx *ctx, uint32_t T, bool fused = true) {
 // Shared memory of a CTA of the rank-table form with `rows` class rows and
 // `threads` threads: packed tile histogram, `first` bits, table, staged words.
 static size_t rank_smem(uint32_t rows, uint32_t T, uint32_t span, int threads) {
-  return (size_t)rows * (T + 1) * 32 * 4 + (size_t)kTileF * ((T + 31) / 32) * 4 + (size_t)rank_words(span) * 64 * 8 +
+  return (size_t)rows * (T + 1) * 32 * 4 + (size_t)kTileF * ((T + 31) / 32) * 4 + (size_t)rank_words(span) * 64 * 4 +
          (size_t)threads / 32 * 64 * 16;
 }
 constexpr size_t kRankSmemMax = 227 * 1024 - 4096;  // dynamic; the kernels' static arrays take less than 4 KB
@@ -57,7 +57,7 @@ static bool rank_form(const pd_ctx *ctx, const pd_train_params *p, const PropSrc
   }
   const int64_t lo = p->thr_low, hi = p->thr_up, span = hi - lo;
   const int64_t fmax = ctx->cfg.feat_type == PD_FEAT_I16 ? 32767 : (1 << 29);
-  if (span < 0 || lo < -fmax || hi > fmax || span + 1 >= (int64_t)kRankWordsMax * 32) return false;
+  if (span < 0 || lo < -fmax || hi > fmax || span + 1 >= (int64_t)kRankWordsMax * 16) return false;
   return rank_smem((uint32_t)ctx->cfg.n_classes, p->n_thresholds, (uint32_t)span, kRankThreads) <= kRankSmemMax;
 }
 

@@ -36,9 +36,9 @@ constexpr int kRankCtas = 1;
 PD_HD constexpr int small_threads(int NC) { return NC <= 4 ? 128 : NC <= 8 ? 256 : 512; }
 PD_HD constexpr int small_ctas(int NC) { return NC <= 4 ? 4 : NC <= 8 ? 2 : 1; }
 constexpr int kSmallSpi = 4;  // samples per warp iteration (8 measured the same, with more registers)
-constexpr uint32_t kRankWordsMax = 64;  // rank-table words per column: threshold ranges up to 2046
+constexpr uint32_t kRankWordsMax = 128;  // rank-table words per column: threshold ranges up to 2046
 // Table words per column for thresholds in [lo, lo + span] (responses reach span + 1).
-PD_HD constexpr uint32_t rank_words(uint32_t span) { return (span + 1) / 32 + 1; }
+PD_HD constexpr uint32_t rank_words(uint32_t span) { return (span + 1) / 16 + 1; }
 PD_HD constexpr int hist_threads(uint32_t TP) { return TP ? kHistThreads : kRankThreads; }
 constexpr int kScanItems = 4096;   // active samples per scan block (256 threads x 16)
 // FP32 gain window rechecked in FP64.  Each FP32 entropy term -p log2 p (fast
@@ -644,16 +644,18 @@ PD_D void hist_samples(const DevSet &ds, const SampleRec *__restrict__ rec, cons
 
 // ---- rank-table form -------------------------------------------------------
 // For threshold ranges up to 2046 the place of a response among the thresholds is
-// looked up instead of searched (36 instructions per evaluation in place of 69): per candidate, word k of a table holds a bit per
-// value of [lo + 32k, lo + 32k + 32) that is a threshold, and the number of
-// distinct thresholds below lo + 32k (as the byte offset of the histogram row and
-// lane).  The place is that number plus the population count of the bits below
-// the response: one 64-bit shared load and ten instructions, where the search
-// took three register levels, three dependent loads and nineteen.  It counts
-// distinct thresholds; a candidate's duplicates (bit t of `first` clear) share
-// their predecessor's counts and are put back when the rows are read.
+// looked up instead of searched (38 instructions per evaluation in place of 69): per
+// candidate, word k of a table holds a bit per value of [lo + 16k, lo + 16k + 16)
+// that is a threshold (low half), and the number of distinct thresholds below lo +
+// 16k, as the byte offset of the histogram row and lane (high half).  The place is
+// that number plus the population count of the bits below the response: one shared
+// load, where the search took three register levels and three dependent loads.  It
+// counts distinct thresholds; a candidate's duplicates (bit t of `first` clear) share
+// their predecessor's counts and are put back when the rows are read.  (32 values and
+// a whole offset in a 64-bit word: two instructions fewer, one more L1 wavefront of
+// about twenty per evaluation, which bound the loop.)
 struct RankTab {
-  uint2 *tab;             // [2][words][32]: {bits, row and lane offset in bytes}
+  uint32_t *tab;          // [2][words][32]: bits | (row and lane offset in bytes) << 16
   uint32_t words;         // per column
   uint32_t *first;        // [64][first_words]: bit t set when sorted threshold t differs from t - 1
   uint32_t first_words;
@@ -661,42 +663,52 @@ struct RankTab {
 };
 
 // The tables of one tile (all threads; ends with a barrier).  Thread (column c,
-// part) walks consecutive sorted thresholds, then the part's table words.
+// part) walks consecutive sorted thresholds, loaded kThrAhead at a time, then the
+// part's table words.
+constexpr uint32_t kThrAhead = 8;
 template <int NT, typename FeatT>
 PD_D void build_rank_tab(const RankTab &rt, const FeatT *__restrict__ thr, uint32_t F, uint32_t T, uint32_t f0) {
   constexpr uint32_t kParts = NT / kTileF;
   __shared__ uint32_t s_part[kParts][kTileF];
   const uint32_t c = threadIdx.x & (kTileF - 1), part = threadIdx.x / kTileF;
-  for (uint32_t i = threadIdx.x; i < rt.words * 32; i += NT) reinterpret_cast<uint4 *>(rt.tab)[i] = make_uint4(0, 0, 0, 0);
+  for (uint32_t i = threadIdx.x; i < rt.words * 16; i += NT) reinterpret_cast<uint4 *>(rt.tab)[i] = make_uint4(0, 0, 0, 0);
   for (uint32_t i = threadIdx.x; i < kTileF * rt.first_words; i += NT) rt.first[i] = 0u;
   __syncthreads();
-  uint2 *col = rt.tab + (c >> 5) * rt.words * 32 + (c & 31);
+  uint32_t *col = rt.tab + (c >> 5) * rt.words * 32 + (c & 31);
   if (f0 + c < F) {
     const uint32_t per = (T + kParts - 1) / kParts, tb = part * per, te = min(T, tb + per);
     const FeatT *p = thr + f0 + c;
     int32_t prev = tb > 0 && tb < te ? (int32_t)ldg(p + (size_t)(tb - 1) * F) : 0;
-    for (uint32_t t = tb; t < te; t++) {
-      const int32_t v = (int32_t)ldg(p + (size_t)t * F);
-      if (t == 0 || v != prev) {
-        const uint32_t b = (uint32_t)(v - rt.lo);
-        atomicOr(&col[(b >> 5) * 32].x, 1u << (b & 31));
-        atomicOr(&rt.first[c * rt.first_words + (t >> 5)], 1u << (t & 31));
+    for (uint32_t t0 = tb; t0 < te; t0 += kThrAhead) {
+      int32_t v[kThrAhead];
+#pragma unroll
+      for (uint32_t i = 0; i < kThrAhead; i++) v[i] = t0 + i < te ? (int32_t)ldg(p + (size_t)(t0 + i) * F) : 0;
+#pragma unroll
+      for (uint32_t i = 0; i < kThrAhead; i++) {
+        const uint32_t t = t0 + i;
+        if (t < te && (t == 0 || v[i] != prev)) {
+          const uint32_t b = (uint32_t)(v[i] - rt.lo);
+          atomicOr(&col[(b >> 4) * 32], 1u << (b & 15));
+          atomicOr(&rt.first[c * rt.first_words + (t >> 5)], 1u << (t & 31));
+        }
+        prev = v[i];
       }
-      prev = v;
     }
   }
   __syncthreads();
   const uint32_t per = (rt.words + kParts - 1) / kParts, wb = part * per, we = min(rt.words, wb + per);
   uint32_t n = 0;
-  for (uint32_t k = wb; k < we; k++) n += __popc(col[k * 32].x);
+#pragma unroll 4
+  for (uint32_t k = wb; k < we; k++) n += __popc(col[k * 32]);
   s_part[part][c] = n;
   __syncthreads();
   uint32_t base = 0;
 #pragma unroll
   for (uint32_t q = 0; q < kParts; q++) base += q < part ? s_part[q][c] : 0u;
+#pragma unroll 4
   for (uint32_t k = wb; k < we; k++) {
-    const uint32_t bits = col[k * 32].x;
-    col[k * 32].y = base * 128u + (c & 31) * 4u;
+    const uint32_t bits = col[k * 32];
+    col[k * 32] = bits | (base * 128u + (c & 31) * 4u) << 16;
     base += __popc(bits);
   }
   __syncthreads();
@@ -713,12 +725,12 @@ PD_D uint32_t low_mask(uint32_t n) {  // bits below n mod 32
 }
 // Byte offset (row and lane) of the response's histogram word in its class block.
 template <bool SMALL>
-PD_D uint32_t rank_offset(int32_t r, int32_t lo, int32_t cap, const uint2 *col) {
+PD_D uint32_t rank_offset(int32_t r, int32_t lo, int32_t cap, const uint32_t *col) {
   uint32_t v;
   if constexpr (SMALL) v = (uint32_t)max(min(r - lo, cap), 0);
   else v = (uint32_t)(min(max(r, lo), lo + cap) - lo);
-  const uint2 e = *reinterpret_cast<const uint2 *>(reinterpret_cast<const char *>(col) + (v & ~31u) * 8u);
-  return e.y + (uint32_t)__popc(e.x & low_mask(v)) * 128u;
+  const uint32_t e = *reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(col) + (v & ~15u) * 8u);
+  return (e >> 16) + (uint32_t)__popc(e & low_mask(v & 15u)) * 128u;
 }
 
 // Staged words of a plugin without its own form, and of tiles that do not take it: position, preload words, size, image pointer, map offset.
@@ -784,7 +796,7 @@ PD_D RankTab rank_tab(uint32_t *at, uint32_t T, int32_t lo, uint32_t span) {
   rt.lo = lo;
   rt.cap = (int32_t)span + 1;
   rt.first = at;
-  rt.tab = reinterpret_cast<uint2 *>(at + kTileF * rt.first_words);
+  rt.tab = at + kTileF * rt.first_words;
   return rt;
 }
 
@@ -800,7 +812,7 @@ PD_D void hist_samples_rank(const DevSet &ds, const SampleRec *__restrict__ rec,
   constexpr uint32_t kWarps = NT / 32;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const typename S::Cand ca = tile_candidate<P, S>(feat, F, f0 + lane), cb = tile_candidate<P, S>(feat, F, f0 + 32 + lane);
-  const uint2 *ta = rt.tab + lane, *tb = ta + rt.words * 32;
+  const uint32_t *ta = rt.tab + lane, *tb = ta + rt.words * 32;
   const int32_t lo = rt.lo, cap = rt.cap;
   const uint32_t class_bytes = (T + 1) * 128;
   uint4 *st = sh_stage + warp * 64;
@@ -1222,7 +1234,8 @@ __device__ __forceinline__ void rank_item(const DevSet &ds, const SampleRec *__r
   uint32_t *sh_hist = reinterpret_cast<uint32_t *>(smem_raw);
   const uint32_t f0 = w.tile * kTileF;
   const RankTab rt = rank_tab(sh_hist + (size_t)K * (T + 1) * 32, T, lo, span);
-  for (uint32_t j = threadIdx.x; j < K * (T + 1) * 32; j += NT) sh_hist[j] = 0u;
+  for (uint32_t j = threadIdx.x; j < K * (T + 1) * 8; j += NT)
+    reinterpret_cast<uint4 *>(sh_hist)[j] = make_uint4(0, 0, 0, 0);
   build_rank_tab<NT>(rt, cand_thr + (size_t)w.slot * T * F, F, T, f0);
   hist_samples_tile<P, SPI, NT>(ds, rec, w, cand_feat + (size_t)w.slot * P::kFeatDim * F, F, f0, sh_hist, rt, T,
                                 [](uint32_t l) { return l; });
@@ -1439,7 +1452,8 @@ __global__ void __launch_bounds__(small_threads(NC), small_ctas(NC))
       s_idx = ~0ull;
     }
   }
-  for (uint32_t j = threadIdx.x; j < NC * TS * 32; j += kSmallThreads) sh_hist[j] = 0u;
+  for (uint32_t j = threadIdx.x; j < NC * TS * 8; j += kSmallThreads)
+    reinterpret_cast<uint4 *>(sh_hist)[j] = make_uint4(0, 0, 0, 0);
   prefetch_fused(fs, w, f0, F, T);
   build_rank_tab<kSmallThreads>(rt, cand_thr + (size_t)slot * T * F, F, T, f0);
   hist_samples_tile<P, kSmallSpi, kSmallThreads>(ds, rec, w, cand_feat + (size_t)slot * P::kFeatDim * F, F, f0, sh_hist, rt, T,
