@@ -40,7 +40,9 @@ constexpr uint32_t kRankWordsMax = 128;  // rank-table words per column: thresho
 // Table words per column for thresholds in [lo, lo + span] (responses reach span + 1).
 PD_HD constexpr uint32_t rank_words(uint32_t span) { return (span + 1) / 16 + 1; }
 PD_HD constexpr int hist_threads(uint32_t TP) { return TP ? kHistThreads : kRankThreads; }
-constexpr int kScanItems = 4096;   // active samples per scan block (256 threads x 16)
+// Active samples per scan block (256 threads x 4): 32 000 samples fill 32 blocks of the
+// scatter (16 a thread in 8 blocks took 16 us, this 6).
+constexpr int kScanItems = 1024;
 // FP32 gain window rechecked in FP64.  Each FP32 entropy term -p log2 p (fast
 // reciprocal and log2) is within about 2e-7 of its exact value and each of the
 // ~K additions of an entropy adds at most 2.4e-7, so |gain32 - gain64| stays
@@ -418,7 +420,8 @@ struct SplitPart {
 };
 
 constexpr int kSplitCols = 128;  // threads of a split CTA, one column each per pass
-constexpr int kSplitRows = 4;    // histogram rows loaded together in pass 1
+// histogram rows loaded together in pass 1 (KM registers each)
+PD_HD constexpr int split_rows(int KM) { return KM <= 4 ? 10 : 4; }
 
 // Reference-formula FP32 entropy (kernels/learn_best_feature.cl:75-93) with the
 // p <= 1e-6 cutoff as the integer test 1e6*c <= n; fast intrinsics, error well
@@ -1704,7 +1707,8 @@ __global__ void k_split_params(const SplitOut *__restrict__ out, uint32_t n, con
   if (o.t < 0 || o.col < 0) return;
   const uint32_t col = (uint32_t)o.col;
   for (int d = 0; d < D; d++) params[(size_t)i * (D + 1) + d] = cand_feat[((size_t)i * D + d) * F + col];
-  for (uint32_t j = 0; j < T; j++)
+#pragma unroll 10
+  for (uint32_t j = 0; j < T; j++)  // the loads do not wait for each other
     if (perm[((size_t)i * T + j) * F + col] == (uint8_t)o.t) params[(size_t)i * (D + 1) + D] = cand_thr[((size_t)i * T + j) * F + col];
 }
 
@@ -1801,7 +1805,8 @@ __global__ void __launch_bounds__(kSplitCols) k_split_g32(SplitArgs a) {
 #pragma unroll
     for (int l = 0; l < KM; l++) c[l] = 0u;
     float g = 0.0f;
-    // rows are loaded kSplitRows at a time so their loads are in flight together
+    // rows are loaded split_rows(KM) at a time so their loads are in flight together
+    constexpr int kSplitRows = split_rows(KM);
     for (uint32_t j0 = 0; j0 < T; j0 += kSplitRows) {
       uint32_t h[kSplitRows][KM];
 #pragma unroll
