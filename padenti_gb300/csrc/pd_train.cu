@@ -299,14 +299,21 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
   const bool rank = rank_form(ctx, p, prop);
   const uint32_t span = rank ? (uint32_t)(p->thr_up - p->thr_low) : 0u;
   // Samples per work item: the chunk, or less when the level has too few tiles to
-  // fill the GPU (four items a resident CTA, at least kMinChunk samples each: the
-  // set-up of a tile costs about as much as 200 samples).  64 maps of 160x120 with
-  // 200 candidates: the root's 8 CTAs of 16384 samples took 0.33 ms, its 500 of 256
-  // take 0.05 ms.
-  constexpr uint64_t kMinChunk = 256;
+  // fill the GPU: four items per SM, fewer when they would be small (the set-up and
+  // flush of a tile cost about as much as 800 samples), one at least.  64 maps of
+  // 160x120 with 200 candidates: the root's 8 CTAs of 16384 samples took 0.33 ms, its
+  // 500 of 256 0.05; four items per SM on every level 0.322 ms of histograms a tree,
+  // this rule 0.280.
+  static constexpr uint64_t kMinChunk = 256;
   const uint64_t total = off[n] - off[0];
-  const uint64_t want = (total * tiles + 4ull * ctx->n_sms - 1) / (4ull * ctx->n_sms);
-  const uint64_t chunk = rank ? std::min<uint64_t>(ctx->chunk, std::max(kMinChunk, (want + 31) / 32 * 32)) : ctx->chunk;
+  const uint64_t per_sm = (total * tiles + ctx->n_sms - 1) / ctx->n_sms;
+  auto round32 = [](uint64_t v) { return std::max<uint64_t>(kMinChunk, (v + 31) / 32 * 32); };
+  const uint64_t items_per_sm = std::min<uint64_t>(4, std::max<uint64_t>(1, per_sm / 1024));
+  const uint64_t chunk =
+      rank ? std::min<uint64_t>(ctx->chunk, round32((per_sm + items_per_sm - 1) / items_per_sm)) : ctx->chunk;
+  // a fused node runs on a CTA of fewer warps: on a small level only short ones do
+  const uint64_t fuse_max = rank ? std::min({(uint64_t)ctx->fuse_max, chunk, round32((per_sm + 3) / 4)})
+                                 : std::min<uint64_t>(ctx->fuse_max, chunk);
   // Per node: fused (a small-node launch of its class count in the rank-table form,
   // an item with multi = 2 in the search form) or chunked.  The list is written
   // straight into pinned staging: the items of k_hist -- for a persistent launch
@@ -319,7 +326,7 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
   for (uint32_t i = 0; i < n; i++) {
     const uint64_t cnt = off[i + 1] - off[i], chunks = (cnt + chunk - 1) / chunk;
     int k = cnt ? -1 : -2;
-    if (split_slots && chunks == 1 && cnt <= ctx->fuse_max) {
+    if (split_slots && cnt && cnt <= fuse_max) {
       if (!rank) {
         k = -3;
       } else {
