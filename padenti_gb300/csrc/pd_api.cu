@@ -80,7 +80,12 @@ extern "C" int pd_ctx_create(const pd_config *cfg, int device, pd_ctx **out) {
     return set_error(PD_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
   }
   for (auto &ev : c->ev) cudaEventCreate(&ev);
-  const int rc = init_tables(c);
+  e = cudaEventCreateWithFlags(&c->hist_fork, cudaEventDisableTiming);
+  for (int i = 0; i < 4 && e == cudaSuccess; i++) {
+    e = cudaStreamCreateWithFlags(&c->hist_side[i], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->hist_join[i], cudaEventDisableTiming);
+  }
+  const int rc = e == cudaSuccess ? init_tables(c) : set_error(PD_ERR_CUDA, "cudaStreamCreate: %s", cudaGetErrorString(e));
   if (rc != PD_OK) {
     pd_ctx_destroy(c);
     return rc;
@@ -140,6 +145,11 @@ extern "C" int pd_ctx_destroy(pd_ctx *ctx) {
   ctx->h_chk.release();
   for (auto &ev : ctx->ev)
     if (ev) cudaEventDestroy(ev);
+  for (int i = 0; i < 4; i++) {
+    if (ctx->hist_join[i]) cudaEventDestroy(ctx->hist_join[i]);
+    if (ctx->hist_side[i]) cudaStreamDestroy(ctx->hist_side[i]);
+  }
+  if (ctx->hist_fork) cudaEventDestroy(ctx->hist_fork);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
   return PD_OK;

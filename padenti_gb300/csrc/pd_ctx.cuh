@@ -19,6 +19,10 @@ struct pd_ctx {
   pd::RtcPlugin *rtc = nullptr;  // the compiled user feature plugin (PD_PLUGIN_USER)
   bool tree_feature = false;     // its computeFeature reads the tree: the node map is kept
   cudaStream_t stream = nullptr;
+  // the small-node histogram launches of a level run beside its k_hist: forked from
+  // stream, joined to it before anything else is enqueued (pd_hist_grid.cuh)
+  cudaStream_t hist_side[4] = {};
+  cudaEvent_t hist_fork = nullptr, hist_join[4] = {};
   uint64_t hist_budget = 8ull << 30;
   uint32_t chunk = 16384;  // samples per histogram work item (at most 65535)
   uint32_t hist_spi = 8;  // samples per iteration of the histogram kernel (2, 4 or 8)

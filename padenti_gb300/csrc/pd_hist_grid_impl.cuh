@@ -41,7 +41,8 @@ static int launch_hist_grid_as(pd_ctx *ctx, const HistGrid &g) {
 
 // The small nodes of one class bucket: k_hist_small<P, NC>, one CTA per tile.
 template <class P, int NC>
-static int launch_small_as(pd_ctx *ctx, const HistGrid &g, const WorkItem *items, uint64_t n, size_t smem) {
+static int launch_small_as(pd_ctx *ctx, const HistGrid &g, const WorkItem *items, uint64_t n, size_t smem,
+                           cudaStream_t st) {
   using FeatT = typename P::feat_t;
   auto kern = k_hist_small<P, NC>;
   PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -49,7 +50,7 @@ static int launch_small_as(pd_ctx *ctx, const HistGrid &g, const WorkItem *items
   const uint64_t most = 0x7fffffffull / g.tiles;
   for (uint64_t b = 0; b < n; b += most) {
     const uint64_t cnt = std::min<uint64_t>(n - b, most);
-    kern<<<(unsigned)(cnt * g.tiles), small_threads(NC), smem, ctx->stream>>>(
+    kern<<<(unsigned)(cnt * g.tiles), small_threads(NC), smem, st>>>(
         g.ds, g.rec, items + b, static_cast<const FeatT *>(g.cand_feat), static_cast<const FeatT *>(g.cand_thr), g.F,
         g.T, g.K, g.fs, g.thr_lo, g.thr_span);
     PD_CUDA(cudaGetLastError());
@@ -61,15 +62,19 @@ static int launch_small_as(pd_ctx *ctx, const HistGrid &g, const WorkItem *items
 template <class P>
 static int launch_small(pd_ctx *ctx, const HistGrid &g) {
   const WorkItem *items = g.items + g.n_items;
-  for (const auto &s : g.small) {
+  for (int b = 0; b < 4; b++) {
+    const auto &s = g.small[b];
     if (!s.n_items) continue;
+    cudaStream_t st;
+    PD_TRY(hist_stream(ctx, g, b, &st));
     switch (s.nc) {
-      case 4: PD_TRY((launch_small_as<P, 4>(ctx, g, items, s.n_items, s.smem))); break;
-      case 8: PD_TRY((launch_small_as<P, 8>(ctx, g, items, s.n_items, s.smem))); break;
-      case 16: PD_TRY((launch_small_as<P, 16>(ctx, g, items, s.n_items, s.smem))); break;
-      case 32: PD_TRY((launch_small_as<P, 32>(ctx, g, items, s.n_items, s.smem))); break;
+      case 4: PD_TRY((launch_small_as<P, 4>(ctx, g, items, s.n_items, s.smem, st))); break;
+      case 8: PD_TRY((launch_small_as<P, 8>(ctx, g, items, s.n_items, s.smem, st))); break;
+      case 16: PD_TRY((launch_small_as<P, 16>(ctx, g, items, s.n_items, s.smem, st))); break;
+      case 32: PD_TRY((launch_small_as<P, 32>(ctx, g, items, s.n_items, s.smem, st))); break;
       default: return set_error(PD_ERR_STATE, "no small-node kernel of %d classes", s.nc);
     }
+    PD_TRY(hist_join(ctx, b, st));
     items += s.n_items;
   }
   return PD_OK;
@@ -86,10 +91,7 @@ static int launch_hist_grid_tp(pd_ctx *ctx, const HistGrid &g) {
 }
 
 template <class P>
-int launch_hist_grid(pd_ctx *ctx, const HistGrid &g) {
-  if (g.ev_before) PD_CUDA(cudaEventRecord(g.ev_before, ctx->stream));
-  PD_TRY(launch_small<P>(ctx, g));
-  if (!g.n_items) return PD_OK;
+static int launch_big(pd_ctx *ctx, const HistGrid &g) {
   switch (g.TP) {
     case 0: return ctx->hist_spi == 8 ? launch_hist_grid_as<P, 0, 8>(ctx, g) : launch_hist_grid_as<P, 0, 4>(ctx, g);
     case 2: return launch_hist_grid_tp<P, 2>(ctx, g);
@@ -103,6 +105,14 @@ int launch_hist_grid(pd_ctx *ctx, const HistGrid &g) {
     case 512: return launch_hist_grid_tp<P, 512>(ctx, g);
     default: return set_error(PD_ERR_UNSUPPORTED, "n_thresholds %u", g.T);
   }
+}
+
+template <class P>
+int launch_hist_grid(pd_ctx *ctx, const HistGrid &g) {
+  if (g.ev_before) PD_CUDA(cudaEventRecord(g.ev_before, ctx->stream));
+  PD_TRY(hist_fork(ctx, g));
+  if (g.n_items) PD_TRY(launch_big<P>(ctx, g));
+  return launch_small<P>(ctx, g);
 }
 
 }  // namespace pd

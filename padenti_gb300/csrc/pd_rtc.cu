@@ -153,8 +153,8 @@ int rtc_set_smem(pd_ctx *ctx, cudaKernel_t k, size_t smem, int carveout_pct) {
   return PD_OK;
 }
 
-int rtc_launch(pd_ctx *ctx, cudaKernel_t k, dim3 grid, dim3 block, size_t smem, void **args) {
-  PD_CUDA(cudaLaunchKernel((const void *)k, grid, block, args, smem, ctx->stream));
+int rtc_launch(pd_ctx *ctx, cudaKernel_t k, dim3 grid, dim3 block, size_t smem, void **args, cudaStream_t st) {
+  PD_CUDA(cudaLaunchKernel((const void *)k, grid, block, args, smem, st ? st : ctx->stream));
   ctx->launches++;
   return PD_OK;
 }
@@ -183,35 +183,40 @@ int launch_hist_grid_rtc(pd_ctx *ctx, const HistGrid &g) {
   if (g.n_items)
     PD_TRY(rtc_hist(ctx, "pd::k_hist<pd::UserPlugin, " + std::to_string(g.TP) + ", " + std::to_string(spi) + ">", &uk));
   if (g.ev_before) PD_CUDA(cudaEventRecord(g.ev_before, ctx->stream));
+  PD_TRY(hist_fork(ctx, g));
+  if (g.n_items) {
+    // shared memory carve-out for the resident CTAs (dynamic + a static allowance + reserved)
+    const size_t per_cta = g.smem + 4096 + 1024;
+    const int pct = (int)std::min<size_t>(100, (resident * per_cta * 100 + 233471) / 233472);
+    PD_TRY(rtc_set_smem(ctx, uk, g.smem, pct));
+    if (g.queue) PD_CUDA(cudaMemsetAsync(g.queue, 0, 4, ctx->stream));
+    for (uint64_t b = 0; b < g.n_items; b += most) {
+      const uint64_t cnt = std::min<uint64_t>(g.n_items - b, most);
+      const WorkItem *it = g.items + b;
+      uint32_t n = (uint32_t)cnt;
+      unsigned *queue = g.queue;
+      void *args[] = {&ds, &rec, &it, &n, &queue, &cf, &ct, &hist, &F, &T, &K, &fs, &lo, &span};
+      const unsigned grid = g.queue ? (unsigned)std::min<uint64_t>(cnt * g.tiles, (uint64_t)ctx->n_sms * resident)
+                                    : (unsigned)(cnt * g.tiles);
+      PD_TRY(rtc_launch(ctx, uk, dim3(grid), dim3(hist_threads(g.TP)), g.smem, args));
+      if (g.queue) break;
+    }
+  }
   const WorkItem *items = g.items + g.n_items;
   for (int i = 0; i < 4; i++) {
     const auto &s = g.small[i];
     if (!s.n_items) continue;
+    cudaStream_t st;
+    PD_TRY(hist_stream(ctx, g, i, &st));
     PD_TRY(rtc_set_smem(ctx, sk[i], s.smem, small_carveout(s.nc, s.smem)));
     for (uint64_t b = 0; b < s.n_items; b += most) {
       const uint64_t cnt = std::min<uint64_t>(s.n_items - b, most);
       const WorkItem *it = items + b;
       void *args[] = {&ds, &rec, &it, &cf, &ct, &F, &T, &K, &fs, &lo, &span};
-      PD_TRY(rtc_launch(ctx, sk[i], dim3((unsigned)(cnt * g.tiles)), dim3(small_threads(s.nc)), s.smem, args));
+      PD_TRY(rtc_launch(ctx, sk[i], dim3((unsigned)(cnt * g.tiles)), dim3(small_threads(s.nc)), s.smem, args, st));
     }
+    PD_TRY(hist_join(ctx, i, st));
     items += s.n_items;
-  }
-  if (!g.n_items) return PD_OK;
-  // shared memory carve-out for the resident CTAs (dynamic + a static allowance + reserved)
-  const size_t per_cta = g.smem + 4096 + 1024;
-  const int pct = (int)std::min<size_t>(100, (resident * per_cta * 100 + 233471) / 233472);
-  PD_TRY(rtc_set_smem(ctx, uk, g.smem, pct));
-  if (g.queue) PD_CUDA(cudaMemsetAsync(g.queue, 0, 4, ctx->stream));
-  for (uint64_t b = 0; b < g.n_items; b += most) {
-    const uint64_t cnt = std::min<uint64_t>(g.n_items - b, most);
-    const WorkItem *it = g.items + b;
-    uint32_t n = (uint32_t)cnt;
-    unsigned *queue = g.queue;
-    void *args[] = {&ds, &rec, &it, &n, &queue, &cf, &ct, &hist, &F, &T, &K, &fs, &lo, &span};
-    const unsigned grid = g.queue ? (unsigned)std::min<uint64_t>(cnt * g.tiles, (uint64_t)ctx->n_sms * resident)
-                                  : (unsigned)(cnt * g.tiles);
-    PD_TRY(rtc_launch(ctx, uk, dim3(grid), dim3(hist_threads(g.TP)), g.smem, args));
-    if (g.queue) break;
   }
   return PD_OK;
 }

@@ -21,7 +21,7 @@ struct RtcKernels {
 int rtc_kernels(pd_ctx *ctx, const RtcKernels **out);
 // Dynamic shared memory limit (and carve-out when pct >= 0) of a kernel.
 int rtc_set_smem(pd_ctx *ctx, cudaKernel_t k, size_t smem, int carveout_pct = -1);
-int rtc_launch(pd_ctx *ctx, cudaKernel_t k, dim3 grid, dim3 block, size_t smem, void **args);
+int rtc_launch(pd_ctx *ctx, cudaKernel_t k, dim3 grid, dim3 block, size_t smem, void **args, cudaStream_t st = nullptr);
 void rtc_release(pd_ctx *ctx);
 
 inline bool is_user_plugin(const pd_ctx *ctx) { return ctx->cfg.plugin == PD_PLUGIN_USER; }

@@ -25,14 +25,16 @@ constexpr int kHistThreads = 256;  // 8 warps, each on its own samples (search f
 // that most of the SM's 256 KB stays L1 for the probe gathers, which bound the loop:
 // root of 200 640x480 depth maps (8.2e8 evaluations), one CTA of 512 threads 1.70 ms
 // (L1 hit rate 82 %, 18 cycles per 32 evaluations), two of 256 2.58 ms (35 %, 26
-// cycles); 768 and 1024 threads were 7 and 18 % slower over a tree (more windows
-// in flight than L1 holds).  The search form's two CTAs: 2.68 ms.
+// cycles; both with 64-bit table words).  768 threads are 5-8 % slower over a tree and
+// 640 2 % (more windows in flight than L1 holds), 1024 were 18 %.  The search form's
+// two CTAs: 2.68 ms.
 constexpr int kRankThreads = 512;
 constexpr int kRankCtas = 1;
 // Small nodes (split fused), by class rows: 16 warps per SM, in as many CTAs as the
 // histogram rows leave L1 for, so that the barriers of one item hide behind the
-// others (a depth-16 tree on 600 maps, all histogram launches: 114.8 ms; 8 rows in
-// three CTAs of 128 threads and 16 rows in two: 142.5 ms).
+// others (a depth-16 tree on 600 maps, all histogram launches, with 64-bit table
+// words: 114.8 ms; 8 rows in three CTAs of 128 threads and 16 rows in two: 142.5 ms.
+// With 32-bit words 108.5 ms; five CTAs for 4 rows 116, 192 to 384 threads no faster).
 PD_HD constexpr int small_threads(int NC) { return NC <= 4 ? 128 : NC <= 8 ? 256 : 512; }
 PD_HD constexpr int small_ctas(int NC) { return NC <= 4 ? 4 : NC <= 8 ? 2 : 1; }
 constexpr int kSmallSpi = 4;  // samples per warp iteration (8 measured the same, with more registers)
