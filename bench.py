@@ -286,7 +286,9 @@ def sampler_bench(a, pg, N, px, lb):
             draw.append(st["ms_draw"])
         wall = (time.perf_counter() - t0) * 1000 / reps
         ms_scan, ms_draw = float(np.median(scan)), float(np.median(draw))
-        scan_bytes = n * a.width * a.height * 3  # image bytes (2 per pixel) + label bytes (1 per pixel)
+        # image bytes (2 per pixel); the uniform sampler's scan counts labels too (1 per pixel)
+        scan_key = "k_sample_scan" if name == "uniform" else "k_sample_scan_no_labels"
+        scan_bytes = n * a.width * a.height * (3 if name == "uniform" else 2)
         # host buffers in, samples out
         imgs, lbs = px[:n], lb[:n]  # the stacked-array form of sample_batch
         sm.sample_batch(imgs, lbs)
@@ -302,7 +304,7 @@ def sampler_bench(a, pg, N, px, lb):
             roofline=dict(kernel="k_sample_scan", bound="hbm", achieved=scan_bytes / (ms_scan / 1000) / 1e9,
                           peak=peak, unit="GB/s", frac=scan_bytes / (ms_scan / 1000) / 1e9 / peak,
                           algorithmic_bytes=scan_bytes,
-                          traffic=(lambda v: None if v is None else v * n)(profile_dram_per_image("k_sample_scan")),
+                          traffic=(lambda v: None if v is None else v * n)(profile_dram_per_image(scan_key)),
                           traffic_note="DRAM bytes of a 300-image ncu capture, scaled by the images"),
             e2e=dict(value=n / (e2e_ms / 1000), unit="images/s", ms=e2e_ms, h2d_bytes=est["h2d_bytes"],
                      d2h_bytes=est["d2h_bytes"]))
@@ -1010,8 +1012,8 @@ def run_ours(a):
                 algorithmic_bytes_per_launch=hist_bytes / max(1, hist_launches),
                 launch_ms=hist_ms / max(1, hist_launches),
                 evals_per_s_in_kernel=evals / hist_s if hist_s > 0 else None,
-                note="the histogram kernel is bound by instruction issue and the L1 data pipe (probe gathers, "
-                     "threshold search), not by HBM")
+                note="the histogram kernel is bound by the L1 data pipe (probe gathers) and instruction issue, "
+                     "not by HBM")
     # the histogram kernel's own bound: instruction issue (lane slots of warp instructions)
     issue_roof = None
     ip = ROOT / "profiles" / "k_hist_issue_300x640x480.json"

@@ -161,8 +161,11 @@ int pd_plugin_check(const pd_config *cfg, const char *source, char *log, size_t 
  * reference does with its 20 GiB host cap (cl_tree_trainer_impl.hpp:47-50). */
 int pd_ctx_set_hist_budget(pd_ctx *ctx, uint64_t bytes);
 /* Launch-shape knobs of the histogram kernel (results do not depend on them):
- *   "chunk"     samples per histogram work item, [256, 65535] (default 16384);
+ *   "chunk"     samples per histogram work item, [256, 65535] (default 16384); at most
+ *               that many where thresholds are looked up (ranges up to 2046): levels
+ *               too small to fill the GPU are cut finer;
  *   "hist_spi"  samples evaluated together per warp iteration, 2, 4 or 8 (default 8);
+ *               2 acts as 4 where thresholds are looked up;
  *   "fuse_max"  nodes with at most this many samples (and within one work item)
  *               get their split computed inside the histogram kernel, [0, 65535];
  *   "cand_order" 1 (default): each node's candidate table is laid out in the
