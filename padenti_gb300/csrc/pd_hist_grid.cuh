@@ -19,7 +19,8 @@ struct HistGrid {
   uint32_t tiles;
   // rank-table form: small nodes (fused split) by the class rows of their kernel
   struct Small {
-    int nc;               // k_hist_small<P, nc>; 0: no such launch
+    int nc;               // k_hist_small<P, nc>
+    bool may;             // a level of this training call may need it
     uint64_t n_items;
     size_t smem;
   } small[4];

@@ -10,6 +10,8 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "pd_hist_grid.cuh"
@@ -124,24 +126,47 @@ int rtc_kernels(pd_ctx *ctx, const RtcKernels **out) {
   return PD_OK;
 }
 
-// A histogram kernel of the plugin, compiled on first use.
-static int rtc_hist(pd_ctx *ctx, const std::string &expr, cudaKernel_t *out) {
+// Histogram kernels of the plugin, compiled on first use: those missing at once, a
+// thread each (NVRTC compiles concurrently; a thread's error is reported by the
+// caller's).  An RGB feature's first tree with its three kernels: 2.84 s one after the
+// other, 1.17 together (one search-form kernel took 1.89).
+static int rtc_hist(pd_ctx *ctx, const std::vector<std::string> &exprs) {
   PD_CHECK(ctx->rtc, PD_ERR_STATE, "the user feature plugin is not compiled (pd_plugin_compile)");
-  auto it = ctx->rtc->hist.find(expr);
-  if (it != ctx->rtc->hist.end()) {
-    *out = it->second;
-    return PD_OK;
+  struct Job {
+    std::string expr, cubin, log;
+    std::vector<std::string> low;
+    int rc = PD_OK;
+  };
+  std::vector<Job> jobs;
+  for (const auto &e : exprs)
+    if (!ctx->rtc->hist.count(e)) jobs.emplace_back().expr = e;
+  auto compile = [&](Job &j) noexcept {
+    try {
+      j.rc = compile_unit(ctx->cfg, ctx->rtc->source, ctx->rtc->arch, {j.expr}, &j.cubin, &j.low, nullptr);
+      if (j.rc != PD_OK) j.log = pd_last_error();
+    } catch (const std::exception &) {
+      j.rc = PD_ERR_STATE;  // out of host memory
+    }
+  };
+  std::vector<std::thread> threads;
+  threads.reserve(jobs.size());
+  for (size_t i = 1; i < jobs.size(); i++) {
+    try {
+      threads.emplace_back(compile, std::ref(jobs[i]));
+    } catch (const std::system_error &) {
+      compile(jobs[i]);  // no thread to be had
+    }
   }
-  const std::vector<std::string> exprs = {expr};
-  std::string cubin;
-  std::vector<std::string> low;
-  PD_TRY(compile_unit(ctx->cfg, ctx->rtc->source, ctx->rtc->arch, exprs, &cubin, &low, nullptr));
-  cudaLibrary_t lib = nullptr;
-  std::vector<cudaKernel_t> ks;
-  PD_TRY(load_kernels(cubin, low, &lib, &ks));
-  ctx->rtc->libs.push_back(lib);
-  ctx->rtc->hist[expr] = ks[0];
-  *out = ks[0];
+  if (!jobs.empty()) compile(jobs[0]);
+  for (auto &t : threads) t.join();
+  for (auto &j : jobs) {
+    if (j.rc != PD_OK) return set_error(j.rc, "%s", j.log.c_str());
+    cudaLibrary_t lib = nullptr;
+    std::vector<cudaKernel_t> ks;
+    PD_TRY(load_kernels(j.cubin, j.low, &lib, &ks));
+    ctx->rtc->libs.push_back(lib);
+    ctx->rtc->hist[j.expr] = ks[0];
+  }
   return PD_OK;
 }
 
@@ -176,12 +201,16 @@ int launch_hist_grid_rtc(pd_ctx *ctx, const HistGrid &g) {
   uint32_t span = g.thr_span;
   const uint64_t most = 0x7fffffffull / g.tiles;  // items of one grid
   // the kernels first, so that their compilation stays outside the timed launches
-  cudaKernel_t uk = nullptr, sk[4] = {};
+  const std::string big = "pd::k_hist<pd::UserPlugin, " + std::to_string(g.TP) + ", " + std::to_string(spi) + ">";
+  auto small = [&](int i) { return "pd::k_hist_small<pd::UserPlugin, " + std::to_string(g.small[i].nc) + ">"; };
+  std::vector<std::string> exprs;
+  if (g.n_items) exprs.push_back(big);
   for (int i = 0; i < 4; i++)
-    if (g.small[i].n_items)
-      PD_TRY(rtc_hist(ctx, "pd::k_hist_small<pd::UserPlugin, " + std::to_string(g.small[i].nc) + ">", &sk[i]));
-  if (g.n_items)
-    PD_TRY(rtc_hist(ctx, "pd::k_hist<pd::UserPlugin, " + std::to_string(g.TP) + ", " + std::to_string(spi) + ">", &uk));
+    if (g.small[i].may) exprs.push_back(small(i));
+  PD_TRY(rtc_hist(ctx, exprs));
+  cudaKernel_t uk = g.n_items ? ctx->rtc->hist[big] : nullptr, sk[4] = {};
+  for (int i = 0; i < 4; i++)
+    if (g.small[i].n_items) sk[i] = ctx->rtc->hist[small(i)];
   if (g.ev_before) PD_CUDA(cudaEventRecord(g.ev_before, ctx->stream));
   PD_TRY(hist_fork(ctx, g));
   if (g.n_items) {

@@ -448,6 +448,8 @@ static int launch_hist(pd_ctx *ctx, const pd_train_params *p, const uint64_t *of
   g.tiles = tiles;
   for (int b = 0; b < 4; b++) {
     g.small[b].nc = kSmallRows[b];
+    g.small[b].may = n_small[b] || (rank && split_slots && ctx->fuse_max && (b == 1 || (b == 3 && K > 8)) &&
+                                    rank_smem(kSmallRows[b], T, span, small_threads(kSmallRows[b])) <= kRankSmemMax);
     g.small[b].n_items = n_small[b];
     g.small[b].smem = n_small[b] ? rank_smem(kSmallRows[b], T, span, small_threads(kSmallRows[b])) : 0;
   }
