@@ -104,7 +104,9 @@ struct pd_ctx {
   pd::DevBuf f_lc, f_feat, f_thr, f_post, f_meta;
   pd::DevBuf f_cand;                   // FastNode or NodeRec of every forest node
   pd::DevBuf f_post4;                  // posteriors padded to four classes a word (k_pad_posteriors)
+  pd::DevBuf f_gen;                    // NodeRec beside FastNode, for images past the fast form's sides
   uint64_t cand_version = ~0ull;       // forest_version f_cand was built for
+  uint64_t gen_version = ~0ull;        // forest_version f_gen was built for
   bool forest_fast = false;            // every node takes the plugin's fast path (built-in plugins)
   pd::DevBuf f_fast;                   // its device flag
   pd::DevBuf p_img, p_mask, p_out;     // staging for host-buffer prediction

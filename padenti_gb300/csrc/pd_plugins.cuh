@@ -17,6 +17,8 @@
 //   fast_words(im, x, y, pre, w)  the words of a pixel;
 //   eval_fast<MAPPED>(a, b, cand)  the response from words a = w[0..3], b = w[4..7];
 //                            MAPPED: on the trainer's copy of the images;
+//   kFastSide                the longest image side this form is exact for (training and
+//                            batches take sides below 2^16, the other prediction calls any);
 // and kOrderDim, the feature dims (kOrderDim, kOrderDim + 1) of its first probe
 // offset, by which the trainer orders a node's candidates.
 // eval(prep, f) runs all of it for a single evaluation.
@@ -129,7 +131,7 @@ struct OffsetConst {
 
 // The same rounding in one fused multiply-add.  With i = fl(1/d), u' = u + 1/4
 // sgn(u) and M = 3*2^22, fl(u' i + (M + x)) - M is x + round_half_away(u / d) for
-// |u| <= 2^21, |d| in [1, 65535] and 0 <= x < 2^16: floats in [2^23, 2^24) are the
+// |u| <= 2^21, |d| in [1, 65535] and 0 <= x < 2^21: floats in [2^23, 2^24) are the
 // integers, so the fused operation rounds the exact u' i + M + x once, to the
 // nearest integer.  |u|/d + 1/2 lies a multiple of 1/(2d) above an integer; the
 // quarter moves it to at least 1/(4d) from both ends of its unit interval, so no
@@ -257,6 +259,7 @@ struct DepthDiff2 {
   static PD_D int32_t eval_train(const Prep &p, const Cand &c) { return eval<FAST, true>(p, c); }
   static PD_D int32_t eval(const Prep &p, const int32_t *f) { return eval(p, candidate(f)); }
   // ---- words 1/d, M + x, M + y, -, image, w, h ----
+  static constexpr uint32_t kFastSide = 1u << 21;  // M + x + an offset of up to 2^21 stays below 2^24
   static constexpr bool kSmallResp = true;    // |response| < 2^17
   struct FastCand {
     float o[4];
@@ -373,6 +376,7 @@ struct DepthDiff1 {
   // ---- words 1/d, M + x, M + y, -, image, w | h << 16, d.  A zero centre depth
   // reads every probe as outside (w = 0); the rounding is odd in d, so a negative
   // one (a depth above 32767 read as short) needs no other form. ----
+  static constexpr uint32_t kFastSide = 65535u;  // both sides in one word
   static constexpr bool kSmallResp = true;
   struct FastCand {
     float o[2];
@@ -464,6 +468,7 @@ struct ChannelDiff {
   // ---- words 3w, x, y, -, the pixel's address, w, h.  A probe is uy * 3w + (3 ux +
   // c) bytes from the pixel (an offset that leaves the image loads nothing, whatever
   // 3 ux wraps to). ----
+  static constexpr uint32_t kFastSide = 1u << 29;  // 3w is a positive 32-bit number
   static constexpr bool kSmallResp = true;
   struct FastCand {
     int32_t ux, uy, vx, vy;

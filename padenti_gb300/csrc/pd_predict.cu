@@ -108,6 +108,45 @@ static int ensure_forest_nodes(pd_ctx *ctx) {
   return PD_OK;
 }
 
+// Whether a W x H image is walked in the plugin's fast form: the whole forest takes it,
+// and the form is exact for the sides.  Longer images take the general records, which
+// hold for every side (the eight words of a pixel have no room for more).
+template <class P>
+static bool fast_form(const pd_ctx *ctx, uint32_t W, uint32_t H) {
+  if constexpr (P::kRtcOnly) return false;
+  else return ctx->forest_fast && std::max(W, H) <= P::kFastSide;
+}
+
+// The general record of every node: f_cand, or for a forest in the fast form, whose
+// f_cand holds FastNode, f_gen, built when an image first needs it.
+template <class P>
+static int general_nodes(pd_ctx *ctx, const NodeRec<P> **out) {
+  if (!ctx->forest_fast) {
+    *out = ctx->f_cand.as<NodeRec<P>>();
+    return PD_OK;
+  }
+  const unsigned long long nodes = ctx->h_lc.size();
+  if (ctx->gen_version != ctx->forest_version) {
+    using FeatT = typename P::feat_t;
+    PD_TRY(ctx->f_gen.ensure(nodes * sizeof(NodeRec<P>) + 16));
+    k_forest_nodes<P><<<(unsigned)((nodes + 255) / 256), 256, 0, ctx->stream>>>(
+        ctx->f_feat.as<FeatT>(), ctx->f_thr.as<FeatT>(), ctx->f_lc.as<int32_t>(), nodes, ctx->f_gen.as<NodeRec<P>>());
+    PD_CUDA(cudaGetLastError());
+    ctx->launches++;
+    ctx->gen_version = ctx->forest_version;
+  }
+  *out = ctx->f_gen.as<NodeRec<P>>();
+  return PD_OK;
+}
+
+// The records of the form (AF: fast) that a call takes.
+template <class P, bool AF>
+static int form_nodes(pd_ctx *ctx, const Node<P, AF> **out) {
+  if constexpr (AF) *out = ctx->f_cand.as<FastNode<P>>();
+  else PD_TRY(general_nodes<P>(ctx, out));
+  return PD_OK;
+}
+
 template <class P>
 static int launch_posterior(pd_ctx *ctx, uint32_t n, const void *images, uint32_t W, uint32_t H,
                             const uint8_t *masks, float *out) {
@@ -134,14 +173,16 @@ static int launch_posterior(pd_ctx *ctx, uint32_t n, const void *images, uint32_
   if constexpr (!P::kRtcOnly) {
     auto launch = [&]<bool AF>() -> int {
       auto kern = k_predict_posterior<P, AF>;
+      const Node<P, AF> *nd = nullptr;
+      PD_TRY((form_nodes<P, AF>(ctx, &nd)));
       PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       kern<<<grid, dim3(kPredX, kPredY), smem, ctx->stream>>>(
-          static_cast<const uint8_t *>(images), img_bytes, W, H, masks, out, ctx->f_cand.as<Node<P, AF>>(),
+          static_cast<const uint8_t *>(images), img_bytes, W, H, masks, out, nd,
           ctx->f_post4.as<float4>(), ctx->f_meta.as<TreeMeta>(), nt, (uint32_t)ctx->cfg.n_classes,
           ctx->magic_tab.as<uint32_t>());
       return PD_OK;
     };
-    PD_TRY(ctx->forest_fast ? launch.template operator()<true>() : launch.template operator()<false>());
+    PD_TRY(fast_form<P>(ctx, W, H) ? launch.template operator()<true>() : launch.template operator()<false>());
     PD_CUDA(cudaGetLastError());
     ctx->launches++;
   }
@@ -479,13 +520,15 @@ extern "C" int pd_predict_leaf(pd_ctx *ctx, uint32_t tree, const void *image, ui
       return rtc_launch(ctx, rk->predict_leaf, grid, dim3(kPredX, kPredY), 0, args);
     }
     if constexpr (!P::kRtcOnly) {
-      auto launch = [&]<bool AF>() {
+      auto launch = [&]<bool AF>() -> int {
+        const Node<P, AF> *nd = nullptr;
+        PD_TRY((form_nodes<P, AF>(ctx, &nd)));
         k_predict_leaf<P, AF><<<grid, dim3(kPredX, kPredY), 0, st>>>(
             ctx->p_img.as<uint8_t>(), width, height, mask ? ctx->p_mask.as<uint8_t>() : nullptr,
-            ctx->p_out.as<int32_t>(), ctx->f_cand.as<Node<P, AF>>() + off, depth, ctx->magic_tab.as<uint32_t>());
+            ctx->p_out.as<int32_t>(), nd + off, depth, ctx->magic_tab.as<uint32_t>());
+        return PD_OK;
       };
-      if (ctx->forest_fast) launch.template operator()<true>();
-      else launch.template operator()<false>();
+      PD_TRY(fast_form<P>(ctx, width, height) ? launch.template operator()<true>() : launch.template operator()<false>());
       PD_CUDA(cudaGetLastError());
     }
     return PD_OK;
