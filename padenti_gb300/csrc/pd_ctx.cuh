@@ -75,8 +75,8 @@ struct pd_ctx {
   pd::DevBuf hist, g32;
   pd::DevBuf items, hist_queue;  // work list, slots to zero, slots to split
   // Results of a slice in one buffer, for one copy back: SplitOut [n], left class
-  // counts [n][K], feature values and threshold [n][D + 1], rechecked candidates
-  // (set_results).
+  // counts [n][K], feature values and threshold [n][D + 1], rechecked candidates and
+  // the report of samples_disagree (set_results).
   pd::DevBuf split_res;
   void *res_out = nullptr, *res_par = nullptr;
   uint32_t *res_cl = nullptr;

@@ -182,13 +182,13 @@ static int set_results(pd_ctx *ctx, uint32_t n) {
   auto up = [](size_t v) { return (v + 15) / 16 * 16; };
   const size_t K = ctx->cfg.n_classes, par = up((size_t)n * (ctx->cfg.feat_dim + 1) * feat_size(ctx->cfg.feat_type));
   const size_t out = up((size_t)n * sizeof(SplitOut)), cl = up((size_t)n * K * 4);
-  PD_TRY(ctx->split_res.ensure(out + cl + par + 16));
+  PD_TRY(ctx->split_res.ensure(out + cl + par + 16));  // 16: SplitArgs::rechecked
   uint8_t *b = ctx->split_res.as<uint8_t>();
   ctx->res_out = b;
   ctx->res_cl = reinterpret_cast<uint32_t *>(b + out);
   ctx->res_par = b + out + cl;
   ctx->res_recheck = reinterpret_cast<unsigned long long *>(b + out + cl + par);
-  ctx->res_bytes = out + cl + par + 8;
+  ctx->res_bytes = out + cl + par + 16;
   return PD_OK;
 }
 
@@ -648,9 +648,10 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
   PD_TRY(ctx->scan_blocks.ensure((S / kScanItems + 4) * 8));
   PD_TRY(ctx->h_chk.ensure(16));
   PD_CUDA(cudaMemsetAsync(ctx->snode.ptr, 0, S * 4, st));
-  // the regrouping of a level is checked at the next level's synchronisation: until
-  // then a position it missed (a feature that is no function of its inputs) reads
-  // sample 0
+  // The regrouping of a level is checked at the next level's synchronisation.  Until
+  // then a position it missed (a feature that is no function of its inputs) holds a
+  // sample all the same: the first of the set, or one of an earlier level.  The
+  // kernels before the check take any samples (samples_disagree).
   PD_CUDA(cudaMemsetAsync(ctx->act[1].ptr, 0, S * 4, st));
   PD_CUDA(cudaMemsetAsync(ctx->act_slot[1].ptr, 0, S * 4, st));
   PD_CUDA(cudaMemsetAsync(ctx->act_rec[1].ptr, 0, S * sizeof(SampleRec), st));
@@ -730,7 +731,7 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
       const int32_t *d_nodes = ctx->d_pre.as<int32_t>();
       const uint32_t *d_ctot = reinterpret_cast<const uint32_t *>(ctx->d_pre.as<uint8_t>() + node_bytes);
       PD_TRY(set_results(ctx, ns));
-      PD_CUDA(cudaMemsetAsync(ctx->res_recheck, 0, sizeof(unsigned long long), st));
+      PD_CUDA(cudaMemsetAsync(ctx->res_recheck, 0, 16, st));
       std::vector<uint64_t> off(cur_off.begin() + s0, cur_off.begin() + s0 + ns + 1);
       PD_CUDA(cudaEventRecord(ev[0], st));
       const uint32_t *d_ord = nullptr;
@@ -774,12 +775,15 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
       FeatT *h_par = &level_par[(size_t)s0 * (D + 1)];
       memcpy(h_cl, host(ctx->res_cl), (size_t)ns * K * 4);
       memcpy(h_par, host(ctx->res_par), (size_t)ns * (D + 1) * sizeof(FeatT));
-      unsigned long long rechecked = 0;
-      memcpy(&rechecked, host(ctx->res_recheck), 8);
+      unsigned long long rechecked[2];
+      memcpy(rechecked, host(ctx->res_recheck), 16);
+      PD_CHECK(rechecked[1] == 0, PD_ERR_STATE,
+               "reassignment disagrees with the split counts: a node of depth %u has other samples than its class totals",
+               depth);
       stats.ms_candidates += elapsed(ev[0], ev[1]);
       stats.ms_hist += elapsed(ev[6], ev[2]);
       stats.ms_split += elapsed(ev[2], ev[3]);
-      stats.split_rechecked += rechecked;
+      stats.split_rechecked += rechecked[0];
 
       if (shard) {
         // the ranks' best splits -> the global ones: largest exact gain, ties to the lowest t * F + f
@@ -880,7 +884,7 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
     for (uint32_t i = 0; i < nf; i++) {
       SlotNext x;
       x.k_l = x.k_r = x.child = -1;
-      x.pad = 0;
+      x.beg = (uint32_t)next_off.back();
       x.adj_l = x.adj_r = 0;
       if (split_now[i]) {
         const uint64_t n = (uint64_t)frontier[i], L = 2 * n + 1, R = 2 * n + 2;
@@ -906,6 +910,8 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
           for (uint32_t l = 0; l < K; l++) next_tot.push_back(nt[l] - cl[l]);
         }
       }
+      x.end = (uint32_t)next_off.back();
+      x.mid = x.k_r >= 0 ? (uint32_t)next_off[x.k_r] : x.end;
       sn[i] = x;
     }
     // the level's splits by slot, in one copy
@@ -948,7 +954,7 @@ static int train_tree_impl(pd_ctx *ctx, const pd_train_params *p, uint32_t tree_
       k_scan_reduce<<<nb, 256, 0, st>>>(ctx->flags.as<uint8_t>(), (uint32_t)n_act, bs);
       k_scan_blocks<<<1, 1024, 0, st>>>(bs, nb, bs + nb);
       k_scatter<<<nb, 256, 0, st>>>(ctx->flags.as<uint8_t>(), (uint32_t)n_act, bs, ctx->act[cur].as<uint32_t>(),
-                                    ctx->act_slot[cur].as<uint32_t>(), d_next, (uint32_t)n_next,
+                                    ctx->act_slot[cur].as<uint32_t>(), d_next,
                                     ctx->act[1 - cur].as<uint32_t>(), ctx->act_slot[1 - cur].as<uint32_t>(),
                                     ctx->act_rec[cur].as<SampleRec>(), ctx->act_rec[1 - cur].as<SampleRec>(),
                                     bs + nb + 1);
@@ -1175,7 +1181,7 @@ extern "C" int pd_split(pd_ctx *ctx, const pd_train_params *params, const uint32
   PD_TRY(dc.ensure((size_t)n_nodes * K * 4 + 4));
   PD_CUDA(h2d(ctx, dh.ptr, hist, (size_t)n_nodes * K * T * F * 4));
   PD_CUDA(h2d(ctx, dc.ptr, class_tot, (size_t)n_nodes * K * 4));
-  PD_CUDA(cudaMemsetAsync(ctx->res_recheck, 0, 8, ctx->stream));
+  PD_CUDA(cudaMemsetAsync(ctx->res_recheck, 0, 16, ctx->stream));
   PD_TRY(launch_split<true>(ctx, params, n_nodes, dh.as<uint32_t>(), nullptr, dc.as<uint32_t>()));
   std::vector<SplitOut> o(n_nodes);
   PD_CUDA(d2h(ctx, o.data(), ctx->res_out, n_nodes * sizeof(SplitOut)));

@@ -421,6 +421,14 @@ struct SplitPart {
   int32_t col;    // column of the candidate table
 };
 
+// A level's samples are regrouped by evaluating the splits again, and the next level's
+// histograms and splits run before the host has read the regrouping's check (one
+// synchronisation a level).  A user feature that is no function of its inputs can
+// leave a node with other samples than its class totals say, so every split kernel
+// compares the counts with the totals before it indexes a table with their difference,
+// and on a mismatch picks nothing and reports it here; the host then fails the call.
+PD_D void samples_disagree(unsigned long long *rechecked) { rechecked[1] = 1ull; }
+
 constexpr int kSplitCols = 128;  // threads of a split CTA, one column each per pass
 // histogram rows loaded together in pass 1 (KM registers each)
 PD_HD constexpr int split_rows(int KM) { return KM <= 4 ? 10 : 4; }
@@ -478,7 +486,7 @@ struct SplitArgs {
   SplitPart *part_best;       // [slots][parts]
   SplitOut *out;
   uint32_t *out_cl;           // [slots][K] left class counts of the winner
-  unsigned long long *rechecked;
+  unsigned long long *rechecked;  // [0] exact evaluations; [1] nonzero: see samples_disagree (not when CUM)
   const uint32_t *slot_list;  // slots to process (null: blockIdx.y)
   const uint32_t *ord;        // [slots][F] original index of each column (null: identity)
 };
@@ -916,7 +924,7 @@ struct FusedSplit {
   unsigned *done;             // [slots]
   SplitOut *out;
   uint32_t *out_cl;           // [slots][K]
-  unsigned long long *rechecked;
+  unsigned long long *rechecked;  // [0] exact evaluations; [1] nonzero: see samples_disagree
   const uint32_t *ord;        // [slots][F] original index of each column (null: identity)
 };
 
@@ -938,12 +946,14 @@ PD_D void fused_split(const FusedSplit &fs, const WorkItem &w, uint32_t *sh_hist
   __shared__ int s_j0;
   __shared__ uint8_t s_cls[PD_MAX_CLASSES];  // the classes present in the node, in class order
   __shared__ uint32_t s_nc;
+  __shared__ bool s_bad;
   const uint32_t slot = w.slot, f0 = w.tile * kTileF;
   const uint32_t TS = T + 1;  // histogram rows per class
   for (uint32_t l = threadIdx.x; l < K; l += blockDim.x) s_tot[l] = fs.class_tot[(size_t)slot * K + l];
   __syncthreads();
   if (threadIdx.x == 0) {
     s_nlist = 0u;
+    s_bad = false;
     s_pmin = ~0ull;
     s_j0 = 0;
     uint32_t nc = 0;
@@ -975,14 +985,18 @@ PD_D void fused_split(const FusedSplit &fs, const WorkItem &w, uint32_t *sh_hist
       run += h[j * 32];
       h[j * 32] = run;
     }
+    // every sample of the class is in one row, the last (no threshold reached) included
+    const uint32_t all = run + h[T * 32], tot = s_tot[s_cls[q >> 5]], f = f0 + (q & 31);
+    if ((f < F && (all & 0xffffu) != tot) || (f + 32 < F && (all >> 16) != tot)) s_bad = true;
   }
   __syncthreads();
+  if (s_bad && threadIdx.x == 0) samples_disagree(fs.rechecked);
   uint32_t N = 0, classes = 0;
   for (uint32_t l = 0; l < K; l++) {
     N += s_tot[l];
     classes += s_tot[l] != 0u;
   }
-  const bool ok = N != 0 && (uint64_t)N < fs.L_len;
+  const bool ok = N != 0 && (uint64_t)N < fs.L_len && !s_bad;
   double best = -DBL_MAX;
   long long best_idx = LLONG_MAX;
   int best_j = -1, best_c = -1;
@@ -1422,7 +1436,7 @@ __global__ void __launch_bounds__(small_threads(NC), small_ctas(NC))
   constexpr uint32_t kParts = kSmallThreads / kTileF;  // threads per candidate column
   constexpr bool kPrefix = kParts > 2;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ uint32_t s_tot[NC];
+  __shared__ uint32_t s_tot[NC], s_seen[NC + 1];  // samples of each class present: by the totals, in the item
   __shared__ uint8_t s_map[PD_MAX_CLASSES], s_cls[NC];
   __shared__ uint32_t s_nc;
   __shared__ float s_max[kSmallThreads / 32];
@@ -1443,15 +1457,18 @@ __global__ void __launch_bounds__(small_threads(NC), small_ctas(NC))
       const uint32_t l = l0 + lane, tot = l < K ? fs.class_tot[(size_t)slot * K + l] : 0u;
       const uint32_t m = __ballot_sync(0xffffffffu, tot != 0u);
       const uint32_t i = nc + __popc(m & ((1u << lane) - 1u));
-      if (tot != 0u && i < NC) {
-        s_map[l] = (uint8_t)i;
+      const bool in = tot != 0u && i < NC;
+      if (l < K) s_map[l] = (uint8_t)(in ? i : NC);
+      if (in) {
         s_cls[i] = (uint8_t)l;
         s_tot[i] = tot;
       }
       nc += __popc(m);
     }
     if (lane >= nc && lane < NC) s_tot[lane] = 0u;
+    if (lane < NC) s_seen[lane] = 0u;
     if (lane == 0) {
+      s_seen[NC] = 0u;
       s_nc = nc;
       s_key = 0ull;
       s_idx = ~0ull;
@@ -1462,15 +1479,22 @@ __global__ void __launch_bounds__(small_threads(NC), small_ctas(NC))
   prefetch_fused(fs, w, f0, F, T);
   build_rank_tab<kSmallThreads>(rt, cand_thr + (size_t)slot * T * F, F, T, f0);
   hist_samples_tile<P, kSmallSpi, kSmallThreads>(ds, rec, w, cand_feat + (size_t)slot * P::kFeatDim * F, F, f0, sh_hist, rt, T,
-                                         [&](uint32_t l) { return (uint32_t)s_map[l]; });
+                                         [&](uint32_t l) {
+                                           const uint32_t i = s_map[l];
+                                           atomicAdd(&s_seen[i], 1u);
+                                           return i < NC ? i : 0u;  // NC: a class the totals lack
+                                         });
   __syncthreads();
+  // no class has more samples than its total (both sum to N: each has as many)
+  const bool agree = !__syncthreads_or(threadIdx.x < NC && s_seen[threadIdx.x] != s_tot[threadIdx.x]);
+  if (!agree && threadIdx.x == 0) samples_disagree(fs.rechecked);
 
   const uint32_t nc = s_nc, N = w.end - w.begin;
   const uint32_t c = threadIdx.x & (kTileF - 1), part = threadIdx.x / kTileF;
   const uint32_t *fw = rt.first + c * rt.first_words;
   uint32_t D = 0;  // distinct thresholds of the column (0 past the last column)
   for (uint32_t k = 0; k < rt.first_words; k++) D += __popc(fw[k]);
-  const bool ok = (uint64_t)N < fs.L_len;
+  const bool ok = agree && (uint64_t)N < fs.L_len;
   if constexpr (kPrefix) {
     // cumulative counts in place, a thread per (class, packed column)
     for (uint32_t q = threadIdx.x; q < nc * 32; q += kSmallThreads) {
@@ -1802,6 +1826,7 @@ __global__ void __launch_bounds__(kSplitCols) k_split_g32(SplitArgs a) {
   float *G = a.g32 + (size_t)slot * T * F;
   const uint32_t fb = part * a.cols, fe = min(F, fb + a.cols);
   float lmax = -FLT_MAX;
+  bool over = false;
   for (uint32_t f = fb + threadIdx.x; f < fe; f += blockDim.x) {
     uint32_t c[KM];
 #pragma unroll
@@ -1845,7 +1870,12 @@ __global__ void __launch_bounds__(kSplitCols) k_split_g32(SplitArgs a) {
         lmax = fmaxf(lmax, g);
       }
     }
+    if constexpr (!CUM) {  // counts grow with j: none is above its total at any j
+#pragma unroll
+      for (int l = 0; l < KM; l++) over |= c[l] > tot[l];
+    }
   }
+  if (over) samples_disagree(a.rechecked);
   for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = lmax;
   __syncthreads();
@@ -1933,7 +1963,8 @@ __global__ void __launch_bounds__(kSplitCols) k_split_pick(SplitArgs a) {
   if (threadIdx.x == 0) s_n = 0u;
   uint32_t N;
   load_tot<KM>(a, slot, tot, N);
-  if (N == 0 || (uint64_t)N >= a.L_len) {
+  const bool disagree = !CUM && __ldcg(a.rechecked + 1) != 0ull;
+  if (N == 0 || (uint64_t)N >= a.L_len || disagree) {
     if (part == 0 && threadIdx.x == 0) {
       SplitOut o;
       o.t = o.f = o.j = o.col = -1;
@@ -2128,7 +2159,8 @@ __global__ void __launch_bounds__(kSplitCols) k_split_pick(SplitArgs a) {
 struct SlotNext {
   long long adj_l, adj_r;  // next position base (next offset of child - samples of earlier parents)
   int32_t k_l, k_r;        // next frontier slot of each child or -1
-  int32_t child, pad;      // left child of the slot's node, -1 when it was not split
+  int32_t child;           // left child of the slot's node, -1 when it was not split
+  uint32_t beg, mid, end;  // next positions of its left child [beg, mid) and right child [mid, end)
 };
 
 // par: feature values and threshold of each slot's split [slot][D + 1].  Everything is
@@ -2218,12 +2250,14 @@ static __global__ void __launch_bounds__(1024) k_scan_blocks(unsigned long long 
 // Stable regrouping: sample i of parent slot p goes to
 // adj[p] + (number of earlier samples with the same flag).  Because parents are
 // in slot order and their children in the same order, this keeps every child's
-// samples in their previous (image-major) order.
+// samples in their previous (image-major) order.  A sample past its child's range (the
+// child got other samples than the split counted) is not placed but counted in *err:
+// with none, every child has exactly its samples.
 static __global__ void __launch_bounds__(256) k_scatter(const uint8_t *__restrict__ flags, uint32_t n,
                                                  const unsigned long long *__restrict__ bsum,
                                                  const uint32_t *__restrict__ act,
                                                  const uint32_t *__restrict__ act_slot,
-                                                 const SlotNext *__restrict__ nxt, uint32_t n_next,
+                                                 const SlotNext *__restrict__ nxt,
                                                  uint32_t *__restrict__ act_out,
                                                  uint32_t *__restrict__ slot_out,
                                                  const SampleRec *__restrict__ rec,
@@ -2257,6 +2291,7 @@ static __global__ void __launch_bounds__(256) k_scatter(const uint8_t *__restric
     const SlotNext sn = nxt[act_slot[i]];
     long long pos;
     uint32_t kslot;
+    const uint32_t lo = fl[k] == 1 ? sn.beg : sn.mid, hi = fl[k] == 1 ? sn.mid : sn.end;
     if (fl[k] == 1) {
       pos = sn.adj_l + (long long)(run & 0xffffffffull);
       kslot = (uint32_t)sn.k_l;
@@ -2266,7 +2301,7 @@ static __global__ void __launch_bounds__(256) k_scatter(const uint8_t *__restric
       kslot = (uint32_t)sn.k_r;
       run += 1ull << 32;
     }
-    if (pos < 0 || pos >= (long long)n_next) {
+    if (pos < (long long)lo || pos >= (long long)hi) {
       atomicAdd(err, 1ull);
       continue;
     }
