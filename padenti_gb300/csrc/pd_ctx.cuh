@@ -141,6 +141,26 @@ struct pd_ctx {
 };
 
 namespace pd {
+// Lets launches of a kernel take `smem` bytes of dynamic shared memory.  The limit is a
+// property of the function, shared by every context of the process, and calls of
+// several contexts may run at once: it is raised to the device's maximum and never to a
+// launch's own size, which another thread's smaller launch would take away between the
+// call and the launch.  It is a permission: occupancy follows from what a launch asks
+// for.  Every kernel may take 32 KB (48 less its static arrays) without.
+template <typename Kernel>
+int allow_smem(const pd_ctx *c, Kernel *kernel, size_t smem) {
+  if (smem <= 32768) return PD_OK;
+  const void *fn = reinterpret_cast<const void *>(kernel);
+  cudaFuncAttributes fa;
+  PD_CUDA(cudaFuncGetAttributes(&fa, fn));
+  int most = 0;
+  PD_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+  most -= (int)fa.sharedSizeBytes;
+  PD_CHECK(smem <= (size_t)most, PD_ERR_CUDA, "a kernel needs %zu bytes of shared memory; the GPU offers %d", smem, most);
+  if (fa.maxDynamicSharedSizeBytes < most)
+    PD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  return PD_OK;
+}
 // Counted copies on the context stream.
 inline cudaError_t h2d(pd_ctx *c, void *dst, const void *src, size_t n) {
   c->bytes_h2d += n;

@@ -11,7 +11,7 @@ template <class P, uint32_t TP, int SPI>
 static int launch_hist_grid_as(pd_ctx *ctx, const HistGrid &g) {
   using FeatT = typename P::feat_t;
   auto kern = k_hist<P, TP, SPI>;
-  PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+  PD_TRY(allow_smem(ctx, kern, g.smem));
   // carve out only the shared memory the resident CTAs need; the rest stays L1
   // for the probe gathers (resident CTAs are register-limited; search form: 3 at 2
   // samples per iteration, 2 at 4 or 8)
@@ -45,7 +45,7 @@ static int launch_small_as(pd_ctx *ctx, const HistGrid &g, const WorkItem *items
                            cudaStream_t st) {
   using FeatT = typename P::feat_t;
   auto kern = k_hist_small<P, NC>;
-  PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PD_TRY(allow_smem(ctx, kern, smem));
   PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, small_carveout(NC, smem)));
   const uint64_t most = 0x7fffffffull / g.tiles;
   for (uint64_t b = 0; b < n; b += most) {

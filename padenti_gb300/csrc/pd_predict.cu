@@ -175,7 +175,7 @@ static int launch_posterior(pd_ctx *ctx, uint32_t n, const void *images, uint32_
       auto kern = k_predict_posterior<P, AF>;
       const Node<P, AF> *nd = nullptr;
       PD_TRY((form_nodes<P, AF>(ctx, &nd)));
-      PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      PD_TRY(allow_smem(ctx, kern, smem));
       kern<<<grid, dim3(kPredX, kPredY), smem, ctx->stream>>>(
           static_cast<const uint8_t *>(images), img_bytes, W, H, masks, out, nd,
           ctx->f_post4.as<float4>(), ctx->f_meta.as<TreeMeta>(), nt, (uint32_t)ctx->cfg.n_classes,
@@ -448,7 +448,7 @@ extern "C" int pd_predict_posterior_batch(pd_ctx *ctx, uint32_t n, const void *c
         fn = (const void *)rk->predict_batch;
       } else if constexpr (!P::kRtcOnly) {
         fn = ctx->forest_fast ? (const void *)k_predict_batch<P, true> : (const void *)k_predict_batch<P, false>;
-        PD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PD_TRY(allow_smem(ctx, fn, smem));
       }
       cudaGraph_t g = nullptr;
       PD_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));

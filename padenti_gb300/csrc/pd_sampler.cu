@@ -961,7 +961,7 @@ int launch_class_weighted(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &p
   const bool bitmap = most <= kBitmapPixels;
   const size_t smem = bitmap ? ((size_t)most + 127) / 128 * 16 : (size_t)pl.sort_n * 4;
   auto bucket_samples = bitmap ? k_bucket_samples<true> : k_bucket_samples<false>;
-  PD_CUDA(cudaFuncSetAttribute(bucket_samples, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PD_TRY(allow_smem(ctx, bucket_samples, smem));
   bucket_samples<<<n, kSmThreads, smem, st>>>(imgs, bsz, tot, K, slots, pl.stride, pl.sort_n, out, counts);
   PD_CUDA(cudaGetLastError());
   *launched += 1;
@@ -995,7 +995,7 @@ int launch_batch(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32
   if (s->kind == PD_SAMPLER_UNIFORM) {
     const uint32_t buckets = std::max(pl.sort_n, kSmThreads);
     const size_t smem = ((size_t)s->n_samples * 2 + buckets) * 4;
-    PD_CUDA(cudaFuncSetAttribute(k_sample_uniform, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PD_TRY(allow_smem(ctx, k_sample_uniform, smem));
     k_sample_uniform<<<n, kSmThreads, smem, st>>>(labels, imgs, crc, cnt, s->n_samples, s->seed, buckets, out, counts,
                                                   err);
   } else {

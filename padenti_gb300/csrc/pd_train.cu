@@ -242,7 +242,7 @@ static int launch_candidates(pd_ctx *ctx, const pd_train_params *p, uint32_t tre
       void *args[] = {&d_nodes, &tr, &f_, &bb, &o, &ps};
       PD_TRY(rtc_launch(ctx, rk->cand_order, dim3(n), dim3(kOrderThreads), osmem, args));
     } else if constexpr (!P::kRtcOnly) {
-      PD_CUDA(cudaFuncSetAttribute(k_cand_order<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)osmem));
+      PD_TRY(allow_smem(ctx, k_cand_order<P>, osmem));
       k_cand_order<P><<<n, kOrderThreads, osmem, ctx->stream>>>(d_nodes, tree, F, b, ctx->cand_ord.as<uint32_t>(),
                                                                 prop ? *prop : PropSrc{});
       PD_CUDA(cudaGetLastError());
@@ -269,7 +269,7 @@ static int launch_candidates(pd_ctx *ctx, const pd_train_params *p, uint32_t tre
   }
   const size_t smem = (size_t)p->n_thresholds * kCandThreads * (packed ? 4 : sizeof(FeatT) + 1);
   auto kern = packed ? k_candidates<FeatT, true> : k_candidates<FeatT, false>;
-  PD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PD_TRY(allow_smem(ctx, kern, smem));
   kern<<<grid, kCandThreads, smem, ctx->stream>>>(
       d_nodes, n, tree, F, p->n_thresholds, P::kFeatDim, b, ord, ctx->cand_feat.as<FeatT>(),
       ctx->cand_thr.as<FeatT>(), ctx->cand_perm.as<uint8_t>(), prop ? *prop : PropSrc{});
