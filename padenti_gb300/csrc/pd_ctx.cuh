@@ -103,12 +103,11 @@ struct pd_ctx {
   bool forest_dirty = true;
   pd::DevBuf f_lc, f_feat, f_thr, f_post, f_meta;
   pd::DevBuf f_cand;                   // FastNode or NodeRec of every forest node
-  pd::DevBuf f_post4;                  // posteriors padded to four classes a word (k_pad_posteriors)
+  pd::DevBuf f_post4;                  // posterior rows padded to four classes a word, where K % 4 (k_pad_posteriors)
   pd::DevBuf f_gen;                    // NodeRec beside FastNode, for images past the fast form's sides
   uint64_t cand_version = ~0ull;       // forest_version f_cand was built for
   uint64_t gen_version = ~0ull;        // forest_version f_gen was built for
   bool forest_fast = false;            // every node takes the plugin's fast path (built-in plugins)
-  pd::DevBuf f_fast;                   // its device flag
   pd::DevBuf p_img, p_mask, p_out;     // staging for host-buffer prediction
   uint64_t forest_version = 0;         // bumped when the forest arrays are uploaded again
   // mixed-size prediction batches: buffers, the layout they were built for and

@@ -32,7 +32,7 @@ static int upload_forest(pd_ctx *ctx) {
   PD_TRY(ctx->f_feat.ensure(ctx->h_feat.size() + 4));
   PD_TRY(ctx->f_thr.ensure(ctx->h_thr.size() + 4));
   PD_TRY(ctx->f_post.ensure(ctx->h_post.size() * 4 + 4));
-  PD_TRY(ctx->f_meta.ensure(nt * sizeof(TreeMeta) + 16));
+  PD_TRY(ctx->f_meta.ensure(nt * sizeof(TreeMeta) + 16));  // 16: the flag of k_forest_fast
   if (nodes) {
     PD_CUDA(h2d(ctx, ctx->f_lc.ptr, ctx->h_lc.data(), nodes * 4));
     PD_CUDA(h2d(ctx, ctx->f_feat.ptr, ctx->h_feat.data(), ctx->h_feat.size()));
@@ -73,12 +73,14 @@ static int ensure_forest_nodes(pd_ctx *ctx) {
   const FeatT *ft = ctx->f_feat.as<FeatT>(), *th = ctx->f_thr.as<FeatT>();
   const int32_t *lc = ctx->f_lc.as<int32_t>();
   const dim3 grid((unsigned)((nodes + 255) / 256 + (nodes == 0)));
-  const uint32_t K = (uint32_t)ctx->cfg.n_classes, KP = (K + 3) / 4 * 4;
-  PD_TRY(ctx->f_post4.ensure(nodes * KP * 4 + 16));
-  k_pad_posteriors<<<(unsigned)((nodes * KP + 255) / 256 + (nodes == 0)), 256, 0, ctx->stream>>>(
-      ctx->f_post.as<float>(), nodes, K, ctx->f_post4.as<float>());
-  PD_CUDA(cudaGetLastError());
-  ctx->launches++;
+  const uint32_t K = (uint32_t)ctx->cfg.n_classes, K4 = (K + 3) / 4;
+  if (K % 4) {
+    PD_TRY(ctx->f_post4.ensure(nodes * K4 * 16 + 16));
+    k_pad_posteriors<<<(unsigned)((nodes * K4 + 255) / 256 + (nodes == 0)), 256, 0, ctx->stream>>>(
+        ctx->f_post.as<float>(), nodes, K, ctx->f_post4.as<float4>());
+    PD_CUDA(cudaGetLastError());
+    ctx->launches++;
+  }
   if (is_user_plugin(ctx)) {
     const RtcKernels *rk = nullptr;
     PD_TRY(rtc_kernels(ctx, &rk));
@@ -88,15 +90,14 @@ static int ensure_forest_nodes(pd_ctx *ctx) {
   } else if constexpr (!P::kRtcOnly) {
     // the fast form's records, and whether every node takes it; else the general ones
     static_assert(sizeof(FastNode<P>) <= sizeof(NodeRec<P>), "both forms fit f_cand");
-    PD_TRY(ctx->f_fast.ensure(16));
-    int all = 1;
-    PD_CUDA(h2d(ctx, ctx->f_fast.ptr, &all, 4));
-    k_forest_fast<P><<<grid, 256, 0, ctx->stream>>>(ft, th, lc, nodes, ctx->f_cand.as<FastNode<P>>(),
-                                                    ctx->f_fast.as<int>());
+    int slow = 0;
+    int *any_slow = reinterpret_cast<int *>(ctx->f_meta.as<TreeMeta>() + ctx->tree_depth.size());
+    PD_CUDA(cudaMemsetAsync(any_slow, 0, 4, ctx->stream));
+    k_forest_fast<P><<<grid, 256, 0, ctx->stream>>>(ft, th, lc, nodes, ctx->f_cand.as<FastNode<P>>(), any_slow);
     PD_CUDA(cudaGetLastError());
-    PD_CUDA(d2h(ctx, &all, ctx->f_fast.ptr, 4));
+    PD_CUDA(d2h(ctx, &slow, any_slow, 4));
     PD_CUDA(cudaStreamSynchronize(ctx->stream));
-    ctx->forest_fast = all != 0;
+    ctx->forest_fast = slow == 0;
     ctx->launches++;
     if (!ctx->forest_fast) {
       k_forest_nodes<P><<<grid, 256, 0, ctx->stream>>>(ft, th, lc, nodes, ctx->f_cand.as<NodeRec<P>>());
@@ -106,6 +107,12 @@ static int ensure_forest_nodes(pd_ctx *ctx) {
   }
   ctx->cand_version = ctx->forest_version;
   return PD_OK;
+}
+
+// Posterior rows of whole float4 words: as uploaded where the class count is a multiple
+// of four, else padded (k_pad_posteriors).
+static const float4 *posterior_rows(const pd_ctx *ctx) {
+  return ctx->cfg.n_classes % 4 ? ctx->f_post4.as<float4>() : ctx->f_post.as<float4>();
 }
 
 // Whether a W x H image is walked in the plugin's fast form: the whole forest takes it,
@@ -164,7 +171,7 @@ static int launch_posterior(pd_ctx *ctx, uint32_t n, const void *images, uint32_
     uint64_t ib = img_bytes;
     uint32_t w_ = W, h_ = H, nt_ = nt, k_ = (uint32_t)ctx->cfg.n_classes;
     const void *nd = ctx->f_cand.ptr;
-    const float *po = ctx->f_post4.as<float>();
+    const float4 *po = posterior_rows(ctx);
     const TreeMeta *me = ctx->f_meta.as<TreeMeta>();
     const uint32_t *mg = ctx->magic_tab.as<uint32_t>();
     void *args[] = {&im, &ib, &w_, &h_, &masks, &out, &nd, &po, &me, &nt_, &k_, &mg};
@@ -178,7 +185,7 @@ static int launch_posterior(pd_ctx *ctx, uint32_t n, const void *images, uint32_
       PD_TRY(allow_smem(ctx, kern, smem));
       kern<<<grid, dim3(kPredX, kPredY), smem, ctx->stream>>>(
           static_cast<const uint8_t *>(images), img_bytes, W, H, masks, out, nd,
-          ctx->f_post4.as<float4>(), ctx->f_meta.as<TreeMeta>(), nt, (uint32_t)ctx->cfg.n_classes,
+          posterior_rows(ctx), ctx->f_meta.as<TreeMeta>(), nt, (uint32_t)ctx->cfg.n_classes,
           ctx->magic_tab.as<uint32_t>());
       return PD_OK;
     };
@@ -436,7 +443,7 @@ extern "C" int pd_predict_posterior_batch(pd_ctx *ctx, uint32_t n, const void *c
       const BatchImage *bd = ctx->b_desc.as<BatchImage>();
       uint32_t n_ = n, nt_ = nt, k_ = K;
       const void *nd = ctx->f_cand.ptr;
-      const float *po = ctx->f_post4.as<float>();
+      const float4 *po = posterior_rows(ctx);
       const TreeMeta *me = ctx->f_meta.as<TreeMeta>();
       const uint32_t *mg = ctx->magic_tab.as<uint32_t>();
       void *args[] = {&im, &mk, &o, &bd, &n_, &nd, &po, &me, &nt_, &k_, &mg};

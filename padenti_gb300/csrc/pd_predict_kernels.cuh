@@ -109,12 +109,12 @@ __global__ void k_forest_nodes(const typename P::feat_t *__restrict__ feat, cons
   }
 }
 
-// The FastNode of every forest node; clears *all_fast when a node needs the
+// The FastNode of every forest node; sets *any_slow when a node needs the
 // plugin's slow path (the NodeRec form is built then).
 template <class P>
 __global__ void k_forest_fast(const typename P::feat_t *__restrict__ feat, const typename P::feat_t *__restrict__ thr,
                               const int32_t *__restrict__ lc, unsigned long long n_nodes, FastNode<P> *__restrict__ out,
-                              int *__restrict__ all_fast) {
+                              int *__restrict__ any_slow) {
   const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   if (i >= n_nodes) return;
   const typename P::feat_t *f = feat + i * P::kFeatDim;
@@ -123,7 +123,7 @@ __global__ void k_forest_fast(const typename P::feat_t *__restrict__ feat, const
   n.thr = (int32_t)thr[i];
   n.lc = lc[i];
   out[i] = n;
-  if (!P::fast(P::candidate(f))) *all_fast = 0;
+  if (!P::fast(P::candidate(f))) *any_slow = 1;
 }
 
 // What bounds it (60 640x480 maps, 3 trees of depth 16, 9 classes): the L1 data pipe
@@ -170,14 +170,17 @@ PD_D void predict_pixel(const ImageRef<typename P::img_t> &im, uint32_t x, uint3
   }
 }
 
-// post [n][K] -> out [n][4 ceil(K / 4)], padded with zeros.
+// post [n][K] -> out [n][ceil(K / 4)], padded with zeros: a thread per word of four
+// classes.  Runs once per forest, where K is no multiple of four.
 static __global__ void k_pad_posteriors(const float *__restrict__ post, unsigned long long n, uint32_t K,
-                                        float *__restrict__ out) {
-  const uint32_t KP = (K + 3) / 4 * 4;
+                                        float4 *__restrict__ out) {
+  const uint32_t K4 = (K + 3) / 4;
   const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-  if (i >= n * KP) return;
-  const uint32_t l = (uint32_t)(i % KP);
-  out[i] = l < K ? post[i / KP * K + l] : 0.0f;
+  if (i >= n * K4) return;
+  const unsigned long long node = i >> 32 ? i / K4 : (uint32_t)i / K4;
+  const uint32_t l = 4 * (uint32_t)(i - node * K4);
+  const float *p = post + node * K + l;
+  out[i] = make_float4(p[0], l + 1 < K ? p[1] : 0.0f, l + 2 < K ? p[2] : 0.0f, l + 3 < K ? p[3] : 0.0f);
 }
 
 // grid (ceil(W/32), ceil(H/8), n_images); dynamic smem n_trees*256 int32.
