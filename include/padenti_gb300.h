@@ -428,7 +428,11 @@ int pd_sampler_stride(const pd_sampler *s, uint32_t *stride);
  * sample() returns; 0 for a uniform sampler on an image without labelled
  * pixels, where the reference draws from an empty buffer).  A label above
  * nClasses is an error for the class-weighted sampler (the reference indexes
- * past its buckets). */
+ * past its buckets).  The class-weighted sampler works in device memory that the
+ * context keeps until it is destroyed: 4 bytes per pixel of up to 1 GiB's worth of
+ * images at a time (fewer at a time where less is free, one at least; what a
+ * larger image takes is given back), 4 (nClasses + 1) bytes per 512 pixels and 4
+ * stride bytes per image of the batch. */
 int pd_sample(pd_ctx *ctx, const pd_sampler *s, uint32_t n_images, const void *const *images,
               const uint8_t *const *labels, const uint32_t *widths, const uint32_t *heights,
               uint32_t stride, uint32_t *samples, uint32_t *counts);

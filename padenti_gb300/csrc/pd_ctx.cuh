@@ -120,7 +120,7 @@ struct pd_ctx {
   pd::DevBuf sm_data, sm_lab;    // staged image data and labels of a host batch
   pd::DevBuf sm_desc;            // SampImage per image, item -> image map, checksums, counts, error
   pd::DevBuf sm_out;             // samples and counts of a host batch
-  pd::DevBuf sm_counts, sm_draws, sm_slots;  // class-weighted: segment counts, MT19937 outputs, buckets
+  pd::DevBuf sm_counts, sm_draws, sm_slots;  // class-weighted: segment counts, MT19937 outputs (reserve_draws), buckets
   pd::HostBuf h_sm, h_sm_desc;   // pinned staging of a host batch and of its descriptors
   // pd_sample's two pipeline slots: a group is staged into one while the device
   // works on the other's (pinned data, descriptors, results; device copies; events

@@ -924,11 +924,8 @@ int launch_class_weighted(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &p
   const SampImage *h = reinterpret_cast<const SampImage *>(host_desc + lay.imgs);
   auto segs_of = [&](uint32_t i) { return (h[i].n_pix + kSeg - 1) / kSeg; };
   const uint32_t segs = h[n - 1].seg0 + segs_of(n - 1);
-  uint64_t draw_words = 0;
-  for (uint32_t i = 0; i < n; i++) draw_words = std::max(draw_words, h[i].draw_off + ((uint64_t)h[i].n_pix + 3) / 4 * 4);
   const size_t slot_bytes = (size_t)n * std::max(1u, pl.stride) * 4;
   PD_TRY(ctx->sm_counts.ensure(((size_t)segs * (K + 1) + (size_t)n * (K + 1)) * 4));
-  PD_TRY(ctx->sm_draws.ensure(draw_words * 4));
   PD_TRY(ctx->sm_slots.ensure(slot_bytes));
   uint32_t *c = ctx->sm_counts.as<uint32_t>(), *draw0 = c + (size_t)segs * K, *tot = draw0 + segs,
            *n_draws = tot + (size_t)n * K, *draws = ctx->sm_draws.as<uint32_t>(), *slots = ctx->sm_slots.as<uint32_t>();
@@ -1009,19 +1006,44 @@ int launch_batch(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32
   return PD_OK;
 }
 
-// Fills the pinned descriptor block for images described by (data_lo, data
-// bytes, lab_off, n_pix, out_off) and returns the item count.
-// Words of MT19937 outputs kept at a time by the class-weighted sampler (images are
-// taken in groups of at most that many pixels, one image at least).
-constexpr uint64_t kDrawGroup = 1ull << 29;
-
 struct ImagePlace {
   uint64_t data_lo, data_end, lab_off, out_off;
   uint64_t data_bytes;
   uint32_t n_pix;
 };
 
-int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> &place, DescLayout *lay_out) {
+// Draws of an image in the class-weighted sampler's buffer: a word a pixel.
+uint64_t draw_words(const ImagePlace &p) { return ((uint64_t)p.n_pix + 3) / 4 * 4; }
+
+// The class-weighted sampler's buffer of MT19937 outputs, for a group of images at a
+// time (one at least): the draws of the whole batch, at most twice the bytes that a
+// host batch stages at once (sample_group: 1 GiB of draws, 873 maps of 640x480).  A
+// group should fill the GPU, as its draws are a serial chain: the drawing phase of 500
+// maps in one group takes 0.72 ms, in two 0.80, in four 1.02, in eight 1.52.  Where
+// that much memory is not free, smaller groups.
+int reserve_draws(pd_ctx *ctx, const std::vector<ImagePlace> &place, uint64_t *group) {
+  uint64_t all = 0, one = 0;
+  for (const ImagePlace &p : place) {
+    all += draw_words(p);
+    one = std::max(one, draw_words(p));
+  }
+  for (uint64_t words = std::max(one, std::min(all, ctx->sample_group / 2));; words = std::max(one, words / 2)) {
+    const int rc = ctx->sm_draws.ensure(words * 4);
+    *group = words;
+    if (rc != PD_ERR_NOMEM || words == one) return rc;
+  }
+}
+
+// Gives back what a single larger image took of it.
+void trim_draws(pd_ctx *ctx) {
+  if (ctx->sm_draws.cap > 2 * ctx->sample_group) ctx->sm_draws.release();
+}
+
+// Fills the pinned descriptor block for images described by (data_lo, data
+// bytes, lab_off, n_pix, out_off); draw_group: words of draws kept at a time
+// (class-weighted).
+int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> &place, uint64_t draw_group,
+              DescLayout *lay_out) {
   const uint32_t n = (uint32_t)place.size();
   uint64_t n_crc = 0, n_lab = 0;
   std::vector<uint32_t> slices(n), chunks(n);
@@ -1044,9 +1066,8 @@ int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> 
   uint64_t segs = 0, draws = 0;
   for (uint32_t i = 0; i < n; i++) {
     const ImagePlace &p = place[i];
-    // draws are kept for kDrawGroup words of images at a time (one image at least)
-    const uint64_t dw = ((uint64_t)p.n_pix + 3) / 4 * 4;
-    if (draws && draws + dw > kDrawGroup) draws = 0;
+    const uint64_t dw = draw_words(p);
+    if (draws && draws + dw > draw_group) draws = 0;
     im[i] = SampImage{p.data_lo, p.data_end, p.lab_off, p.out_off, p.n_pix, (p.n_pix + 15) / 16, slices[i], ic, il,
                       (uint32_t)segs, draws};
     segs += (p.n_pix + kSeg - 1) / kSeg;
@@ -1219,7 +1240,12 @@ extern "C" int pd_sample(pd_ctx *ctx, const pd_sampler *s, uint32_t n_images, co
       for (auto &x : th) x.join();
     }
     DescLayout &lay = lays[si];
-    PD_TRY(fill_desc(sl.h_desc, pl, g.place, &lay));
+    uint64_t draw_group = 0;
+    if (s->kind == PD_SAMPLER_CLASS_WEIGHTED) {
+      const int rc = reserve_draws(ctx, g.place, &draw_group);
+      if (rc != PD_OK) return fail(rc);
+    }
+    PD_TRY(fill_desc(sl.h_desc, pl, g.place, draw_group, &lay));
     PD_TRY(sl.d_data.ensure(g.data_cur + g.lab_cur + 16));
     PD_TRY(sl.d_desc.ensure(lay.bytes));
     const uint64_t out_words = (uint64_t)n * stride + n;
@@ -1246,6 +1272,7 @@ extern "C" int pd_sample(pd_ctx *ctx, const pd_sampler *s, uint32_t n_images, co
       if (rc != PD_OK) return fail(rc);
     }
   }
+  trim_draws(ctx);
   ctx->sample_stats.images = n_images;
   ctx->sample_stats.h2d_bytes = ctx->bytes_h2d - h2d0;
   ctx->sample_stats.d2h_bytes = ctx->bytes_d2h - d2h0;
@@ -1278,13 +1305,16 @@ extern "C" int pd_sample_device(pd_ctx *ctx, const pd_sampler *s, uint32_t n_ima
   for (uint32_t i = 0; i < n_images; i++)
     place[i] = ImagePlace{i * db, (i + 1) * db, i * np, (uint64_t)i * stride, db, (uint32_t)np};
   DescLayout lay;
-  PD_TRY(fill_desc(ctx->h_sm_desc, pl, place, &lay));
+  uint64_t draw_group = 0;
+  if (s->kind == PD_SAMPLER_CLASS_WEIGHTED) PD_TRY(reserve_draws(ctx, place, &draw_group));
+  PD_TRY(fill_desc(ctx->h_sm_desc, pl, place, draw_group, &lay));
   PD_TRY(ctx->sm_desc.ensure(lay.bytes));
   PD_TRY(launch_batch(ctx, s, pl, n_images, static_cast<const uint8_t *>(images_device), labels_device,
                       samples_device, counts_device, lay, ctx->sm_desc.as<uint8_t>(), ctx->h_sm_desc.ptr, ctx->ev));
   uint32_t err[2];
   PD_CUDA(d2h(ctx, err, ctx->sm_desc.as<uint8_t>() + lay.err, 8));
   PD_CUDA(cudaStreamSynchronize(ctx->stream));
+  trim_draws(ctx);
   PD_TRY(check_errors(err, 0, s));
   ctx->sample_stats.images = n_images;
   ctx->sample_stats.data_bytes = db * n_images;
