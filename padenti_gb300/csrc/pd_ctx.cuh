@@ -177,6 +177,8 @@ struct PropSrc;
 // totals d_ctot [n][K] on the device), on the context's stream (pd_propose.cu).
 int proposer_infer(pd_proposer *p, const uint32_t *d_ctot, uint32_t n, uint32_t depth, uint32_t n_prop, PropSrc *src);
 int ensure_log2_table(pd_ctx *ctx, uint64_t n);
+// Whether the histogram kernels of a training call take the rank-table form (pd_train.cu).
+bool rank_form(const pd_ctx *ctx, const pd_train_params *p, const PropSrc *prop = nullptr);
 // Host -> device copy of bulk inputs on the context's stream (pd_api.cu).
 int upload_bytes(pd_ctx *ctx, void *dst, const void *src, size_t n);
 int init_tables(pd_ctx *ctx);

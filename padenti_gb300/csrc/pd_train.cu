@@ -48,7 +48,7 @@ constexpr size_t kRankSmemMax = 227 * 1024 - 4096;  // dynamic; the kernels' sta
 // kRankWordsMax words a column, and a CTA's histogram of all classes fits the
 // shared memory beside it (the search form takes what is left, such as 64 classes
 // with many thresholds).
-static bool rank_form(const pd_ctx *ctx, const pd_train_params *p, const PropSrc *prop) {
+bool rank_form(const pd_ctx *ctx, const pd_train_params *p, const PropSrc *prop) {
   if (prop) {  // proposals are clamped to the network's bounds: they must be these
     const int D = ctx->cfg.feat_dim;
     if (prop->lo[D] != (float)p->thr_low || prop->span[D] != (float)((int64_t)p->thr_up - p->thr_low) ||

@@ -4,7 +4,8 @@
 // knobs of pd_ctx_set_tuning -- samples per work item, samples per warp
 // iteration, the largest node whose split is fused into the histogram kernel,
 // the candidate column order and the persistent launch -- are searched per
-// (GPU, configuration, candidate counts, training-set size, depth) by timing
+// (GPU, configuration, candidate counts, form of the histogram kernels, training-set
+// size, depth) by timing
 // whole trees on the uploaded training set, and the winner is cached in a text
 // file.  No knob changes a result, and every trial's tree is checked against
 // the first one.
@@ -39,6 +40,11 @@ static void apply(pd_ctx *c, const Knobs &k) {
 
 static int floor_log2(uint64_t v) { return v ? 63 - __builtin_clzll(v) : 0; }
 
+// An entry holds for the kernels it was timed on: kTuneVersion changes with them, and
+// the threshold range decides between two forms of them (two CTAs of 256 threads an SM,
+// or one of 512), each with best settings of its own.
+constexpr int kTuneVersion = 2;
+
 static std::string tune_key(const pd_ctx *c, const pd_train_params *p, uint32_t end_depth) {
   cudaDeviceProp prop;
   memset(&prop, 0, sizeof(prop));
@@ -49,7 +55,8 @@ static std::string tune_key(const pd_ctx *c, const pd_train_params *p, uint32_t 
   std::ostringstream s;
   s << name << "/sm" << prop.multiProcessorCount << "/cfg" << c->cfg.plugin << "." << c->cfg.img_type << "."
     << c->cfg.n_channels << "." << c->cfg.feat_type << "." << c->cfg.feat_dim << "." << c->cfg.n_classes << "/F"
-    << p->n_features << "/T" << p->n_thresholds << "/S2^" << floor_log2(c->n_samples) << "/I2^"
+    << p->n_features << "/T" << p->n_thresholds << (rank_form(c, p) ? "/rank" : "/search") << "/v" << kTuneVersion
+    << "/S2^" << floor_log2(c->n_samples) << "/I2^"
     << floor_log2(c->n_images) << "/d" << end_depth << "/min" << p->per_leaf_samples_thr;
   return s.str();
 }
