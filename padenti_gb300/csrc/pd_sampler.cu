@@ -548,6 +548,10 @@ __global__ void __launch_bounds__(kSmThreads) k_class_counts(const uint8_t *__re
   const uint32_t p = s * kSeg + 16 * lane;
   const uint4 q = p < g.lab_vecs * 16u ? __ldg(reinterpret_cast<const uint4 *>(labels + g.lab_off + p)) : make_uint4(0, 0, 0, 0);
   const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+  if (!__any_sync(0xFFFFFFFFu, (q.x | q.y | q.z | q.w) != 0u)) {  // a segment without labels
+    for (uint32_t k = lane; k < n_classes; k += 32) counts[(size_t)g.seg0 * n_classes + (size_t)k * segs + s] = 0u;
+    return;
+  }
   uint32_t bad = 0;
   for (uint32_t k0 = 0; k0 < n_classes; k0 += 32) {
     const uint32_t nk = min(n_classes - k0, 32u);

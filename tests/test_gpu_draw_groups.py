@@ -49,3 +49,24 @@ def test_groups_of_draws(bytes_):
                               s.stride, o.ctypes.data, c.ctypes.data))
     for i in range(len(sizes)):
         assert np.array_equal(o[i, :c[i]], ob.sample_class_weighted(ims[i], lbs[i], 400, K, None, 11))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [3, 20, 40])
+def test_stretches_without_labels(K):
+    """Images labelled in a few places only: segments (512 pixels) and pairs of them without a
+    label, and ones with a single labelled pixel at either end."""
+    import oracle_bind as ob
+
+    rng = np.random.default_rng(K)
+    w, h = 131, 100
+    px = rng.integers(0, 5000, (4, h, w)).astype(np.uint16)
+    lb = np.zeros((4, h * w), np.uint8)
+    lb[0, [0, 511, 512, 1023, 1024, 5000, h * w - 1]] = [1, 2, 1, K, 2, 3, 1]
+    lb[1, 4000:4700] = rng.integers(1, K + 1, 700)
+    lb[2, h * w - 40:] = 2
+    lb[3, rng.integers(0, h * w, 30)] = 3
+    s = pg.ClassWeightedImageSampler(12, K, seed=2)
+    lb = lb.reshape(4, h, w)
+    for got, p, l in zip(s.sample_batch(list(px), list(lb)), px, lb):
+        assert np.array_equal(got, ob.sample_class_weighted(p, l, 12, K, None, 2))
