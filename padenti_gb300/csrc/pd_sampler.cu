@@ -917,18 +917,64 @@ const uint32_t *shift_constants() {
   return tab.data();
 }
 
+// Places of the images' draws in the class-weighted sampler's buffer of MT19937 outputs,
+// a word a pixel, for a group of images at a time: a group holds at most `group` words,
+// one image at least.  Returns the words that the largest needs.
+uint64_t place_draws(SampImage *im, uint32_t n, uint64_t group) {
+  uint64_t at = 0, most = 0;
+  for (uint32_t i = 0; i < n; i++) {
+    const uint64_t words = ((uint64_t)im[i].n_pix + 3) / 4 * 4;
+    if (at && at + words > group) at = 0;
+    im[i].draw_off = at;
+    at += words;
+    most = std::max(most, at);
+  }
+  return most;
+}
+
+// That buffer, for images placed in groups of draw_group(ctx): twice the bytes that a
+// host batch stages at once (1 GiB, 873 maps of 640x480).  A group should fill the GPU,
+// as its draws are a serial chain: the drawing phase of 500 maps in one group takes 0.72
+// ms, in two 0.80, in four 1.02, in eight 1.52.  Where that much memory is not free the
+// images are placed again in smaller groups; *again: the descriptors changed.
+uint64_t draw_group(const pd_ctx *ctx) { return ctx->sample_group / 2; }
+int reserve_draws(pd_ctx *ctx, SampImage *im, uint32_t n, bool *again) {
+  *again = false;
+  uint64_t one = 0, most = 0;
+  for (uint32_t i = 0; i < n; i++) {
+    const uint64_t words = ((uint64_t)im[i].n_pix + 3) / 4 * 4;
+    one = std::max(one, words);
+    most = std::max(most, im[i].draw_off + words);
+  }
+  int rc;
+  while ((rc = ctx->sm_draws.ensure(most * 4)) == PD_ERR_NOMEM && most > one) {
+    if (!*again) PD_CUDA(cudaStreamSynchronize(ctx->stream));  // the descriptors' upload reads them
+    *again = true;
+    most = place_draws(im, n, most / 2);
+  }
+  return rc;
+}
+
+// Gives back what a single larger image took of it.
+void trim_draws(pd_ctx *ctx) {
+  if (ctx->sm_draws.cap > 2 * ctx->sample_group) ctx->sm_draws.release();
+}
+
 // The class-weighted sampler's kernels on a batch (images and checksums in place).
 // Its scratch -- segment counts, draws, slots -- belongs to the context, like its
 // stream: calls on one context are serialised.
-int launch_class_weighted(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32_t n, const uint8_t *host_desc,
-                          const DescLayout &lay, const uint8_t *labels, const SampImage *imgs, const uint32_t *crc,
+int launch_class_weighted(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32_t n, uint8_t *host_desc,
+                          const DescLayout &lay, const uint8_t *labels, SampImage *imgs, const uint32_t *crc,
                           const uint32_t *bucket, uint32_t *out, uint32_t *counts, uint32_t *err, uint64_t *launched) {
   cudaStream_t st = ctx->stream;
   const uint32_t K = s->n_classes;
-  const SampImage *h = reinterpret_cast<const SampImage *>(host_desc + lay.imgs);
+  SampImage *h = reinterpret_cast<SampImage *>(host_desc + lay.imgs);
   auto segs_of = [&](uint32_t i) { return (h[i].n_pix + kSeg - 1) / kSeg; };
   const uint32_t segs = h[n - 1].seg0 + segs_of(n - 1);
   const size_t slot_bytes = (size_t)n * std::max(1u, pl.stride) * 4;
+  bool again = false;
+  PD_TRY(reserve_draws(ctx, h, n, &again));
+  if (again) PD_CUDA(h2d(ctx, imgs, h, sizeof(SampImage) * n));
   PD_TRY(ctx->sm_counts.ensure(((size_t)segs * (K + 1) + (size_t)n * (K + 1)) * 4));
   PD_TRY(ctx->sm_slots.ensure(slot_bytes));
   uint32_t *c = ctx->sm_counts.as<uint32_t>(), *draw0 = c + (size_t)segs * K, *tot = draw0 + segs,
@@ -972,10 +1018,10 @@ int launch_class_weighted(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &p
 // Uploads the descriptor block and launches the kernels on a batch that is
 // in device memory.  counts/err stay on the device.
 int launch_batch(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32_t n, const uint8_t *data, const uint8_t *labels, uint32_t *out, uint32_t *counts, const DescLayout &lay,
-                 uint8_t *dev_desc, const void *host_desc, cudaEvent_t *ev) {
+                 uint8_t *dev_desc, void *host_desc, cudaEvent_t *ev) {
   cudaStream_t st = ctx->stream;
   PD_CUDA(h2d(ctx, dev_desc, host_desc, lay.bytes));
-  const SampImage *imgs = reinterpret_cast<const SampImage *>(dev_desc + lay.imgs);
+  SampImage *imgs = reinterpret_cast<SampImage *>(dev_desc + lay.imgs);
   const uint32_t *item_img = reinterpret_cast<const uint32_t *>(dev_desc + lay.items);
   uint32_t *crc = reinterpret_cast<uint32_t *>(dev_desc + lay.crc);
   uint32_t *cnt = reinterpret_cast<uint32_t *>(dev_desc + lay.count);
@@ -1000,7 +1046,7 @@ int launch_batch(pd_ctx *ctx, const pd_sampler *s, const SamplerPlan &pl, uint32
     k_sample_uniform<<<n, kSmThreads, smem, st>>>(labels, imgs, crc, cnt, s->n_samples, s->seed, buckets, out, counts,
                                                   err);
   } else {
-    PD_TRY(launch_class_weighted(ctx, s, pl, n, static_cast<const uint8_t *>(host_desc), lay, labels, imgs, crc,
+    PD_TRY(launch_class_weighted(ctx, s, pl, n, static_cast<uint8_t *>(host_desc), lay, labels, imgs, crc,
                                  reinterpret_cast<const uint32_t *>(dev_desc + lay.bucket), out, counts, err, &launched));
   }
   PD_CUDA(cudaGetLastError());
@@ -1016,37 +1062,9 @@ struct ImagePlace {
   uint32_t n_pix;
 };
 
-// Draws of an image in the class-weighted sampler's buffer: a word a pixel.
-uint64_t draw_words(const ImagePlace &p) { return ((uint64_t)p.n_pix + 3) / 4 * 4; }
-
-// The class-weighted sampler's buffer of MT19937 outputs, for a group of images at a
-// time (one at least): the draws of the whole batch, at most twice the bytes that a
-// host batch stages at once (sample_group: 1 GiB of draws, 873 maps of 640x480).  A
-// group should fill the GPU, as its draws are a serial chain: the drawing phase of 500
-// maps in one group takes 0.72 ms, in two 0.80, in four 1.02, in eight 1.52.  Where
-// that much memory is not free, smaller groups.
-int reserve_draws(pd_ctx *ctx, const std::vector<ImagePlace> &place, uint64_t *group) {
-  uint64_t all = 0, one = 0;
-  for (const ImagePlace &p : place) {
-    all += draw_words(p);
-    one = std::max(one, draw_words(p));
-  }
-  for (uint64_t words = std::max(one, std::min(all, ctx->sample_group / 2));; words = std::max(one, words / 2)) {
-    const int rc = ctx->sm_draws.ensure(words * 4);
-    *group = words;
-    if (rc != PD_ERR_NOMEM || words == one) return rc;
-  }
-}
-
-// Gives back what a single larger image took of it.
-void trim_draws(pd_ctx *ctx) {
-  if (ctx->sm_draws.cap > 2 * ctx->sample_group) ctx->sm_draws.release();
-}
-
 // Fills the pinned descriptor block for images described by (data_lo, data
-// bytes, lab_off, n_pix, out_off); draw_group: words of draws kept at a time
-// (class-weighted).
-int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> &place, uint64_t draw_group,
+// bytes, lab_off, n_pix, out_off); group: of their draws (place_draws).
+int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> &place, uint64_t group,
               DescLayout *lay_out) {
   const uint32_t n = (uint32_t)place.size();
   uint64_t n_crc = 0, n_lab = 0;
@@ -1067,15 +1085,12 @@ int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> 
   uint32_t *crc = reinterpret_cast<uint32_t *>(h + lay.crc);
   uint32_t *cnt = reinterpret_cast<uint32_t *>(h + lay.count);
   uint32_t ic = 0, il = (uint32_t)n_crc;
-  uint64_t segs = 0, draws = 0;
+  uint64_t segs = 0;
   for (uint32_t i = 0; i < n; i++) {
     const ImagePlace &p = place[i];
-    const uint64_t dw = draw_words(p);
-    if (draws && draws + dw > draw_group) draws = 0;
     im[i] = SampImage{p.data_lo, p.data_end, p.lab_off, p.out_off, p.n_pix, (p.n_pix + 15) / 16, slices[i], ic, il,
-                      (uint32_t)segs, draws};
+                      (uint32_t)segs, 0};
     segs += (p.n_pix + kSeg - 1) / kSeg;
-    draws += dw;
     for (uint32_t k = 0; k < slices[i]; k++) item_img[ic++] = i;
     for (uint32_t k = 0; k < chunks[i]; k++) item_img[il++] = i;
     // the initial value 0xFFFFFFFF carried past the image bytes, and the final XOR
@@ -1087,6 +1102,7 @@ int fill_desc(HostBuf &hb, const SamplerPlan &pl, const std::vector<ImagePlace> 
     cnt[i] = 0;
   }
   PD_CHECK(segs < (1ull << 31), PD_ERR_UNSUPPORTED, "batch too large");
+  place_draws(im, n, group);
   std::memcpy(h + lay.shifts, shift_constants(), 4ull * kShiftWords);
   reinterpret_cast<uint32_t *>(h + lay.err)[0] = kNoError;  // first image with a label above nClasses
   reinterpret_cast<uint32_t *>(h + lay.err)[1] = kNoError;  // first image whose draws hit the block limit
@@ -1244,12 +1260,7 @@ extern "C" int pd_sample(pd_ctx *ctx, const pd_sampler *s, uint32_t n_images, co
       for (auto &x : th) x.join();
     }
     DescLayout &lay = lays[si];
-    uint64_t draw_group = 0;
-    if (s->kind == PD_SAMPLER_CLASS_WEIGHTED) {
-      const int rc = reserve_draws(ctx, g.place, &draw_group);
-      if (rc != PD_OK) return fail(rc);
-    }
-    PD_TRY(fill_desc(sl.h_desc, pl, g.place, draw_group, &lay));
+    PD_TRY(fill_desc(sl.h_desc, pl, g.place, draw_group(ctx), &lay));
     PD_TRY(sl.d_data.ensure(g.data_cur + g.lab_cur + 16));
     PD_TRY(sl.d_desc.ensure(lay.bytes));
     const uint64_t out_words = (uint64_t)n * stride + n;
@@ -1309,9 +1320,7 @@ extern "C" int pd_sample_device(pd_ctx *ctx, const pd_sampler *s, uint32_t n_ima
   for (uint32_t i = 0; i < n_images; i++)
     place[i] = ImagePlace{i * db, (i + 1) * db, i * np, (uint64_t)i * stride, db, (uint32_t)np};
   DescLayout lay;
-  uint64_t draw_group = 0;
-  if (s->kind == PD_SAMPLER_CLASS_WEIGHTED) PD_TRY(reserve_draws(ctx, place, &draw_group));
-  PD_TRY(fill_desc(ctx->h_sm_desc, pl, place, draw_group, &lay));
+  PD_TRY(fill_desc(ctx->h_sm_desc, pl, place, draw_group(ctx), &lay));
   PD_TRY(ctx->sm_desc.ensure(lay.bytes));
   PD_TRY(launch_batch(ctx, s, pl, n_images, static_cast<const uint8_t *>(images_device), labels_device,
                       samples_device, counts_device, lay, ctx->sm_desc.as<uint8_t>(), ctx->h_sm_desc.ptr, ctx->ev));
