@@ -100,7 +100,7 @@ extern "C" int pd_ctx_destroy(pd_ctx *ctx) {
   cudaStreamSynchronize(ctx->stream);
   DevBuf *bufs[] = {&ctx->pixels, &ctx->img_off, &ctx->img_wh, &ctx->s_xy, &ctx->s_img, &ctx->s_label,
                     &ctx->log2_tab, &ctx->magic_tab, &ctx->snode, &ctx->act[0], &ctx->act[1], &ctx->act_rec[0], &ctx->act_rec[1], &ctx->s_rec, &ctx->act_slot[0],
-                    &ctx->act_slot[1], &ctx->flags, &ctx->scan_blocks, &ctx->slot_adj, 
+                    &ctx->act_slot[1], &ctx->flags, &ctx->scan_blocks,
                     &ctx->cand_feat, &ctx->cand_thr, &ctx->cand_perm, &ctx->cand_ord, &ctx->parent, &ctx->xlog2_tab, &ctx->hist, &ctx->g32, &ctx->items, &ctx->hist_queue,
                     &ctx->split_res, &ctx->d_pre, &ctx->d_splits, &ctx->split_scratch, &ctx->fused_scratch, &ctx->t_lc,
                     &ctx->t_feat, &ctx->t_thr, &ctx->t_post, &ctx->f_lc, &ctx->f_feat, &ctx->f_thr,
@@ -114,14 +114,10 @@ extern "C" int pd_ctx_destroy(pd_ctx *ctx) {
   ctx->b_out.release();
   ctx->b_desc.release();
   rtc_release(ctx);
-  ctx->sm_data.release();
-  ctx->sm_lab.release();
   ctx->sm_desc.release();
-  ctx->sm_out.release();
   ctx->sm_counts.release();
   ctx->sm_draws.release();
   ctx->sm_slots.release();
-  ctx->h_sm.release();
   ctx->h_sm_desc.release();
   for (auto &sl : ctx->samp) {
     sl.h_data.release();

@@ -69,7 +69,6 @@ struct pd_ctx {
   pd::DevBuf s_rec;                  // SampleRec of every uploaded sample
   pd::DevBuf flags;                  // uint8 per active sample
   pd::DevBuf scan_blocks;            // uint64 per scan block
-  pd::DevBuf slot_adj;               // int64 [4] per slot: adjL, adjR, kL, kR
   pd::DevBuf cand_feat, cand_thr, cand_perm;
   pd::DevBuf cand_ord;       // [slots][F] original candidate index of each column
   pd::DevBuf hist, g32;
@@ -117,11 +116,9 @@ struct pd_ctx {
   cudaGraphExec_t batch_graph = nullptr;
 
   // ---- pixel samplers (pd_sample*) ----
-  pd::DevBuf sm_data, sm_lab;    // staged image data and labels of a host batch
   pd::DevBuf sm_desc;            // SampImage per image, item -> image map, checksums, counts, error
-  pd::DevBuf sm_out;             // samples and counts of a host batch
   pd::DevBuf sm_counts, sm_draws, sm_slots;  // class-weighted: segment counts, MT19937 outputs (reserve_draws), buckets
-  pd::HostBuf h_sm, h_sm_desc;   // pinned staging of a host batch and of its descriptors
+  pd::HostBuf h_sm_desc;         // pinned staging of the descriptors
   // pd_sample's two pipeline slots: a group is staged into one while the device
   // works on the other's (pinned data, descriptors, results; device copies; events
   // around the scan, the draws and the results)
