@@ -263,8 +263,10 @@ PD_D void bitonic_sort_regs(uint32_t (&k)[N]) {
 }
 
 // The draws run in a loop over the MD5 blocks, through a shared-memory column of the
-// thread's own (fully unrolled, 13 blocks of 64 steps outgrow the instruction cache:
-// 5.6 of 9.3 stall cycles per instruction waited for it, 37 % issue-active).
+// thread's own (fully unrolled, 13 blocks of 64 steps outgrow the instruction cache: a
+// middle level of depth-20 trees with 1000 candidates a node took 117 us, this 77).
+// Bound by the integer ALU: 370 nodes x 2000 candidates x 50 thresholds 200 us, ALU
+// pipe 90 %.
 template <typename FeatT, int TP>
 __global__ void __launch_bounds__(kCandThreads) k_candidates_reg(const int32_t *__restrict__ nodes, uint32_t n_nodes,
                                                                  uint32_t tree, uint32_t F, uint32_t T, int D,
@@ -427,6 +429,7 @@ struct SplitPart {
 // leave a node with other samples than its class totals say, so every split kernel
 // compares the counts with the totals before it indexes a table with their difference,
 // and on a mismatch picks nothing and reports it here; the host then fails the call.
+// The comparisons cost a tree up to 0.6 % (600 maps of 640x480: 119.2 -> 119.4 ms).
 PD_D void samples_disagree(unsigned long long *rechecked) { rechecked[1] = 1ull; }
 
 constexpr int kSplitCols = 128;  // threads of a split CTA, one column each per pass
@@ -1485,16 +1488,20 @@ __global__ void __launch_bounds__(small_threads(NC), small_ctas(NC))
                                            return i < NC ? i : 0u;  // NC: a class the totals lack
                                          });
   __syncthreads();
-  // no class has more samples than its total (both sum to N: each has as many)
-  const bool agree = !__syncthreads_or(threadIdx.x < NC && s_seen[threadIdx.x] != s_tot[threadIdx.x]);
-  if (!agree && threadIdx.x == 0) samples_disagree(fs.rechecked);
+  // whether every class has as many samples as its total
+  bool agree = true;
+  if constexpr (kPrefix) {
+    agree = threadIdx.x >= NC || s_seen[threadIdx.x] == s_tot[threadIdx.x];  // to all at the prefix's barrier
+  } else {
+#pragma unroll
+    for (int l = 0; l < NC; l++) agree &= s_seen[l] == s_tot[l];
+  }
 
   const uint32_t nc = s_nc, N = w.end - w.begin;
   const uint32_t c = threadIdx.x & (kTileF - 1), part = threadIdx.x / kTileF;
   const uint32_t *fw = rt.first + c * rt.first_words;
   uint32_t D = 0;  // distinct thresholds of the column (0 past the last column)
   for (uint32_t k = 0; k < rt.first_words; k++) D += __popc(fw[k]);
-  const bool ok = agree && (uint64_t)N < fs.L_len;
   if constexpr (kPrefix) {
     // cumulative counts in place, a thread per (class, packed column)
     for (uint32_t q = threadIdx.x; q < nc * 32; q += kSmallThreads) {
@@ -1515,8 +1522,10 @@ __global__ void __launch_bounds__(small_threads(NC), small_ctas(NC))
         p[j * 32] = run;
       }
     }
-    __syncthreads();
+    agree = !__syncthreads_or(!agree);
   }
+  if (!agree && threadIdx.x == 0) samples_disagree(fs.rechecked);
+  const bool ok = agree && (uint64_t)N < fs.L_len;
   // counts of row j, compact class i, at h[(i * TS + j) * 64]
   const uint16_t *h = reinterpret_cast<const uint16_t *>(sh_hist) + (c & 31) * 2 + (c >> 5);
   double best = -DBL_MAX;
