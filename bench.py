@@ -955,7 +955,7 @@ def run_ours(a):
                                   traffic=None, peak_source=f"{peak_kind_p} (hbm_gbs)",
                                   note="38 algorithmic B/px: the 2-byte depth read once and 9 float posteriors "
                                        "written once; the forest's nodes stay in L2; the kernel is bound by "
-                                       "instruction issue (tree walks), not HBM"),
+                                       "the L1 data pipe (node records, probes), not HBM"),
                     note="500 held-out 640x480 images in one launch, forest of the timed trees, 38 algorithmic B/px")
         if not a.no_cpu:
             pred["cpu_baseline"] = cpu_predict(a, cfg, trees, hx)

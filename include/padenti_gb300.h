@@ -197,9 +197,10 @@ typedef struct {
  * trees of end_depth levels with `params` on the uploaded training set (at
  * most max_trials settings; 0 = no limit), every tree checked equal to the
  * first.  The winner is applied to the context and, with cache_path, appended
- * to that text file under a key of (GPU, SM count, configuration, F, T,
- * training-set size class, depth, min samples per leaf); a later call with the
- * same key applies the cached setting without timing. */
+ * to that text file under a key of (GPU, SM count, configuration, F, T, form of
+ * the histogram kernels (the threshold range decides), version, training-set
+ * size class, depth, min samples per leaf); a later call with the same key
+ * applies the cached setting without timing. */
 int pd_autotune(pd_ctx *ctx, const pd_train_params *params, uint32_t end_depth, uint32_t max_trials,
                 const char *cache_path, pd_tuning *out);
 /* Synchronises the context's stream. */

@@ -531,7 +531,7 @@ constexpr int kResCtas = 5;
 // counts[seg0 * n_classes + k * segs + s].  A warp per segment; 32 classes at a time
 // in counters of the lane's own ([class][lane], no conflicts): one shared add per
 // label, then a warp sum per class.  Labels above n_classes are errors (err: the
-// lowest image).
+// lowest image).  Issue-bound (300 maps, 92 MB of labels: 59 us, 86 % issue-active).
 // Grid: (segments of the largest image / kSmWarps, images).
 __global__ void __launch_bounds__(kSmThreads) k_class_counts(const uint8_t *__restrict__ labels,
                                                              const SampImage *__restrict__ imgs, uint32_t first,
@@ -622,10 +622,10 @@ __global__ void __launch_bounds__(kSmThreads) k_class_prefix(const SampImage *__
 // 224 words go at a time, two a thread (64-bit shared accesses), one barrier each; the
 // words run through a linear array (fixed offsets from one pointer) whose last 624
 // move to its start at the end of a lap.  A step's words are tempered and stored
-// while the next step's loads are in flight, off the chain.  ALU-bound when an SM
-// holds four images (64 % of the pipe), the chain's latency below that; one word a
-// thread in 8 warps 0.22 ms for 500 images, four in 2 warps 0.21, this 0.20.  Every
-// thread of the CTA works in every step: the barriers see whole warps.
+// while the next step's loads are in flight, off the chain.  Bound by the chain's
+// latency (300 images, two an SM: 48 % issue-active, ALU pipe 50 %, 301 MB written in
+// 0.15 ms); one word a thread in 8 warps 0.22 ms for 500 images, four in 2 warps 0.21,
+// this 0.20.  Every thread of the CTA works in every step: the barriers see whole warps.
 constexpr uint32_t kMtStep = 224, kMtThreads = kMtStep / 2, kMtLap = 15;
 constexpr uint32_t kMtWords = kMtN + kMtLap * kMtStep;
 __global__ void __launch_bounds__(kMtThreads) k_mt_draws(const SampImage *__restrict__ imgs, uint32_t first,
@@ -672,9 +672,10 @@ static_assert(kMtLap * kMtStep >= kMtN, "a lap's end does not overlap its start"
 // BITS: of a label, n_classes < 2^BITS; up to 32 classes are counted a lane each (a
 // row's mask of class k is lane k's, and goes to the pixels of class k by a shuffle);
 // BITS = 8: more classes, counted in shared memory.
-// Issue-bound (62 instructions per row of 32 pixels, 50 % issue-active at 24 warps,
-// waiting for the draws); eight rows in flight with four CTAs 0.386 ms, four rows with
-// five 0.378; all rows of a segment unrolled 0.48-0.74 (instruction cache).
+// Issue- and ALU-bound (300 maps: 68 instructions per row of 32 pixels, 71 %
+// issue-active, ALU pipe 73 %, 36 warps an SM).  500 maps: eight rows in flight with
+// four CTAs 0.386 ms, four rows with five 0.378; all rows of a segment unrolled
+// 0.48-0.74 (instruction cache).
 template <int BITS>
 __global__ void __launch_bounds__(kSmThreads, kResCtas) k_reservoir(const uint8_t *__restrict__ labels,
                                                           const SampImage *__restrict__ imgs, uint32_t first,
